@@ -9,6 +9,9 @@
 // keys (not in M's row) are sorted with a block bitonic sort. Longer rows are
 // processed in column windows of kWin columns with a dense shared-memory
 // accumulator and bitmap, which yields sorted output directly.
+//
+// Products with at most kNarrowCols columns (the frontier of a batched search:
+// one column per source) take the narrow path below instead.
 #include "ga_device.cuh"
 
 namespace ga {
@@ -293,12 +296,366 @@ __global__ void __launch_bounds__(kCmThreads) k_cmask(CmArgs<T> p) {
     }
 }
 
+// ------------------------------------------------------------- narrow path
+// B with at most kNarrowCols columns, handled in blocks of 64: a row's pattern
+// inside a block is one 64-bit word. The symbolic pass ORs the words of the B
+// rows an A row selects (8 bytes per A entry, no product is visited) and drops
+// the mask row's; the numeric pass gives every lane two columns of the block,
+// transposes the words of 32 B rows across the warp, and each lane walks the
+// rows that hold its columns, their values placed by popcounts. The sums stay
+// in registers: no hash table, no sort, no atomics.
+//
+// What bounds it: the chain of gathers per 32 A entries (column, word, B row
+// start, values) from the L2, and in FP64 the adder (2 lanes per clock and SM
+// whether one lane of the warp is active or 32), which is why the lanes walk
+// their own lists: visiting the B rows one by one with a lane per column left
+// 3 of 32 lanes active and took 1,520 us for the level below. A row with more
+// than kNarrowHeavy entries is cut into pieces of kNarrowPiece that separate
+// CTAs sum (with 512-thread CTAs and pieces of 2,048 the numeric pass took 171
+// us: the rows of a CTA wait for its longest); the last piece to finish adds
+// the pieces in order.
+//
+// One breadth-first level of 64 sources on R-MAT 16 (complemented product,
+// 1.9M A entries, 2.1e5 frontier entries, 30 % of the pairs masked): 157 us
+// (words 12, symbolic 37, numeric 108); the per-row hash path below takes
+// 4,350 us. The line at kNarrowCols, the largest batch of sources: frontier
+// density 0.002 / 0.05 / 0.3 on the same graph, whole call, this path against
+// the hash and window path: 64 columns 163 / 232 / 453 against 1,400 / 4,860 /
+// 9,074 us; 256 columns 297 / 592 / 1,505 against 2,397 / 8,072 / 17,819 us;
+// 1,024 columns 874 / 2,045 / 5,681 against 4,707 / 15,473 / 54,951 us.
+constexpr int kNarrowCols = 1024;
+constexpr int kNarrowThreads = 512;      // symbolic pass
+constexpr int kNarrowWarps = kNarrowThreads / 32;
+constexpr int kNarrowSumThreads = 128;   // numeric pass: small CTAs, a long row holds up few others
+constexpr int kNarrowSumWarps = kNarrowSumThreads / 32;
+constexpr int kNarrowHeavy = 256;
+constexpr int kNarrowPiece = 512;
+
+struct NarrowTask {
+    int32_t row, piece;   // kNarrowPiece entries of the row
+    int32_t first, count; // the row's pieces: places first .. first + count - 1 of the partial sums
+};
+
+struct NarrowArgs {
+    const unsigned long long* bbits;  // [block][row of B]: columns of the block
+    const int32_t* bpos;              // [block][row of B]: position of the first of them
+    unsigned long long* pat;          // [block][row of A]: columns of the result
+    int64_t bm;                       // rows of B
+    int blocks;
+    NarrowTask* tasks;
+    int32_t* ntask;
+    int32_t* done;                    // per place: pieces finished (at the row's first place)
+    void* part;                       // partial sums, 64 per place and block
+};
+
+// Words of a matrix's rows, one warp per row.
+__global__ void k_row_bits(const int32_t* __restrict__ rst, const int32_t* __restrict__ col, int64_t m, int blocks,
+                           unsigned long long* __restrict__ bits, int32_t* __restrict__ pos) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += warps) {
+        const int32_t e = rst[i + 1];
+        int32_t b = rst[i];
+        for (int x = 0; x < blocks; ++x) {
+            uint32_t lo = 0, hi = 0;
+            int32_t q = b;
+            bool more = true;
+            while (more) {  // warp-uniform
+                const int32_t c = q + lane < e ? col[q + lane] - x * 64 : 64;
+                if (c < 32) lo |= 1u << c;
+                else if (c < 64) hi |= 1u << (c - 32);
+                const int in = __popc(__ballot_sync(0xffffffffu, c < 64));
+                q += in;
+                more = in == 32;
+            }
+            lo = __reduce_or_sync(0xffffffffu, lo);
+            hi = __reduce_or_sync(0xffffffffu, hi);
+            if (lane == 0) {
+                bits[(int64_t)x * m + i] = ((unsigned long long)hi << 32) | lo;
+                pos[(int64_t)x * m + i] = b;
+            }
+            b = q;
+        }
+    }
+}
+
+// Row of warp `wid` in CTA b: warp w's rows are the w-th run of gridDim.x
+// rows, shifted, so that neither neighbouring rows nor rows a power of two
+// apart (both are where an R-MAT graph has its hubs) share a CTA.
+__device__ __forceinline__ int64_t narrow_row(int wid) {
+    return (int64_t)wid * gridDim.x + (blockIdx.x + 1571u * (unsigned)wid) % gridDim.x;
+}
+
+// OR over the warp of a 64-bit word.
+__device__ __forceinline__ unsigned long long warp_or64(unsigned long long w) {
+    const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)w);
+    const uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)(w >> 32));
+    return ((unsigned long long)hi << 32) | lo;
+}
+
+// Result pattern and count of every row; the pieces of long rows.
+__global__ void __launch_bounds__(kNarrowThreads) k_narrow_symbolic(NarrowArgs a, const int32_t* __restrict__ ar,
+                                                                    const int32_t* __restrict__ ac,
+                                                                    const int32_t* __restrict__ mr,
+                                                                    const int32_t* __restrict__ mc, int64_t m,
+                                                                    int32_t* __restrict__ cnt) {
+    __shared__ unsigned long long s_or[kNarrowWarps][kNarrowCols / 64];
+    __shared__ int2 s_row[kNarrowWarps];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t i = narrow_row(wid);
+    const int32_t ab = i < m ? ar[i] : 0, ae = i < m ? ar[i + 1] : 0;
+    const bool heavy = ae - ab > kNarrowHeavy;
+    if (lane < kNarrowCols / 64) s_or[wid][lane] = 0ull;
+    if (lane == 0) s_row[wid] = make_int2(ab, ae);
+    __syncthreads();
+    // long rows: all warps, one row after the other
+    for (int h = 0; h < kNarrowWarps; ++h) {
+        const int32_t hb = s_row[h].x, he = s_row[h].y;
+        if (he - hb <= kNarrowHeavy) continue;
+        for (int x = 0; x < a.blocks; ++x) {
+            const unsigned long long* bb = a.bbits + (int64_t)x * a.bm;
+            unsigned long long w = 0;
+#pragma unroll 4
+            for (int32_t t = hb + (int32_t)threadIdx.x; t < he; t += kNarrowThreads) w |= __ldg(bb + __ldg(ac + t));
+            w = warp_or64(w);
+            if (lane == 0 && w) atomicOr(&s_or[h][x], w);
+        }
+    }
+    __syncthreads();
+    if (i >= m) return;
+    int32_t mq = mr ? mr[i] : 0;
+    const int32_t me = mr ? mr[i + 1] : 0;
+    int n = 0;
+    for (int x = 0; x < a.blocks; ++x) {
+        const unsigned long long* bb = a.bbits + (int64_t)x * a.bm;
+        unsigned long long w = 0, mw = 0;
+        if (heavy) {
+            w = s_or[wid][x];
+        } else {
+#pragma unroll 4
+            for (int32_t t = ab + lane; t < ae; t += 32) w |= __ldg(bb + __ldg(ac + t));
+            w = warp_or64(w);
+        }
+        bool more = mq < me;
+        while (more) {  // warp-uniform: the mask row's columns in this block
+            const int32_t c = mq + lane < me ? mc[mq + lane] - x * 64 : 64;
+            if (c < 64) mw |= 1ull << c;
+            const int in = __popc(__ballot_sync(0xffffffffu, c < 64));
+            mq += in;
+            more = in == 32;
+        }
+        w &= ~warp_or64(mw);
+        if (lane == 0) a.pat[(int64_t)x * m + i] = w;
+        n += __popcll(w);
+    }
+    if (lane != 0) return;
+    cnt[i] = n;
+    if (heavy && n) {
+        const int pieces = (ae - ab + kNarrowPiece - 1) / kNarrowPiece;
+        const int first = atomicAdd(a.ntask, pieces);
+        a.done[first] = 0;
+        for (int c = 0; c < pieces; ++c) a.tasks[first + c] = NarrowTask{(int32_t)i, c, first, pieces};
+    }
+}
+
+// Sums of the lane's two columns of block x (lane, lane + 32) over the A
+// entries [t0, t1), groups of 32 at stride `step`. s_at / s_lo / s_hi / s_a:
+// 32 entries each in shared memory for the warp.
+template <typename T>
+__device__ __forceinline__ void narrow_sums(const CmArgs<T>& p, const NarrowArgs& a, int x, int32_t t0, int32_t t1,
+                                            int32_t step, unsigned long long pw, int32_t* s_at, uint32_t* s_lo,
+                                            uint32_t* s_hi, T* s_a, T& acc0, T& acc1) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const unsigned long long* bb = a.bbits + (int64_t)x * a.bm;
+    for (int32_t g = t0; g < t1; g += step) {
+        const int32_t t = g + lane;
+        unsigned long long w = 0;
+        int32_t k = 0;
+        if (t < t1) {
+            k = __ldg(p.ac + t);
+            w = __ldg(bb + k);
+        }
+        const bool hit = (w & pw) != 0ull;
+        if (__ballot_sync(FULL, hit) == 0u) continue;
+        __syncwarp();  // the last group's lists are read
+        T av = (T)1;
+        if (hit) {
+            s_at[lane] = __ldg(a.bpos + (int64_t)x * a.bm + k);
+            s_a[lane] = av = p.av[t];
+        }
+        // a group of ones (an unweighted graph) needs no products
+        const bool ones = __all_sync(FULL, av == (T)1);
+        s_lo[lane] = (uint32_t)w;
+        s_hi[lane] = (uint32_t)(w >> 32);
+        __syncwarp();
+        // bit j: B row j of the group holds column `lane`; bit 32 + j: column lane + 32
+        const uint32_t m0 = warp_transpose_bits((uint32_t)(w & pw));
+        const uint32_t m1 = warp_transpose_bits((uint32_t)((w & pw) >> 32));
+        unsigned long long mine = ((unsigned long long)m1 << 32) | m0;
+        while (mine) {
+            T v[4], f[4];
+            bool on[4], high[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                on[h] = mine != 0ull;
+                high[h] = false;
+                if (on[h]) {
+                    const int j = __ffsll((long long)mine) - 1;
+                    mine &= mine - 1;
+                    high[h] = j >= 32;
+                    const int r = j & 31;
+                    const int off = high[h] ? __popc(s_lo[r]) + __popc(s_hi[r] & lt) : __popc(s_lo[r] & lt);
+                    v[h] = __ldg(p.bv + s_at[r] + off);
+                    f[h] = s_a[r];
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+                if (on[h]) {
+                    const T c = high[h] ? acc1 : acc0;
+                    const T s = ones ? c + v[h] : mul_add_separate<T>(c, f[h], v[h]);
+                    if (high[h]) acc1 = s;
+                    else acc0 = s;
+                }
+        }
+    }
+}
+
+// Row i's entries of block x, whose first result entry is at o.
+template <typename T>
+__device__ __forceinline__ void narrow_store(const CmArgs<T>& p, int x, int32_t o, unsigned long long pw, T acc0,
+                                             T acc1) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u, lo = (uint32_t)pw, hi = (uint32_t)(pw >> 32);
+    if (lo >> lane & 1u) {
+        const int32_t q = o + __popc(lo & lt);
+        p.cc[q] = x * 64 + lane;
+        p.cv[q] = acc0;
+    }
+    if (hi >> lane & 1u) {
+        const int32_t q = o + __popc(lo) + __popc(hi & lt);
+        p.cc[q] = x * 64 + 32 + lane;
+        p.cv[q] = acc1;
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kNarrowSumThreads) k_narrow_numeric(CmArgs<T> p, NarrowArgs a) {
+    __shared__ T s_acc[kNarrowSumWarps][64];
+    __shared__ int32_t s_at[kNarrowSumWarps][32];
+    __shared__ uint32_t s_lo[kNarrowSumWarps][32], s_hi[kNarrowSumWarps][32];
+    __shared__ T s_a[kNarrowSumWarps][32];
+    __shared__ bool s_last;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    T* part = static_cast<T*>(a.part);
+    const int ntask = *a.ntask;
+    for (int it = blockIdx.x; it < ntask; it += gridDim.x) {
+        const NarrowTask task = a.tasks[it];
+        const int32_t ab = p.ar[task.row] + task.piece * kNarrowPiece;
+        const int32_t ae = min(p.ar[task.row + 1], ab + kNarrowPiece);
+        for (int x = 0; x < a.blocks; ++x) {
+            const unsigned long long pw = a.pat[(int64_t)x * p.m + task.row];
+            T acc0 = (T)0, acc1 = (T)0;
+            if (pw)
+                narrow_sums<T>(p, a, x, ab + wid * 32, ae, kNarrowSumThreads, pw, s_at[wid], s_lo[wid], s_hi[wid],
+                               s_a[wid], acc0, acc1);
+            s_acc[wid][lane] = acc0;
+            s_acc[wid][32 + lane] = acc1;
+            __syncthreads();
+            if (threadIdx.x < 64) {
+                T sum = (T)0;
+                for (int w = 0; w < kNarrowSumWarps; ++w) sum += s_acc[w][threadIdx.x];
+                part[((int64_t)it * a.blocks + x) * 64 + threadIdx.x] = sum;
+            }
+            __syncthreads();
+        }
+        // the row's last piece to finish adds them all, in order
+        if (threadIdx.x < 64) __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(a.done + task.first, 1) == task.count - 1;
+        __syncthreads();
+        if (s_last && wid == 0) {
+            __threadfence();
+            int32_t o = p.cr[task.row];
+            for (int x = 0; x < a.blocks; ++x) {
+                const unsigned long long pw = a.pat[(int64_t)x * p.m + task.row];
+                T acc0 = (T)0, acc1 = (T)0;
+                for (int c = 0; c < task.count; ++c) {
+                    const T* q = part + ((int64_t)(task.first + c) * a.blocks + x) * 64;
+                    acc0 += __ldcg(q + lane);
+                    acc1 += __ldcg(q + 32 + lane);
+                }
+                narrow_store<T>(p, x, o, pw, acc0, acc1);
+                o += __popcll(pw);
+            }
+        }
+        __syncthreads();
+    }
+    const int64_t i = narrow_row(wid);
+    if (i >= p.m) return;
+    const int32_t ab = p.ar[i], ae = p.ar[i + 1];
+    int32_t o = p.cr[i];
+    if (ae - ab > kNarrowHeavy || o == p.cr[i + 1]) return;
+    for (int x = 0; x < a.blocks; ++x) {
+        const unsigned long long pw = a.pat[(int64_t)x * p.m + i];
+        if (pw == 0ull) continue;
+        T acc0 = (T)0, acc1 = (T)0;
+        narrow_sums<T>(p, a, x, ab, ae, 32, pw, s_at[wid], s_lo[wid], s_hi[wid], s_a[wid], acc0, acc1);
+        narrow_store<T>(p, x, o, pw, acc0, acc1);
+        o += __popcll(pw);
+    }
+}
+
+template <typename T>
+static ga_csr cmask_narrow(ga_ctx ctx, ga_csr A, ga_csr B, CmArgs<T> p) {
+    const int64_t m = A->m;
+    const int blocks = (int)((B->n + 63) / 64);
+    const size_t places = (size_t)(A->nnz / kNarrowPiece + A->nnz / kNarrowHeavy + 1);
+    DBuf<unsigned long long> bbits(ctx, (size_t)B->m * blocks), pat(ctx, (size_t)m * blocks);
+    DBuf<int32_t> bpos(ctx, (size_t)B->m * blocks), cnt(ctx, (size_t)m + 1), rst(ctx, (size_t)m + 1);
+    DBuf<NarrowTask> tasks(ctx, places);
+    DBuf<int32_t> done(ctx, places), ntask(ctx, 1);
+    DBuf<T> part(ctx, places * blocks * 64);
+    const NarrowArgs a{bbits.p, bpos.p, pat.p, B->m, blocks, tasks.p, ntask.p, done.p, part.p};
+    const unsigned grid = (unsigned)((m + kNarrowWarps - 1) / kNarrowWarps);
+    {
+        ProfScope ps(ctx, "cmask_symbolic");
+        GA_CUDA(cudaMemsetAsync(ntask.p, 0, sizeof(int32_t), ctx->stream));
+        k_row_bits<<<grid_for(B->m * 32, 256, ctx->num_sms * 64), 256, 0, ctx->stream>>>(B->rst, B->col, B->m, blocks,
+                                                                                         bbits.p, bpos.p);
+        post_launch("cmask_row_bits");
+        k_narrow_symbolic<<<grid, kNarrowThreads, 0, ctx->stream>>>(a, A->rst, A->col, p.mr, p.mc, m, cnt.p);
+        post_launch("cmask_narrow_symbolic");
+    }
+    scan_exclusive_i32(ctx, cnt.p, rst.p, m);
+    const int64_t nnz = read_i32(ctx, rst.p + m);
+    ga_csr C = csr_alloc(ctx, m, B->n, nnz, A->dtype);
+    try {
+        GA_CUDA(cudaMemcpyAsync(C->rst, rst.p, sizeof(int32_t) * (m + 1), cudaMemcpyDeviceToDevice, ctx->stream));
+        if (nnz) {
+            p.cr = C->rst; p.cc = C->col; p.cv = static_cast<T*>(C->val);
+            ProfScope ps(ctx, "cmask_numeric");
+            k_narrow_numeric<T><<<(unsigned)((m + kNarrowSumWarps - 1) / kNarrowSumWarps), kNarrowSumThreads, 0,
+                                  ctx->stream>>>(p, a);
+            post_launch("cmask_narrow_numeric");
+        }
+    } catch (...) {
+        csr_destroy(ctx, C);
+        throw;
+    }
+    return C;
+}
+
 template <typename T>
 static ga_csr cmask_typed(ga_ctx ctx, ga_csr A, ga_csr B, const int32_t* mr, const int32_t* mc) {
     CmArgs<T> p;
     p.ar = A->rst; p.ac = A->col; p.av = static_cast<const T*>(A->val);
     p.br = B->rst; p.bc = B->col; p.bv = static_cast<const T*>(B->val);
     p.mr = mr; p.mc = mc; p.m = A->m;
+    p.flops = nullptr; p.cnt = nullptr; p.cr = nullptr; p.cc = nullptr; p.cv = nullptr;
+    if (A->m > 0 && B->n >= 1 && B->n <= kNarrowCols) return cmask_narrow<T>(ctx, A, B, p);
     DBuf<int64_t> flops(ctx, (size_t)A->m + 1);
     DBuf<int32_t> cnt(ctx, (size_t)A->m + 1);
     p.flops = flops.p; p.cnt = cnt.p;

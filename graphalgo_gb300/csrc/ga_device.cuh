@@ -94,6 +94,20 @@ __device__ __forceinline__ V warp_sum(V v) {
     return v;
 }
 
+// 32 x 32 bit transpose across the warp: bit c of lane r on entry is bit r of
+// lane c on return.
+__device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x) {
+    const int lane = threadIdx.x & 31;
+    uint32_t low = 0x0000ffffu;  // columns whose bit s is 0
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, s);
+        x = (lane & s) ? (x & ~low) | ((y & ~low) >> s) : (x & low) | ((y & low) << s);
+        low ^= low << (s >> 1);
+    }
+    return x;
+}
+
 // --------------------------------------------------------------- hashing
 __device__ __forceinline__ uint32_t hash_col(int32_t c) { return (uint32_t)c * 0x9E3779B1u; }
 
