@@ -107,8 +107,7 @@ def parse_args():
     ap.add_argument("--reps", type=int, default=2)
     ap.add_argument("--sources", type=int, default=64)
     ap.add_argument("--bc-backward", type=int, default=None, choices=[0, 1, 2],
-                    help="BC case: how the backward sweep reads W rows (GA_OPT_BC_BACKWARD: 0 gathers, "
-                         "1 bulk copies, 2 one neighbour at a time)")
+                    help="BC case: value of GA_OPT_BC_BACKWARD (accepted, without effect)")
     ap.add_argument("--ingest-scale", type=int, default=20, help="ingest workload: R-MAT scale of the file")
     ap.add_argument("--workload", choices=["ktruss-sweep", "batch", "serve", "ingest"], default="ktruss-sweep",
                     help="ktruss-sweep: the R-MAT k-truss sweep; batch: TC + 4-truss of many k-NN graphs; "

@@ -84,7 +84,7 @@ struct CachedLoop {
 };
 
 CachedLoop* cache_slot(ga_ctx ctx, int slot) {
-    GA_REQUIRE(slot >= 0 && slot < 4, GA_ERR_INVALID_ARG, "loop cache slot out of range");
+    GA_REQUIRE(slot >= 0 && slot < kLoopSlots, GA_ERR_INVALID_ARG, "loop cache slot out of range");
     if (!ctx->loop_cache[slot]) ctx->loop_cache[slot] = new CachedLoop();
     CachedLoop* c = static_cast<CachedLoop*>(ctx->loop_cache[slot]);
     if (!c->cont) GA_CUDA(cudaMalloc(&c->cont, sizeof(int)));

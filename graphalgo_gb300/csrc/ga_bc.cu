@@ -2,26 +2,47 @@
 // include/betweenness_centrality.h:125-237) with FP64 path counts and
 // dependencies, device-resident from the first frontier to the scores.
 //
-// Layout (vertex x source pairs, ns = number of sources):
-//  * an append-only entry store (source index, sigma, bcu = 1 + delta), one
-//    record per discovered (vertex, source) pair, grouped per (level, vertex);
-//  * per level, a list of frontier rows (vertex, first entry, length) - the
-//    reference's Sigmas[d];
-//  * a visited bitmap per vertex (ns bits) - the reference's Numsp pattern;
-//  * a dense m x ns FP64 matrix W used by the backward sweep.
+// Source columns are handled in blocks of 64 (one 64-bit word per vertex and
+// block); a unit is a (block, vertex) pair, its key block * m + vertex.
+//  * V: per unit, the columns that have reached the vertex (the reference's
+//    Numsp pattern); F: per unit, the columns whose search is at the vertex in
+//    the level being swept, in three buffers used in turn, so that one level's
+//    kernel reads one, writes the next and clears the one before;
+//  * S: m x ns FP64 path counts, W: m x ns FP64 (1 + delta) / sigma, both
+//    read only where a bit of F says there is a value;
+//  * rows: per distance, the units first reached there with their columns (the
+//    reference's Sigmas[d]); the units of heavy vertices (more than `piece`
+//    out-neighbours) from the other end of the same arrays, cut into tasks.
 // Forward level (Front<!Numsp> = A^T * Front, matrix_la.h:800-891 fused with
-// add_nointersect, matrix_la.h:337-372): one warp per unvisited vertex pulls
-// the frontier entries of its in-neighbours into a shared-memory accumulator
-// over the sources, skips sources already visited, and appends the new
-// frontier row to the store (stream compaction by atomic reservation).
-// Backward level k (betweenness_centrality.h:203-218): W<S[k]> = bcu/sigma,
-// then for every row of S[k-1]: acc = A * W restricted to its sources,
-// bcu += acc * sigma, and bc[v] += acc * sigma (the final row sum,
-// betweenness_centrality.h:220-228, accumulated as it is produced).
-// Both sweeps run as device loops (CUDA-graph WHILE nodes).
+// add_nointersect, matrix_la.h:337-372): a pulling warp takes the units that
+// some column has not reached, ANDs the words of 32 in-neighbours with the
+// missing columns, transposes the words across the warp, and every lane sums
+// the counts of the neighbours that hold its two columns; a level with a
+// small frontier pushes along the out-edges instead.
+// Backward level k (betweenness_centrality.h:203-218): for the rows at
+// distance k - 1, acc = A * W over the neighbours at distance k (the same
+// gather over W), delta = acc * sigma, bc[v] += sum of delta (the final row
+// sum, betweenness_centrality.h:220-228, accumulated as it is produced), and
+// W = (1 + delta) / sigma = 1 / sigma + acc for the next level.
+// Both sweeps run as device loops (CUDA-graph WHILE nodes, captured once per
+// context): two kernels per forward level, one per backward level.
 //
-// Source columns. Column j of the state holds source j, except in a batch
-// over the block-diagonal union of several graphs: there column j holds the
+// What bounds it: GB300 adds two FP64 lanes per clock and SM whether one lane
+// of a warp is active or all are (64 sources on R-MAT 20 need 2.8e8 additions
+// each way, 0.55 ms at that rate with full warps), and the chain of dependent
+// gathers per 32 neighbours (column, word, value). In the largest forward
+// level the FP64 pipe is busy 65 % of the time at 28 % of its lanes. So the
+// additions are packed: a lane walks only the neighbours that hold its column,
+// and the columns found share out the lanes (bc_gather). 64 sources on R-MAT
+// 20, one call: 38.0-42.1 ms before (every frontier entry a shared-memory FP64
+// atomic, 20.5 ms forward; every column of every neighbour that any source had
+// at the level, 17.1 ms backward; 1.6 ms to set and clear W), 16.8 ms with
+// each lane summing two fixed columns and the units dealt out in advance, 10.5
+// ms with warps taking units as they go and heavy vertices in warp-sized
+// pieces, 8.0 ms with the columns sharing out the lanes (forward levels 0.04,
+// 0.33, 2.34, 0.62, 0.51, 0.03 ms, backward 0.05, 0.40, 1.27, 1.97, 0.15 ms).
+//
+// Batches over the block-diagonal union of several graphs: column j holds the
 // j-th source of every graph at once. A source only reaches the vertices of
 // its own graph, so each (vertex, column) pair still belongs to one source,
 // and the state is (union vertices) x (largest source count of a graph)
@@ -37,84 +58,146 @@ namespace ga {
 constexpr int kBcThreads = 256;
 constexpr int kBcWarps = kBcThreads / 32;
 constexpr int kBcMaxSources = 1024;
+// A vertex with more than `piece` neighbours is heavy: its list is cut into
+// pieces that separate warps sum; the last piece to finish adds them up, in
+// order (a hub of R-MAT 20 has 64,000 neighbours: one CTA would take longer
+// than the rest of the level). Dense graphs take longer pieces, so that the
+// partial sums stay small beside the graph.
+constexpr int kBcPiece = 512;
+constexpr int kBcPieceDense = 2048;   // more than kBcDense entries per vertex
+constexpr int kBcDense = 256;
+constexpr int kBcLoads = 4;   // values a lane has in flight (8 were 8 % slower: registers spill)
+// Units (forward) and rows (backward) that a warp takes at a time: at most
+// these, fewer where a level has not four takes per warp of the grid. A take's
+// rows are reserved with one atomic, its scores summed together.
+constexpr int kBcUnits = 16;
+constexpr int kBcRows = 8;
 
 struct BcState {
-    int32_t d;        // current forward level
-    int32_t depth;    // number of non-empty levels (forward result)
-    int32_t k;        // backward level
+    int32_t d;        // forward: distance of the frontier; then the largest distance
+    int32_t k;        // backward: distance whose W is set
     int32_t done;
-    // entries appended so far (store size, low 32 bits) and frontier rows
-    // appended so far (high 32 bits): one atomic reserves both
-    unsigned long long er;
-    int32_t overflow;
-    int32_t mode;          // forward direction of the current level: 0 pull, 1 push
-    int32_t ntouched;      // vertices reached by the current push level
-    int32_t stalled;       // a bulk copy of the backward sweep did not complete in time
-    int32_t nhrows;        // backward level: heavy rows listed in hrows
-    unsigned long long cur_work, next_work;  // sum over frontier rows of entries x out-degree
+    int32_t mode;     // forward direction of the level: 0 pull, 1 push
+    int32_t nrows, nhrows, nhtasks;  // lists' ends
+    int32_t ntouched; // push level: units reached
+    int32_t nchunk;   // pieces of the heavy in-neighbour lists
+    int32_t flags;    // 1 self-loop, 8 source out of range, 16 repeated source
+    uint32_t blocks;  // blocks of the level's last kernel that have finished
+    int32_t next;     // next task of the level (warps take tasks as they go)
+    unsigned long long cur_work, next_work;  // sum over frontier rows of columns x out-degree
 };
 
 struct BcArgs {
     const int32_t* atr; const int32_t* atc; const double* atv;  // A^T (in-neighbours)
     const int32_t* ar; const int32_t* ac; const double* av;     // A (out-neighbours)
-    int64_t m;
-    int ns, words;                                              // source columns, 32-bit words per vertex
-    int nsrc;                                                   // sources (level-0 entries)
+    int64_t m, nnz;
+    int ns, nblk;                  // source columns, blocks of 64
+    int piece;                     // neighbours per piece of a heavy vertex
+    int nsrc;
     const int32_t* sources;
-    const int32_t* scol;                                        // column of each source (nullptr: its index)
+    const int32_t* scol;           // column of each source (nullptr: its index)
     BcState* st;
-    int32_t* level_rows;    // level_rows[d] = first row of level d
-    int32_t* cur_start[2];  // per vertex, per parity: first entry of its frontier row
-    int32_t* cur_len[2];
-    uint32_t* vbits;        // m x words
-    int32_t* vcnt;          // sources that reached each vertex
-    int32_t* es; double* ev; double* ed;  // store: source, sigma, bcu
-    int32_t* rv; int32_t* rs; int32_t* rl; // rows: vertex, start, length
-    int64_t cap_entries, cap_rows;
-    double* W;              // m x ns
-    uint32_t* inlvl;        // m bits: vertex has entries at the level being swept
+    unsigned long long* V;         // nblk x m
+    unsigned long long* F[3];      // nblk x m each
+    double* S; double* W;          // m x ns
+    int32_t* rkey; unsigned long long* rmask;  // rows; heavy vertices' from the end (heavy_row)
+    int64_t rlast;                             // last place of the rows
+    int32_t* hfirst;                           // heavy rows: first task
+    int2* htask;                   // (heavy row, piece)
+    int32_t *lrow, *lhrow, *ltask; // per distance: first row, heavy row, task
+    int4* chunk;                   // forward: pieces of the heavy in-lists (vertex, piece, first place, pieces)
+    double* part; unsigned long long* pmask; int32_t* pdone;    // per place: partial sums, columns, arrivals
+    int32_t* tlist;                // push level: units reached, in order of first touch
     double* bc;
-    const int32_t* heavy_in;  // vertices with more than kBcHeavyDeg in-neighbours
-    int nheavy_in;
-    int64_t nnz;            // stored entries of A (direction choice)
-    uint32_t* tbits;        // push levels: m x words, sources that reached each vertex
-    int32_t* tlist;         // push levels: vertices reached, in order of first touch
-    int32_t* tmark;         // push levels: vertex already listed
-    int32_t* hrows;         // backward level: rows of S[k-1] whose vertex has more than kBcHeavyDeg neighbours
 };
 
 // A level pushes (frontier rows scatter along their out-edges with global
-// atomics) when its frontier's work, entries x out-degree, is below
-// nnz / kBcPushDiv; otherwise every unvisited vertex pulls (no atomics on
-// global memory, but a pass over all in-edges).
-constexpr unsigned long long kBcPushDiv = 8;
+// atomics) when its frontier's work, columns x out-degree, is below
+// kBcPushMul * nnz; otherwise every unit with a missing column pulls (no
+// atomics on global memory, but a pass over all in-edges). R-MAT 20, 64
+// sources: at a work of 0.14 nnz pushing took 331 us and pulling 1,640 us, at
+// 1.2 nnz 506 and 803 us; at 18 nnz pulling took 2.3 ms and pushing would
+// issue 5.8e8 atomics.
+constexpr unsigned long long kBcPushMul = 2;
 
-__global__ void k_bc_init(BcArgs p) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nsrc; j += gridDim.x * blockDim.x) {
-        int v = p.sources[j];
-        const int c = p.scol ? p.scol[j] : j;
-        p.es[j] = c;
-        p.ev[j] = 1.0;
-        p.ed[j] = 1.0;
-        atomicOr(&p.vbits[(size_t)v * p.words + (c >> 5)], 1u << (c & 31));
-        atomicAdd(&p.vcnt[v], 1);
-        p.cur_start[0][v] = j;
-        p.cur_len[0][v] = 1;
-        atomicAdd(&p.st->next_work, (unsigned long long)(p.ar[v + 1] - p.ar[v]));
+__device__ __forceinline__ int64_t heavy_row(const BcArgs& p, int64_t h) { return p.rlast - h; }
+
+__device__ __forceinline__ unsigned long long bc_columns(const BcArgs& p, int blk) {
+    const int n = p.ns - blk * 64;
+    return n >= 64 ? ~0ull : (1ull << n) - 1ull;
+}
+
+// Vertex and block of a key.
+__device__ __forceinline__ int bc_block(const BcArgs& p, int32_t key, int32_t& v) {
+    if (p.nblk == 1) {
+        v = key;
+        return 0;
+    }
+    const int blk = (int)(key / (int32_t)p.m);
+    v = key - blk * (int32_t)p.m;
+    return blk;
+}
+
+// Appends the row (key, mask) of vertex v to the rows found so far; lanes with
+// mask 0 have none. Called by whole warps. Returns the lane's row's work.
+__device__ __forceinline__ unsigned long long bc_append(const BcArgs& p, int32_t key, int32_t v,
+                                                        unsigned long long mask) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int32_t od = mask ? p.ar[v + 1] - p.ar[v] : 0;
+    const bool light = mask != 0ull && od <= p.piece;
+    const unsigned lm = __ballot_sync(FULL, light);
+    int32_t base = 0;
+    if (lm && lane == 0) base = atomicAdd(&p.st->nrows, __popc(lm));
+    base = __shfl_sync(FULL, base, 0);
+    if (light) {
+        const int32_t r = base + __popc(lm & ((1u << lane) - 1u));
+        p.rkey[r] = key;
+        p.rmask[r] = mask;
+    } else if (mask) {
+        const int32_t h = atomicAdd(&p.st->nhrows, 1);
+        const int32_t n = (od + p.piece - 1) / p.piece;
+        const int32_t f = atomicAdd(&p.st->nhtasks, n);
+        p.rkey[heavy_row(p, h)] = key;
+        p.rmask[heavy_row(p, h)] = mask;
+        p.hfirst[h] = f;
+        for (int32_t c = 0; c < n; ++c) p.htask[f + c] = make_int2(h, c);
+    }
+    return (unsigned long long)__popcll(mask) * (unsigned long long)od;
+}
+
+// Per vertex (one thread): a self-loop (rows are sorted, so a binary search
+// finds it) and the pieces of heavy in-neighbour lists.
+__global__ void k_bc_scan_vertices(BcArgs p) {
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < p.m; v += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t b = p.ar[v], n = p.ar[v + 1] - b;
+        const int pos = lower_bound_i32(p.ac + b, n, (int32_t)v);
+        if (pos < n && p.ac[b + pos] == (int32_t)v) atomicOr(&p.st->flags, 1);
+        const int32_t in = p.atr[v + 1] - p.atr[v];
+        if (in > p.piece) {
+            const int32_t c = (in + p.piece - 1) / p.piece;
+            const int32_t f = atomicAdd(&p.st->nchunk, c);
+            for (int32_t i = 0; i < c; ++i) p.chunk[f + i] = make_int4((int32_t)v, i, f, c);
+        }
     }
 }
 
-__global__ void k_bc_state_init(BcArgs p) {
-    p.st->d = 0; p.st->depth = 0; p.st->k = 0; p.st->done = 0;
-    p.st->er = (unsigned long long)p.nsrc; p.st->overflow = 0;
-    p.st->mode = 0; p.st->ntouched = 0; p.st->stalled = 0; p.st->nhrows = 0;
-    p.st->cur_work = 0; p.st->next_work = 0;
-    p.level_rows[0] = 0;
+// The sources are in range and distinct (seen: one bit per vertex, cleared).
+__global__ void k_bc_check_sources(BcArgs p, uint32_t* __restrict__ seen) {
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nsrc; j += gridDim.x * blockDim.x) {
+        const int32_t v = p.sources[j];
+        if (v < 0 || (int64_t)v >= p.m) {
+            atomicOr(&p.st->flags, 8);
+            continue;
+        }
+        const uint32_t bit = 1u << (v & 31);
+        if (atomicOr(&seen[v >> 5], bit) & bit) atomicOr(&p.st->flags, 16);
+    }
 }
 
 // Batches with packed columns: on the vertices of graph g (union rows
 // [voff[g], voff[g+1])), the columns at and above its source count are
-// marked visited, so no entry is ever made there and the vertex counts as
+// marked visited, so no value is ever made there and the vertex counts as
 // reached by every column once its own sources have reached it.
 __global__ void k_bc_previsit(BcArgs p, const int64_t* __restrict__ voff, const int32_t* __restrict__ gsrc,
                               int64_t count) {
@@ -125,653 +208,561 @@ __global__ void k_bc_previsit(BcArgs p, const int64_t* __restrict__ voff, const 
             if (voff[mid] <= v) lo = mid; else hi = mid;
         }
         const int have = gsrc[lo];
-        for (int w = 0; w < p.words; ++w) {
-            const int c0 = w * 32;
-            uint32_t bits = 0u;
-            if (have <= c0) bits = 0xffffffffu;
-            else if (have < c0 + 32) bits = ~((1u << (have - c0)) - 1u);
-            if (c0 + 32 > p.ns) bits &= (p.ns - c0 >= 32) ? 0xffffffffu : ((1u << (p.ns - c0)) - 1u);
-            p.vbits[(size_t)v * p.words + w] = bits;
+        for (int b = 0; b < p.nblk; ++b) {
+            const int n = have - b * 64;
+            const unsigned long long own = n <= 0 ? 0ull : n >= 64 ? ~0ull : (1ull << n) - 1ull;
+            p.V[(int64_t)b * p.m + v] = bc_columns(p, b) & ~own;
         }
-        p.vcnt[v] = p.ns - have;
     }
 }
 
-// Level start: the frontier's work decides the direction.
-__global__ void k_bc_level_begin(BcArgs p) {
+// The sources' rows: distance 0, one path. One block; nothing when a check
+// failed (the loops then end at once).
+__global__ void k_bc_init(BcArgs p) {
     BcState* st = p.st;
-    if (st->done) return;
-    st->cur_work = st->next_work;
-    st->next_work = 0;
-    st->ntouched = 0;
-    st->mode = st->cur_work * kBcPushDiv < (unsigned long long)p.nnz ? 1 : 0;
-}
-
-// Vertices with more than kBcHeavyDeg neighbours are handled by a whole CTA
-// (their neighbour lists are split over the CTA's warps).
-constexpr int kBcHeavyDeg = 1024;
-
-// Frontier entries of the in-neighbours in group [g, g+32) of vertex v,
-// flattened over the warp (segment found by ballot/OR + popcount), added to
-// acc for sources v has not reached yet.
-template <bool UNIT>
-__device__ __forceinline__ void bc_pull_group(const BcArgs& p, const int32_t* curS, const int32_t* curL, int32_t g,
-                                              int32_t ae, const uint32_t* vis, double* acc, uint32_t* touched,
-                                              int* s_incl, int* s_off, double* s_a) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int32_t t = g + lane;
-    int len = 0, bs = 0;
-    double a = 0.0;
-    if (t < ae) {
-        const int32_t u = __ldg(p.atc + t);
-        len = curL[u];
-        if (len) {
-            bs = curS[u];
-            a = UNIT ? 1.0 : __ldg(p.atv + t);
-        }
-    }
-    const unsigned nz = __ballot_sync(FULL, len > 0);
-    if (nz == 0) return;
-    const int nseg = __popc(nz);
-    const int incl = warp_incl_scan(len);
-    const int total = __shfl_sync(FULL, incl, 31);
-    if (len > 0) {
-        const int rank = __popc(nz & ((1u << lane) - 1u));
-        s_incl[rank] = incl;
-        s_off[rank] = bs - (incl - len);
-        s_a[rank] = a;
-    }
-    __syncwarp();
-    const int my_end = lane < nseg ? s_incl[lane] - 1 : INT32_MAX;
-    const unsigned lt = (1u << lane) - 1u;
-    int q_base = 0;
-    for (int base = 0; base < total; base += 32) {
-        const int e = my_end - base;
-        const unsigned bm = __reduce_or_sync(FULL, (e >= 0 && e < 32) ? (1u << e) : 0u);
-        const int x = base + lane;
-        if (x < total) {
-            const int q = q_base + __popc(bm & lt);
-            const int32_t j = x + s_off[q];
-            const int s = p.es[j];
-            if (!(vis[s >> 5] & (1u << (s & 31)))) {
-                atomicAdd(&acc[s], s_a[q] * p.ev[j]);
-                atomicOr(&touched[s >> 5], 1u << (s & 31));
+    const bool bad = st->flags != 0;
+    if (!bad) {
+        unsigned long long work = 0;
+        for (int j0 = 0; j0 < p.nsrc; j0 += blockDim.x) {
+            const int j = j0 + threadIdx.x;
+            int32_t v = 0, key = 0;
+            unsigned long long mask = 0;
+            if (j < p.nsrc) {
+                v = p.sources[j];
+                const int c = p.scol ? p.scol[j] : j;
+                mask = 1ull << (c & 63);
+                key = (int32_t)((int64_t)(c >> 6) * p.m + v);
+                p.S[(size_t)v * p.ns + c] = 1.0;
+                // sources are distinct vertices: the unit is this source's alone
+                p.V[key] |= mask;
+                p.F[0][key] = mask;
             }
+            work += bc_append(p, key, v, mask);
         }
-        q_base += __popc(bm);
+        work = warp_sum<unsigned long long>(work);
+        if ((threadIdx.x & 31) == 0 && work) atomicAdd(&st->cur_work, work);
     }
-    __syncwarp();
-}
-
-// Appends v's new frontier row (its touched sources, in source order) by one
-// warp; resets acc/touched. Lane 0 adds the row's next-level work (entries x
-// out-degree) to `work`, which the caller adds to the level total once.
-__device__ __forceinline__ void bc_emit_row(const BcArgs& p, int64_t v, int32_t* nxtS, int32_t* nxtL,
-                                            const uint32_t* vis, double* acc, uint32_t* touched,
-                                            unsigned long long& work) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const uint32_t word = lane < p.words ? touched[lane] : 0u;
-    const int cnt = __popc(word);
-    const int excl = warp_incl_scan(cnt) - cnt;
-    const int count = __shfl_sync(FULL, excl + cnt, 31);
-    if (count == 0) {
-        if (lane == 0) nxtL[v] = 0;
-        return;
-    }
-    int start = 0;
-    if (lane == 0) {
-        const unsigned long long old = atomicAdd(&p.st->er, (1ull << 32) | (unsigned long long)count);
-        start = (int)(old & 0xffffffffull);
-        const int r = (int)(old >> 32);
-        if ((int64_t)start + count > p.cap_entries || (int64_t)r >= p.cap_rows) {
-            atomicExch(&p.st->overflow, 1);
-            start = -1;
-        } else {
-            p.rv[r] = (int32_t)v; p.rs[r] = start; p.rl[r] = count;
-            p.vcnt[v] += count;
-            work += (unsigned long long)count * (unsigned long long)(p.ar[v + 1] - p.ar[v]);
-        }
-        nxtS[v] = start;
-        nxtL[v] = start < 0 ? 0 : count;
-    }
-    start = __shfl_sync(FULL, start, 0);
-    if (start >= 0 && word) {
-        int pos = start + excl;
-        uint32_t w = word;
-        while (w) {
-            const int b = __ffs(w) - 1;
-            w &= w - 1;
-            const int s = lane * 32 + b;
-            p.es[pos] = s;
-            p.ev[pos] = acc[s];
-            p.ed[pos] = 1.0;
-            ++pos;
-        }
-        p.vbits[(size_t)v * p.words + lane] = vis[lane] | word;
-    }
-    __syncwarp();
-    for (int s = lane; s < p.ns; s += 32) acc[s] = 0.0;
-    if (lane < p.words) touched[lane] = 0u;
-    __syncwarp();
-}
-
-// One forward level: dynamic per-warp shared memory = acc[ns] doubles +
-// touched[words] + visited[words] + 32-entry flattening scratch. Heavy
-// vertices first, one per CTA with all warps pulling into warp 0's
-// accumulator; then the rest, one per warp.
-template <bool UNIT>
-__global__ void __launch_bounds__(kBcThreads) k_bc_forward(BcArgs p) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const size_t per_warp = ((size_t)p.ns * sizeof(double) + 2 * (size_t)p.words * sizeof(uint32_t) +
-                             32 * (2 * sizeof(int) + sizeof(double)) + 15) & ~(size_t)15;
-    auto region = [&](int w, double*& acc, uint32_t*& touched, uint32_t*& vis, int*& s_incl, int*& s_off,
-                      double*& s_a) {
-        unsigned char* base = smem + w * per_warp;
-        acc = reinterpret_cast<double*>(base);
-        touched = reinterpret_cast<uint32_t*>(base + (size_t)p.ns * sizeof(double));
-        vis = touched + p.words;
-        s_incl = reinterpret_cast<int*>(vis + p.words);
-        s_off = s_incl + 32;
-        s_a = reinterpret_cast<double*>(s_off + 32);
-    };
-    double* acc; uint32_t* touched; uint32_t* vis; int* s_incl; int* s_off; double* s_a;
-    region(wid, acc, touched, vis, s_incl, s_off, s_a);
-    double* acc0; uint32_t* touched0; uint32_t* vis0; int* i0; int* o0; double* a0;
-    region(0, acc0, touched0, vis0, i0, o0, a0);
-
-    if (p.st->done || p.st->mode != 0) return;
-    unsigned long long work = 0;  // lane 0: next-level work of the rows this warp emits
-    const int d = p.st->d;
-    const int par = d & 1;
-    const int32_t* curS = p.cur_start[par];
-    const int32_t* curL = p.cur_len[par];
-    int32_t* nxtS = p.cur_start[par ^ 1];
-    int32_t* nxtL = p.cur_len[par ^ 1];
-
-    for (int s = lane; s < p.ns; s += 32) acc[s] = 0.0;
-    if (lane < p.words) touched[lane] = 0u;
     __syncthreads();
-
-    // heavy vertices: the CTA's warps split the in-neighbours
-    for (int h = blockIdx.x; h < p.nheavy_in; h += gridDim.x) {
-        const int64_t v = p.heavy_in[h];
-        const bool active = p.vcnt[v] < p.ns;  // uniform over the CTA
-        if (active) {
-            if (wid == 0 && lane < p.words) vis0[lane] = p.vbits[(size_t)v * p.words + lane];
-            __syncthreads();
-            const int32_t ab = p.atr[v], ae = p.atr[v + 1];
-            for (int32_t g = ab + wid * 32; g < ae; g += kBcWarps * 32)
-                bc_pull_group<UNIT>(p, curS, curL, g, ae, vis0, acc0, touched0, s_incl, s_off, s_a);
-            __syncthreads();
-            if (wid == 0) bc_emit_row(p, v, nxtS, nxtL, vis0, acc0, touched0, work);
-        } else if (threadIdx.x == 0) {
-            nxtL[v] = 0;
-        }
-        __syncthreads();
-    }
-
-    // the rest: warp w takes the vertices w, w + W, w + 2W, ... (W warps in
-    // the grid), 32 of them at a time: each lane checks one (heavy vertices
-    // were done above; one that every source has reached, or without
-    // in-neighbours, gets an empty next row), then the warp pulls the others
-    // one by one
-    const unsigned FULL = 0xffffffffu;
-    const int64_t warps = (int64_t)gridDim.x * kBcWarps;
-    for (int64_t v0 = (int64_t)blockIdx.x * kBcWarps + wid; v0 < p.m; v0 += warps * 32) {
-        const int64_t vl = v0 + (int64_t)lane * warps;
-        int32_t lab = 0, lae = 0;
-        bool act = false;
-        if (vl < p.m) {
-            lab = p.atr[vl];
-            lae = p.atr[vl + 1];
-            if (lae - lab <= kBcHeavyDeg) {
-                act = lae > lab && p.vcnt[vl] < p.ns;
-                if (!act) nxtL[vl] = 0;
-            }
-        }
-        unsigned am = __ballot_sync(FULL, act);
-        while (am) {
-            const int src = __ffs(am) - 1;
-            am &= am - 1;
-            const int64_t v = v0 + (int64_t)src * warps;
-            const int32_t ab = __shfl_sync(FULL, lab, src), ae = __shfl_sync(FULL, lae, src);
-            if (lane < p.words) vis[lane] = p.vbits[(size_t)v * p.words + lane];
-            __syncwarp();
-            for (int32_t g = ab; g < ae; g += 32)
-                bc_pull_group<UNIT>(p, curS, curL, g, ae, vis, acc, touched, s_incl, s_off, s_a);
-            bc_emit_row(p, v, nxtS, nxtL, vis, acc, touched, work);
-        }
-    }
-    if (lane == 0 && work) atomicAdd(&p.st->next_work, work);
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    p.lrow[0] = 0;
+    p.lhrow[0] = 0;
+    p.ltask[0] = 0;
+    p.lrow[1] = *(volatile int32_t*)&st->nrows;
+    p.lhrow[1] = *(volatile int32_t*)&st->nhrows;
+    p.ltask[1] = *(volatile int32_t*)&st->nhtasks;
+    st->done = bad;
+    const unsigned long long work = *(volatile unsigned long long*)&st->cur_work;
+    st->mode = work < kBcPushMul * (unsigned long long)p.nnz ? 1 : 0;
 }
 
-// Push level, one frontier row (vertex u, entries [e0, e0+len)) and the
-// out-neighbours [t0, t1) of u, lanes over neighbours 32 at a time (group
-// stride `step`): for every entry (source s, sigma) and neighbour w that s has
-// not reached, W[w][s] += A[u][w] * sigma, and w's touched bit for s is set;
-// the first touch of w lists it.
-template <bool UNIT>
-__device__ __forceinline__ void bc_push_row(const BcArgs& p, int32_t e0, int32_t len, int32_t t0, int32_t t1,
-                                            int32_t step) {
+// The columns of a 64-bit word side by side: s_col[i] = its i-th set bit.
+__device__ __forceinline__ void bc_list_columns(unsigned long long word, uint8_t* s_col) {
     const int lane = threadIdx.x & 31;
-    for (int32_t g = t0; g < t1; g += step) {
-        const int32_t t = g + lane;
-        if (t >= t1) continue;
-        const int32_t w = __ldg(p.ac + t);
-        const double a = UNIT ? 1.0 : __ldg(p.av + t);
-        const uint32_t* vis = p.vbits + (size_t)w * p.words;
-        for (int e = 0; e < len; ++e) {
-            const int s = p.es[e0 + e];
-            const uint32_t bit = 1u << (s & 31);
-            if (vis[s >> 5] & bit) continue;
-            atomicAdd(&p.W[(size_t)w * p.ns + s], a * p.ev[e0 + e]);
-            const uint32_t old = atomicOr(&p.tbits[(size_t)w * p.words + (s >> 5)], bit);
-            if (old == 0u && atomicExch(&p.tmark[w], 1) == 0) p.tlist[atomicAdd(&p.st->ntouched, 1)] = w;
-        }
-    }
+    const uint32_t lt = (1u << lane) - 1u, lo = (uint32_t)word, hi = (uint32_t)(word >> 32);
+    if (lo >> lane & 1u) s_col[__popc(lo & lt)] = (uint8_t)lane;
+    if (hi >> lane & 1u) s_col[__popc(lo) + __popc(hi & lt)] = (uint8_t)(32 + lane);
 }
 
-// Frontier items of level d: the sources at level 0, else the rows found
-// while level d-1 ran, [level_rows[d-1], level_rows[d]).
-__device__ __forceinline__ void bc_frontier_item(const BcArgs& p, int d, int64_t it, int32_t& u, int32_t& e0,
-                                                 int32_t& len) {
-    if (d == 0) {
-        u = p.sources[it]; e0 = (int32_t)it; len = 1;
-    } else {
-        const int64_t r = p.level_rows[d - 1] + it;
-        u = p.rv[r]; e0 = p.rs[r]; len = p.rl[r];
-    }
-}
-
-template <bool UNIT>
-__global__ void __launch_bounds__(kBcThreads) k_bc_push(BcArgs p) {
-    const BcState* st = p.st;
-    if (st->done || st->mode != 1) return;
-    const int d = st->d;
-    const int wid = threadIdx.x >> 5;
-    const int64_t items = d == 0 ? p.nsrc : (int64_t)p.level_rows[d] - p.level_rows[d - 1];
-    // rows of high-degree vertices: the CTA's warps split the neighbours
-    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
-        int32_t u, e0, len;
-        bc_frontier_item(p, d, it, u, e0, len);
-        const int32_t ab = p.ar[u], ae = p.ar[u + 1];
-        if (ae - ab <= kBcHeavyDeg) continue;
-        bc_push_row<UNIT>(p, e0, len, ab + wid * 32, ae, kBcWarps * 32);
-    }
-    const int64_t warps = (int64_t)gridDim.x * kBcWarps;
-    for (int64_t it = (int64_t)blockIdx.x * kBcWarps + wid; it < items; it += warps) {
-        int32_t u, e0, len;
-        bc_frontier_item(p, d, it, u, e0, len);
-        const int32_t ab = p.ar[u], ae = p.ar[u + 1];
-        if (ae - ab > kBcHeavyDeg) continue;
-        bc_push_row<UNIT>(p, e0, len, ab, ae, 32);
-    }
-}
-
-// Push level, after the scatter: every vertex's next-frontier length is
-// cleared, then each reached vertex appends its row (one warp each) from its
-// W row and touched bits, which are reset.
-__global__ void k_bc_push_clear(BcArgs p) {
-    const BcState* st = p.st;
-    if (st->done || st->mode != 1) return;
-    int32_t* nxtL = p.cur_len[(st->d & 1) ^ 1];
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < p.m; v += (int64_t)gridDim.x * blockDim.x)
-        nxtL[v] = 0;
-}
-
-__global__ void __launch_bounds__(kBcThreads) k_bc_push_emit(BcArgs p) {
-    const BcState* st = p.st;
-    if (st->done || st->mode != 1) return;
-    const int lane = threadIdx.x & 31;
-    const int par = st->d & 1;
-    int32_t* nxtS = p.cur_start[par ^ 1];
-    int32_t* nxtL = p.cur_len[par ^ 1];
-    const int n = st->ntouched;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    unsigned long long work = 0;  // lane 0: next-level work of the rows this warp emits
-    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        const int32_t w = p.tlist[i];
-        bc_emit_row(p, w, nxtS, nxtL, p.vbits + (size_t)w * p.words, p.W + (size_t)w * p.ns,
-                    p.tbits + (size_t)w * p.words, work);
-        if (lane == 0) p.tmark[w] = 0;
-    }
-    if (lane == 0 && work) atomicAdd(&p.st->next_work, work);
-}
-
-__global__ void k_bc_forward_finalize(BcArgs p, LoopCtl ctl) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    BcState* st = p.st;
-    bool more = false;
-    if (!st->done) {
-        const int d = st->d;
-        const int32_t rows = (int32_t)(st->er >> 32);
-        if (st->overflow || rows == p.level_rows[d]) {
-            st->depth = d;
-            st->done = 1;
-        } else {
-            p.level_rows[d + 1] = rows;
-            st->d = d + 1;
-            if ((int64_t)st->d > p.m) { st->depth = st->d; st->done = 1; }
-            else more = true;
-        }
-    }
-    if (!more) st->k = st->depth - 1;
-    loop_continue(ctl, more);
-}
-
-// W<S[k]> = bcu / sigma and mark the level's vertices (set = true), or clear
-// both again (set = false).
-__global__ void k_bc_set_w(BcArgs p, bool set) {
-    const int k = p.st->k;
-    if (k < 1) return;
-    const int lane = threadIdx.x & 31;
-    const int32_t r0 = p.level_rows[k], r1 = p.level_rows[k + 1];
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t r = r0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < r1; r += warps) {
-        const int32_t v = p.rv[r], s0 = p.rs[r], n = p.rl[r];
-        double* wrow = p.W + (size_t)v * p.ns;
-        for (int e = lane; e < n; e += 32) {
-            int s = p.es[s0 + e];
-            wrow[s] = set ? p.ed[s0 + e] / p.ev[s0 + e] : 0.0;
-        }
-        if (lane == 0) {
-            if (set) atomicOr(&p.inlvl[v >> 5], 1u << (v & 31));
-            else atomicAnd(&p.inlvl[v >> 5], ~(1u << (v & 31)));
-        }
-    }
-    // before the backward level: the heavy rows of S[k-1], listed so that
-    // the CTAs of the backward kernel can share them out
-    if (set) {
-        const int32_t q0 = p.level_rows[k - 1];
-        for (int64_t r = q0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < r0;
-             r += (int64_t)gridDim.x * blockDim.x) {
-            const int32_t v = p.rv[r];
-            if (p.ar[v + 1] - p.ar[v] > kBcHeavyDeg) p.hrows[atomicAdd(&p.st->nhrows, 1)] = (int32_t)r;
-        }
-    }
-}
-
-constexpr int kBcPer = 4;  // row entries per lane per pass of the backward sweep
-
-// How the backward sweep reads the W rows of a row's level-k neighbours
-// (GA_OPT_BC_BACKWARD): 0 gathers of up to kBcHits neighbours' rows issued
-// together; 1 bulk copies of whole W rows into shared memory, two batches of
-// kBcHits rows in flight per warp (needs an even source count of at most
-// kBcBulkMaxCols and a 16-byte aligned W); 2 one neighbour at a time.
-enum { kBcBwdGather = 0, kBcBwdBulk = 1, kBcBwdSingle = 2 };
-constexpr int kBcHits = 4;
-constexpr int kBcBulkMaxCols = 128;
-constexpr long long kBcWaitCycles = 2000000000ll;  // about a second at 2 GHz
-
-// The hit lanes of one group (bit mask `hits`) in ascending order, up to
-// kBcHits of them: their neighbours and values, broadcast to the warp.
-__device__ __forceinline__ int bc_take_hits(unsigned& hits, int32_t w, double a, int32_t (&ws)[kBcHits],
-                                            double (&as)[kBcHits]) {
-    const unsigned FULL = 0xffffffffu;
-    int n = 0;
-#pragma unroll
-    for (int h = 0; h < kBcHits; ++h) {
-        ws[h] = -1;
-        as[h] = 0.0;
-        if (hits) {  // warp-uniform
-            const int src = __ffs(hits) - 1;
-            hits &= hits - 1;
-            ws[h] = __shfl_sync(FULL, w, src);
-            as[h] = __shfl_sync(FULL, a, src);
-            n = h + 1;
-        }
-    }
-    return n;
-}
-
-// Per-warp state of the bulk form: two stages of kBcHits W rows in shared
-// memory, one barrier per stage and its expected parity.
-struct BcRing {
-    double* rows;    // 2 * kBcHits rows of ns doubles
-    uint64_t* bar;   // 2 barriers
-    uint32_t phase;  // bit s: parity the next wait on stage s expects
-    bool ok;         // false once a wait ran out
+// Shared memory of one warp for the sums over its neighbours.
+struct BcWarp {
+    int32_t row[32];   // the group's neighbours: first index of their values
+    uint8_t col[64];   // columns side by side
 };
 
-// acc[u] += sum over out-neighbours t in [t0, t1) step `stride` (groups of
-// 32 fetched together, level-k neighbours picked by ballot) of
-// A[v][w] * W[w][s[u]]. The neighbours' contributions are added in the same
-// order (ascending t) in every mode.
-template <bool UNIT, int MODE>
-__device__ __forceinline__ void bc_push_range(const BcArgs& p, int32_t t0, int32_t t1, int32_t stride,
-                                              const int (&s)[kBcPer], double (&acc)[kBcPer], BcRing& ring) {
+// Sums over neighbours [t0, t1): for every column c that some neighbour w has
+// in bits[w] & need, the sum of X[w * ns + c] (times the edge's value) over
+// those w. Returns these columns; the lane holds the sums acc0 of column c0
+// and acc1 of column c1 (-1: none).
+//
+// A first pass over the words finds the columns, which then share out the
+// lanes: one column per lane and list (two lists above 32 columns), or, with
+// at most 16 columns, 2 to 32 lanes per column, each with its share of the
+// neighbours. The neighbours are visited 32 at a time: the words transposed
+// across the warp give each lane the list of neighbours that hold its column,
+// and the warp takes as many steps as the longest list.
+template <bool UNIT>
+__device__ __forceinline__ unsigned long long bc_gather(const int32_t* __restrict__ col,
+                                                        const double* __restrict__ val, int32_t t0, int32_t t1,
+                                                        const unsigned long long* bits, const double* X, int ns,
+                                                        unsigned long long need, BcWarp& sh, double* s_a,
+                                                        double& acc0, double& acc1, int& c0, int& c1) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    // bulk form: the batch whose copies are in flight
-    int pend_n = 0, pend_stage = 0, next_stage = 0;
-    double pend_a[kBcHits];
-    auto consume = [&](int stage, int n, const double (&as)[kBcHits]) {
-        const bool ok = mbar_wait(ring.bar + stage, (ring.phase >> stage) & 1u, kBcWaitCycles);
-        ring.phase ^= 1u << stage;
-        if (!ok) {
-            if (lane == 0) atomicExch(&p.st->stalled, 1);
-            ring.ok = false;
-            return;
-        }
-        const double* base = ring.rows + (size_t)stage * kBcHits * p.ns;
+    acc0 = acc1 = 0.0;
+    c0 = c1 = -1;
+    int32_t t = t0 + lane;
+    int32_t w = t < t1 ? __ldg(col + t) : 0;
+    unsigned long long f = t < t1 ? bits[w] & need : 0ull;
+    unsigned long long any = f;
+#pragma unroll 4
+    for (int32_t g = t + 32; g < t1; g += 32) any |= bits[__ldg(col + g)];
+    any &= need;
+    const uint32_t flo = __reduce_or_sync(FULL, (uint32_t)any), fhi = __reduce_or_sync(FULL, (uint32_t)(any >> 32));
+    const unsigned long long found = ((unsigned long long)fhi << 32) | flo;
+    if (found == 0ull) return 0ull;
+    const int n = __popcll(found);
+    __syncwarp();
+    bc_list_columns(found, sh.col);
+    __syncwarp();
+    const int lg = n > 16 ? 0 : n > 8 ? 1 : n > 4 ? 2 : n > 2 ? 3 : n > 1 ? 4 : 5;
+    if ((lane >> lg) < n) c0 = sh.col[lane >> lg];
+    if (lane + 32 < n) c1 = sh.col[lane + 32];
+    // the lane's share of a group's neighbours
+    uint32_t share = 0;
+    if (c0 >= 0) {
+        share = lg == 0 ? 0xffffffffu : lg == 1 ? 0x55555555u : lg == 2 ? 0x11111111u : lg == 3 ? 0x01010101u
+              : lg == 4 ? 0x00010001u : 1u;
+        share <<= lane & ((1 << lg) - 1);
+    }
+    auto walk = [&](uint32_t mine, int c, double& acc) {
+        while (mine) {
+            double x[kBcLoads], a[kBcLoads];
+            bool on[kBcLoads];
 #pragma unroll
-        for (int h = 0; h < kBcHits; ++h) {
-            if (h >= n) break;
-            const double* row = base + (size_t)h * p.ns;
+            for (int h = 0; h < kBcLoads; ++h) {
+                on[h] = mine != 0u;
+                if (on[h]) {
+                    const int j = __ffs(mine) - 1;
+                    mine &= mine - 1;
+                    x[h] = X[sh.row[j] + c];
+                    if (!UNIT) a[h] = s_a[j];
+                }
+            }
 #pragma unroll
-            for (int u = 0; u < kBcPer; ++u)
-                if (s[u] >= 0) acc[u] += as[h] * row[s[u]];
+            for (int h = 0; h < kBcLoads; ++h)
+                if (on[h]) acc = UNIT ? acc + x[h] : acc + a[h] * x[h];
         }
     };
-    for (int32_t g = t0; g < t1; g += stride) {
-        const int32_t t = g + lane;
-        int32_t w = -1;
-        double a = 0.0;
-        if (t < t1) {
-            const int32_t x = __ldg(p.ac + t);
-            if (__ldg(p.inlvl + (x >> 5)) & (1u << (x & 31))) {
-                w = x;
-                a = UNIT ? 1.0 : __ldg(p.av + t);
-            }
-        }
-        unsigned hits = __ballot_sync(FULL, w >= 0);
-        if (MODE == kBcBwdSingle || (MODE == kBcBwdBulk && !ring.ok)) {
-            while (hits) {
-                const int src = __ffs(hits) - 1;
-                hits &= hits - 1;
-                const int32_t ww = __shfl_sync(FULL, w, src);
-                const double aa = __shfl_sync(FULL, a, src);
-                const double* wrow = p.W + (size_t)ww * p.ns;
-#pragma unroll
-                for (int u = 0; u < kBcPer; ++u)
-                    if (s[u] >= 0) acc[u] += aa * wrow[s[u]];
-            }
-        } else if (MODE == kBcBwdGather) {
-            while (hits) {
-                int32_t ws[kBcHits];
-                double as[kBcHits];
-                bc_take_hits(hits, w, a, ws, as);
-                double x[kBcHits][kBcPer];
-#pragma unroll
-                for (int h = 0; h < kBcHits; ++h)
-#pragma unroll
-                    for (int u = 0; u < kBcPer; ++u)
-                        x[h][u] = (ws[h] >= 0 && s[u] >= 0) ? p.W[(size_t)ws[h] * p.ns + s[u]] : 0.0;
-#pragma unroll
-                for (int h = 0; h < kBcHits; ++h)
-                    if (ws[h] >= 0)
-#pragma unroll
-                        for (int u = 0; u < kBcPer; ++u)
-                            if (s[u] >= 0) acc[u] += as[h] * x[h][u];
-            }
-        } else {
-            while (hits) {
-                int32_t ws[kBcHits];
-                double as[kBcHits];
-                const int n = bc_take_hits(hits, w, a, ws, as);
-                // the stage is free once every lane has read its previous batch
-                __syncwarp();
-                if (lane == 0) {
-                    const uint32_t bytes = (uint32_t)p.ns * sizeof(double);
-                    double* base = ring.rows + (size_t)next_stage * kBcHits * p.ns;
-                    fence_proxy_async_smem();
-                    mbar_arrive_expect_tx(ring.bar + next_stage, bytes * (uint32_t)n);
-#pragma unroll
-                    for (int h = 0; h < kBcHits; ++h)
-                        if (h < n)
-                            bulk_copy_g2s(base + (size_t)h * p.ns, p.W + (size_t)ws[h] * p.ns, bytes,
-                                          ring.bar + next_stage);
-                }
-                if (pend_n) consume(pend_stage, pend_n, pend_a);
-                pend_n = n;
-                pend_stage = next_stage;
-#pragma unroll
-                for (int h = 0; h < kBcHits; ++h) pend_a[h] = as[h];
-                next_stage ^= 1;
-                if (!ring.ok) break;
-            }
-        }
-    }
-    if (MODE == kBcBwdBulk && pend_n) {
-        if (ring.ok) consume(pend_stage, pend_n, pend_a);
-        else (void)mbar_wait(ring.bar + pend_stage, (ring.phase >> pend_stage) & 1u, kBcWaitCycles);
-    }
-}
-
-// Rows of S[k-1]: acc_s = sum_w A[v][w] * W[w][s] over out-neighbours w that
-// sit at level k; bcu += acc*sigma; bc[v] += sum_s acc*sigma. Rows of heavy
-// vertices are shared by all warps of a CTA, the others take one warp.
-template <bool UNIT, int MODE>
-__global__ void __launch_bounds__(kBcThreads, 3) k_bc_backward(BcArgs p) {
-    __shared__ double sacc[kBcMaxSources];
-    __shared__ double s_vsum;
-    extern __shared__ __align__(16) unsigned char bsmem[];
-    const int k = p.st->k;
-    if (k < 1) return;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int32_t r0 = p.level_rows[k - 1], r1 = p.level_rows[k];
-    BcRing ring;
-    ring.rows = nullptr;
-    ring.bar = nullptr;
-    ring.phase = 0;
-    ring.ok = true;
-    if (MODE == kBcBwdBulk) {
-        ring.rows = reinterpret_cast<double*>(bsmem) + (size_t)wid * 2 * kBcHits * p.ns;
-        ring.bar = reinterpret_cast<uint64_t*>(bsmem + (size_t)kBcWarps * 2 * kBcHits * p.ns * sizeof(double)) +
-                   2 * wid;
-        if (lane == 0) {
-            mbar_init(ring.bar, 1);
-            mbar_init(ring.bar + 1, 1);
-            mbar_init_fence();
+    for (int32_t g = t0; g < t1; g += 32) {
+        const int32_t cw = w, ct = t;
+        const unsigned long long cf = f;
+        // the next group's words load while this group is summed
+        t += 32;
+        w = t < t1 ? __ldg(col + t) : 0;
+        f = t < t1 ? bits[w] & need : 0ull;
+        if (__ballot_sync(FULL, cf != 0ull) == 0u) continue;
+        __syncwarp();  // the last group's list is read
+        sh.row[lane] = cw * ns;
+        if (!UNIT && cf) s_a[lane] = __ldg(val + ct);
+        __syncwarp();
+        // bit j: neighbour j holds the column
+        const uint32_t m0 = flo ? warp_transpose_bits((uint32_t)cf) : 0u;
+        const uint32_t m1 = fhi ? warp_transpose_bits((uint32_t)(cf >> 32)) : 0u;
+        uint32_t lo = __shfl_sync(FULL, m0, c0 & 31), hi = __shfl_sync(FULL, m1, c0 & 31);
+        walk((c0 & 32 ? hi : lo) & share, c0, acc0);
+        if (n > 32) {
+            __syncwarp();
+            lo = __shfl_sync(FULL, m0, c1 & 31);
+            hi = __shfl_sync(FULL, m1, c1 & 31);
+            walk(c1 < 0 ? 0u : c1 & 32 ? hi : lo, c1, acc1);
         }
         __syncwarp();
     }
+    for (int o = 1; o < (1 << lg); o <<= 1) acc0 += __shfl_xor_sync(FULL, acc0, o);
+    if (lane & ((1 << lg) - 1)) c0 = -1;  // one lane per column
+    return found;
+}
 
-    // heavy rows (listed by k_bc_set_w), one per CTA at a time: its warps
-    // share the row, each warp taking every 8th group of 32 neighbours
-    const int nh = p.st->nhrows;
-    for (int hr = blockIdx.x; hr < nh; hr += gridDim.x) {
-        const int32_t r = p.hrows[hr];
-        const int32_t v = p.rv[r];
-        const int32_t ab = p.ar[v], ae = p.ar[v + 1];
-        const int32_t e0 = p.rs[r], n = p.rl[r];
-        for (int e = threadIdx.x; e < n; e += blockDim.x) sacc[e] = 0.0;
-        if (threadIdx.x == 0) s_vsum = 0.0;
-        __syncthreads();
-        for (int base = 0; base < n; base += 32 * kBcPer) {
-            int s[kBcPer];
-            double acc[kBcPer];
-#pragma unroll
-            for (int u = 0; u < kBcPer; ++u) {
-                const int e = base + u * 32 + lane;
-                s[u] = e < n ? p.es[e0 + e] : -1;
-                acc[u] = 0.0;
-            }
-            bc_push_range<UNIT, MODE>(p, ab + wid * 32, ae, kBcWarps * 32, s, acc, ring);
-#pragma unroll
-            for (int u = 0; u < kBcPer; ++u) {
-                const int e = base + u * 32 + lane;
-                if (e < n && acc[u] != 0.0) atomicAdd(&sacc[e], acc[u]);
-            }
-        }
-        __syncthreads();
-        double part = 0.0;
-        for (int e = threadIdx.x; e < n; e += blockDim.x) {
-            const double c = sacc[e] * p.ev[e0 + e];
-            p.ed[e0 + e] += c;
-            part += c;
-        }
-        part = warp_sum<double>(part);
-        if (lane == 0 && part != 0.0) atomicAdd(&s_vsum, part);
-        __syncthreads();
-        if (threadIdx.x == 0 && s_vsum != 0.0) atomicAdd(&p.bc[v], s_vsum);
-        __syncthreads();
+// One heavy piece, by a warp: neighbours [t0, t1) of one unit. Its sums go to
+// the piece's place; true when the piece is the last of `count` to arrive at
+// `first`, with the columns of all of them and their sums (acc0: column
+// `lane`, acc1: column 32 + `lane`).
+template <bool UNIT>
+__device__ __forceinline__ bool bc_piece(const BcArgs& p, const int32_t* col, const double* val, int32_t t0,
+                                         int32_t t1, const unsigned long long* bits, const double* X,
+                                         unsigned long long need, int64_t place, int64_t first, int32_t count,
+                                         BcWarp& sh, double* s_a, double& acc0, double& acc1,
+                                         unsigned long long& mask) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int c0, c1;
+    mask = bc_gather<UNIT>(col, val, t0, t1, bits, X, p.ns, need, sh, s_a, acc0, acc1, c0, c1);
+    if (c0 >= 0) p.part[place * 64 + c0] = acc0;
+    if (c1 >= 0) p.part[place * 64 + c1] = acc1;
+    if (lane == 0) p.pmask[place] = mask;
+    __threadfence();
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) {
+        last = atomicAdd(p.pdone + first, 1) == count - 1;
+        if (last) p.pdone[first] = 0;
     }
+    if (!__shfl_sync(FULL, last, 0)) return false;
+    __threadfence();
+    acc0 = acc1 = 0.0;
+    mask = 0ull;
+    for (int32_t c = 0; c < count; ++c) {
+        const unsigned long long m = __ldcg(p.pmask + first + c);
+        if (m >> lane & 1ull) acc0 += __ldcg(p.part + (first + c) * 64 + lane);
+        if (m >> (lane + 32) & 1ull) acc1 += __ldcg(p.part + (first + c) * 64 + 32 + lane);
+        mask |= m;
+    }
+    return true;
+}
 
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t r = r0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < r1; r += warps) {
-        const int32_t v = p.rv[r];
-        const int32_t ab = p.ar[v], ae = p.ar[v + 1];
-        if (ae - ab > kBcHeavyDeg) continue;  // done above
-        const int32_t e0 = p.rs[r], n = p.rl[r];
-        double vsum = 0.0;
-        for (int base = 0; base < n; base += 32 * kBcPer) {
-            int s[kBcPer];
-            double acc[kBcPer];
-#pragma unroll
-            for (int u = 0; u < kBcPer; ++u) {
-                const int e = base + u * 32 + lane;
-                s[u] = e < n ? p.es[e0 + e] : -1;
-                acc[u] = 0.0;
+// Items per take.
+__device__ __forceinline__ int bc_take(int64_t items, int most) {
+    const int64_t n = items / ((int64_t)gridDim.x * kBcWarps * 4);
+    return n < 1 ? 1 : n > most ? most : (int)n;
+}
+
+// The warp's next task of the level.
+__device__ __forceinline__ int32_t bc_next(const BcArgs& p) {
+    int32_t t = 0;
+    if ((threadIdx.x & 31) == 0) t = atomicAdd(&p.st->next, 1);
+    return __shfl_sync(0xffffffffu, t, 0);
+}
+
+// Push: the row (unit key with columns mask) of vertex u and its
+// out-neighbours [t0, t1), lanes over neighbours: S[w][c] += A[u][w] * S[u][c]
+// for every column c that has not reached w; the first touch of w's unit lists
+// it.
+template <bool UNIT>
+__device__ __forceinline__ void bc_push_row(const BcArgs& p, unsigned long long* Fn, int blk, int32_t u,
+                                            unsigned long long mask, int32_t t0, int32_t t1) {
+    const int lane = threadIdx.x & 31;
+    const double* src = p.S + (size_t)u * p.ns + blk * 64;
+    for (int32_t t = t0 + lane; t < t1; t += 32) {
+        const int32_t w = __ldg(p.ac + t);
+        const int64_t key = (int64_t)blk * p.m + w;
+        unsigned long long add = mask & ~p.V[key];
+        if (add == 0ull) continue;
+        const double a = UNIT ? 1.0 : __ldg(p.av + t);
+        if (atomicOr(Fn + key, add) == 0ull) p.tlist[atomicAdd(&p.st->ntouched, 1)] = (int32_t)key;
+        double* dst = p.S + (size_t)w * p.ns + blk * 64;
+        while (add) {
+            const int c = __ffsll((long long)add) - 1;
+            add &= add - 1;
+            atomicAdd(dst + c, UNIT ? src[c] : a * src[c]);
+        }
+    }
+}
+
+// One forward level.
+template <bool UNIT>
+__global__ void __launch_bounds__(kBcThreads, 4) k_bc_forward(const BcArgs* __restrict__ ap) {
+    __shared__ BcWarp s_warp[kBcWarps];
+    __shared__ double s_a[UNIT ? 1 : kBcWarps][32];
+    const BcArgs& p = *ap;
+    const BcState* st = p.st;
+    if (st->done) return;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double* my_a = UNIT ? nullptr : s_a[UNIT ? 0 : wid];
+    const int d = st->d;
+    const unsigned long long* Fc = p.F[d % 3];
+    unsigned long long* Fn = p.F[(d + 1) % 3];
+    unsigned long long work = 0;
+    if (st->mode != 0) {
+        const int32_t task0 = p.ltask[d], ntask = p.ltask[d + 1] - task0;
+        const int32_t row0 = p.lrow[d], nrow = p.lrow[d + 1] - row0;
+        for (int32_t t = bc_next(p); t < ntask + nrow; t = bc_next(p)) {
+            int32_t u;
+            if (t < ntask) {
+                const int2 task = p.htask[task0 + t];
+                const int64_t hr = heavy_row(p, task.x);
+                const int blk = bc_block(p, p.rkey[hr], u);
+                const int32_t b = p.ar[u] + task.y * p.piece;
+                bc_push_row<UNIT>(p, Fn, blk, u, p.rmask[hr], b, min(p.ar[u + 1], b + p.piece));
+            } else {
+                const int32_t r = row0 + t - ntask;
+                const int blk = bc_block(p, p.rkey[r], u);
+                bc_push_row<UNIT>(p, Fn, blk, u, p.rmask[r], p.ar[u], p.ar[u + 1]);
             }
-            bc_push_range<UNIT, MODE>(p, ab, ae, 32, s, acc, ring);
-#pragma unroll
-            for (int u = 0; u < kBcPer; ++u) {
-                const int e = base + u * 32 + lane;
-                if (e < n) {
-                    const double c = acc[u] * p.ev[e0 + e];
-                    p.ed[e0 + e] += c;
-                    vsum += c;
+        }
+    } else {
+        // pieces of heavy vertices' in-neighbour lists, then the other units,
+        // a take's far apart (hubs sit together)
+        const int nchunk = st->nchunk;
+        const int64_t units = p.m * p.nblk, nheavy = (int64_t)nchunk * p.nblk;
+        const int take = bc_take(units, kBcUnits);
+        const int64_t ntake = (units + take - 1) / take;
+        for (int64_t t = bc_next(p); t < nheavy + ntake; t = bc_next(p)) {
+            if (t < nheavy) {
+                const int blk = (int)(t / nchunk);
+                const int64_t off = (int64_t)blk * nchunk;
+                const int4 c = p.chunk[t - off];
+                const int32_t v = c.x;
+                const int64_t key = (int64_t)blk * p.m + v;
+                const unsigned long long vis = __ldcg(p.V + key), need = bc_columns(p, blk) & ~vis;
+                if (need == 0ull) continue;  // the same for all pieces: only the last to arrive changes V
+                const int32_t b = p.atr[v] + c.y * p.piece;
+                double acc0, acc1;
+                unsigned long long mask;
+                if (!bc_piece<UNIT>(p, p.atc, p.atv, b, min(p.atr[v + 1], b + p.piece), Fc + (int64_t)blk * p.m,
+                                    p.S + blk * 64, need, off + c.z + c.y, off + c.z, c.w, s_warp[wid], my_a, acc0, acc1,
+                                    mask))
+                    continue;
+                double* dst = p.S + (size_t)v * p.ns + blk * 64 + lane;
+                if (mask >> lane & 1ull) dst[0] = acc0;
+                if (mask >> (lane + 32) & 1ull) dst[32] = acc1;
+                const unsigned long long mine = lane == 0 ? mask : 0ull;
+                if (mine) {
+                    p.V[key] = vis | mine;
+                    Fn[key] = mine;
+                }
+                work += bc_append(p, (int32_t)key, v, mine);
+                continue;
+            }
+            const int64_t key = t - nheavy + (int64_t)lane * ntake;
+            int32_t v = 0, ab = 0, ae = 0;
+            int blk = 0;
+            unsigned long long need = 0, vis = 0, found = 0;
+            if (lane < take && key < units) {
+                blk = bc_block(p, (int32_t)key, v);
+                ab = p.atr[v];
+                ae = p.atr[v + 1];
+                if (ae > ab && ae - ab <= p.piece) {
+                    vis = p.V[key];
+                    need = bc_columns(p, blk) & ~vis;
                 }
             }
+            unsigned act = __ballot_sync(FULL, need != 0ull);
+            while (act) {
+                const int l = __ffs(act) - 1;
+                act &= act - 1;
+                const int32_t b = __shfl_sync(FULL, ab, l), e = __shfl_sync(FULL, ae, l);
+                const int32_t vv = __shfl_sync(FULL, v, l);
+                const int bb = __shfl_sync(FULL, blk, l);
+                const unsigned long long nd = __shfl_sync(FULL, need, l);
+                double acc0, acc1;
+                int c0, c1;
+                const unsigned long long got = bc_gather<UNIT>(p.atc, p.atv, b, e, Fc + (int64_t)bb * p.m,
+                                                               p.S + bb * 64, p.ns, nd, s_warp[wid], my_a, acc0,
+                                                               acc1, c0, c1);
+                double* dst = p.S + (size_t)vv * p.ns + bb * 64;
+                if (c0 >= 0) dst[c0] = acc0;
+                if (c1 >= 0) dst[c1] = acc1;
+                if (lane == l) found = got;
+            }
+            if (found) {
+                p.V[key] = vis | found;
+                Fn[key] = found;
+            }
+            if (__ballot_sync(FULL, found != 0ull)) work += bc_append(p, (int32_t)key, v, found);
         }
-        vsum = warp_sum<double>(vsum);
-        if (lane == 0 && vsum != 0.0) atomicAdd(&p.bc[v], vsum);
+    }
+    work = warp_sum<unsigned long long>(work);
+    if (lane == 0 && work) atomicAdd(&p.st->next_work, work);
+    // the buffer after next: the last level's frontier leaves it
+    if (d > 0) {
+        unsigned long long* Fo = p.F[(d - 1) % 3];
+        const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+        for (int64_t r = p.lrow[d - 1] + i0; r < p.lrow[d]; r += step) Fo[p.rkey[r]] = 0ull;
+        for (int64_t r = p.lhrow[d - 1] + i0; r < p.lhrow[d]; r += step) Fo[p.rkey[heavy_row(p, r)]] = 0ull;
     }
 }
 
-__global__ void k_bc_backward_finalize(BcArgs p, LoopCtl ctl) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Ends a forward level: a push level's units append their rows; the last
+// block closes the level's lists, chooses the next one's direction and tells
+// the loop whether to go on.
+__global__ void __launch_bounds__(kBcThreads) k_bc_forward_end(const BcArgs* __restrict__ ap, LoopCtl ctl) {
+    __shared__ bool s_last;
+    const BcArgs& p = *ap;
     BcState* st = p.st;
-    st->nhrows = 0;
-    if (st->k >= 1) st->k -= 1;
-    loop_continue(ctl, st->k >= 1);
+    const int lane = threadIdx.x & 31;
+    const int d = st->d;
+    if (!st->done && st->mode != 0) {
+        unsigned long long* Fn = p.F[(d + 1) % 3];
+        const int n = st->ntouched;
+        unsigned long long work = 0;
+        for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n;
+             i0 += (int64_t)gridDim.x * blockDim.x) {
+            const int64_t i = i0 + lane;
+            int32_t key = 0, v = 0;
+            unsigned long long mask = 0;
+            if (i < n) {
+                key = p.tlist[i];
+                bc_block(p, key, v);
+                mask = Fn[key];
+                p.V[key] |= mask;
+            }
+            work += bc_append(p, key, v, mask);
+        }
+        work = warp_sum<unsigned long long>(work);
+        if (lane == 0 && work) atomicAdd(&st->next_work, work);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&st->blocks, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last || threadIdx.x != 0) return;
+    __threadfence();
+    st->blocks = 0;
+    st->next = 0;
+    bool more = false;
+    if (!st->done) {
+        const int32_t rows = *(volatile int32_t*)&st->nrows, hrows = *(volatile int32_t*)&st->nhrows;
+        if (rows == p.lrow[d + 1] && hrows == p.lhrow[d + 1]) {
+            st->done = 1;
+        } else {
+            p.lrow[d + 2] = rows;
+            p.lhrow[d + 2] = hrows;
+            p.ltask[d + 2] = *(volatile int32_t*)&st->nhtasks;
+            const unsigned long long work = *(volatile unsigned long long*)&st->next_work;
+            st->cur_work = work;
+            st->next_work = 0;
+            st->ntouched = 0;
+            st->mode = work < kBcPushMul * (unsigned long long)p.nnz ? 1 : 0;
+            st->d = d + 1;
+            // distances are below m
+            more = (int64_t)(d + 1) < p.m;
+            if (!more) st->done = 1;
+        }
+    }
+    if (!more) st->k = st->flags ? 0 : st->d;
+    loop_continue(ctl, more);
 }
 
-// Per vertex (one thread): a self-loop (flags bit 1; rows are sorted, so a
-// binary search finds it) and the list of vertices with more than
-// kBcHeavyDeg in-neighbours (count in flags[1]).
-__global__ void k_bc_scan_vertices(const int32_t* __restrict__ r, const int32_t* __restrict__ c,
-                                   const int32_t* __restrict__ tr, int64_t m, int32_t* __restrict__ heavy,
-                                   int* __restrict__ flags) {
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < m; v += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t b = r[v], n = r[v + 1] - b;
-        const int pos = lower_bound_i32(c + b, n, (int32_t)v);
-        if (pos < n && c[b + pos] == (int32_t)v) atomicOr(flags, 1);
-        if (tr[v + 1] - tr[v] > kBcHeavyDeg) heavy[atomicAdd(flags + 1, 1)] = (int32_t)v;
+// Before the backward loop: W = 1 / sigma and the bits of the largest distance.
+__global__ void k_bc_back_init(const BcArgs* __restrict__ ap) {
+    const BcArgs& p = *ap;
+    const int k = p.st->k;
+    if (k < 2) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int64_t nl = p.lrow[k + 1] - p.lrow[k], n = nl + p.lhrow[k + 1] - p.lhrow[k];
+    unsigned long long* L = p.F[k % 3];
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+        const int64_t r = i < nl ? p.lrow[k] + i : heavy_row(p, p.lhrow[k] + i - nl);
+        const int32_t key = p.rkey[r];
+        const unsigned long long mask = p.rmask[r];
+        int32_t v;
+        const int blk = bc_block(p, key, v);
+        const size_t at = (size_t)v * p.ns + blk * 64 + lane;
+        if (mask >> lane & 1ull) p.W[at] = 1.0 / p.S[at];
+        if (mask >> (lane + 32) & 1ull) p.W[at + 32] = 1.0 / p.S[at + 32];
+        if (lane == 0) L[key] = mask;
     }
 }
 
-__global__ void k_bc_check_sources(const int32_t* __restrict__ src, int ns, int64_t m, int* __restrict__ mark,
-                                   int* __restrict__ flags) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < ns; j += gridDim.x * blockDim.x) {
-        int v = src[j];
-        if (v < 0 || (int64_t)v >= m) { atomicOr(flags, 8); continue; }
-        if (atomicAdd(&mark[v], 1) != 0) atomicOr(flags, 16);
+// One backward level: the rows at distance k - 1 (their neighbours at
+// distance k have W and their bits in F[k % 3]).
+template <bool UNIT>
+__global__ void __launch_bounds__(kBcThreads, 4) k_bc_backward(const BcArgs* __restrict__ ap, LoopCtl ctl) {
+    __shared__ BcWarp s_warp[kBcWarps];
+    __shared__ double s_a[UNIT ? 1 : kBcWarps][32];
+    __shared__ double s_acc[kBcWarps][64];
+    __shared__ double s_part[kBcWarps][kBcRows][33];
+    __shared__ bool s_last;
+    const BcArgs& p = *ap;
+    BcState* st = p.st;
+    const int k = st->k;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double* my_a = UNIT ? nullptr : s_a[UNIT ? 0 : wid];
+    if (k >= 2) {
+        const unsigned long long* Lk = p.F[k % 3];
+        unsigned long long* Ln = p.F[(k - 1) % 3];
+        const bool next = k > 2;  // distance 1 needs no W: the sources take no score from their own searches
+        // a row's sums (s_acc, by column) become its scores, W and bits; the
+        // lane's part of the score. The row's columns are put side by side: up
+        // to 32 of them take one round of FP64 work instead of two.
+        auto finish = [&](int32_t v, int blk, int32_t key, unsigned long long mask) {
+            __syncwarp();
+            bc_list_columns(mask, s_warp[wid].col);
+            __syncwarp();
+            const int n = __popcll(mask);
+            double part = 0.0;
+            for (int e = lane; e < n; e += 32) {
+                const int c = s_warp[wid].col[e];
+                const size_t at = (size_t)v * p.ns + blk * 64 + c;
+                const double sg = p.S[at], a = s_acc[wid][c];
+                part += a * sg;
+                if (next) p.W[at] = 1.0 / sg + a;
+            }
+            if (lane == 0) Ln[key] = mask;
+            __syncwarp();
+            return part;
+        };
+        const int32_t task0 = p.ltask[k - 1], ntask = p.ltask[k] - task0;
+        const int32_t row0 = p.lrow[k - 1], row1 = p.lrow[k];
+        const int take = bc_take(row1 - row0, kBcRows);
+        const int32_t ntake = (row1 - row0 + take - 1) / take;
+        for (int32_t t = bc_next(p); t < ntask + ntake; t = bc_next(p)) {
+            if (t < ntask) {  // a piece of a heavy row
+                const int2 task = p.htask[task0 + t];
+                const int64_t hr = heavy_row(p, task.x);
+                const int32_t key = p.rkey[hr];
+                const unsigned long long mask = p.rmask[hr];
+                int32_t v;
+                const int blk = bc_block(p, key, v);
+                const int32_t vb = p.ar[v], ve = p.ar[v + 1], b = vb + task.y * p.piece;
+                const int32_t first = p.hfirst[task.x] - task0;
+                double acc0, acc1;
+                unsigned long long got;
+                if (!bc_piece<UNIT>(p, p.ac, p.av, b, min(ve, b + p.piece), Lk + (int64_t)blk * p.m, p.W + blk * 64,
+                                    mask, first + task.y, first, (ve - vb + p.piece - 1) / p.piece, s_warp[wid], my_a,
+                                    acc0, acc1, got))
+                    continue;
+                s_acc[wid][lane] = acc0;
+                s_acc[wid][32 + lane] = acc1;
+                const double part = warp_sum<double>(finish(v, blk, key, mask));
+                if (lane == 0 && part != 0.0) atomicAdd(&p.bc[v], part);
+                continue;
+            }
+            // a take of the other rows; their score sums are added together
+            // (10 FP64 instructions for up to eight rows instead of 5 per row)
+            const int32_t r0 = row0 + (t - ntask) * take, nr = min(take, row1 - r0);
+            int32_t lkey = 0, lv = 0, lb = 0, le = 0;
+            int lblk = 0;
+            unsigned long long lmask = 0;
+            if (lane < nr) {
+                lkey = p.rkey[r0 + lane];
+                lmask = p.rmask[r0 + lane];
+                lblk = bc_block(p, lkey, lv);
+                lb = p.ar[lv];
+                le = p.ar[lv + 1];
+            }
+            for (int i = 0; i < nr; ++i) {
+                const unsigned FULL = 0xffffffffu;
+                const unsigned long long mask = __shfl_sync(FULL, lmask, i);
+                const int blk = __shfl_sync(FULL, lblk, i);
+                double acc0, acc1;
+                int c0, c1;
+                bc_gather<UNIT>(p.ac, p.av, __shfl_sync(FULL, lb, i), __shfl_sync(FULL, le, i),
+                                Lk + (int64_t)blk * p.m, p.W + blk * 64, p.ns, mask, s_warp[wid], my_a, acc0, acc1, c0,
+                                c1);
+                s_acc[wid][lane] = 0.0;
+                s_acc[wid][32 + lane] = 0.0;
+                __syncwarp();
+                if (c0 >= 0) s_acc[wid][c0] = acc0;
+                if (c1 >= 0) s_acc[wid][c1] = acc1;
+                s_part[wid][i][lane] = finish(__shfl_sync(FULL, lv, i), blk, __shfl_sync(FULL, lkey, i), mask);
+            }
+            for (int i = nr; i < kBcRows; ++i) s_part[wid][i][lane] = 0.0;
+            __syncwarp();
+            // four lanes per row, eight columns each
+            const int r = lane & 7, q = lane >> 3;
+            double s = 0.0;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) s += s_part[wid][r][q * 8 + c];
+            s += __shfl_xor_sync(0xffffffffu, s, 8);
+            s += __shfl_xor_sync(0xffffffffu, s, 16);
+            if (lane < nr && s != 0.0) atomicAdd(&p.bc[lv], s);
+            __syncwarp();
+        }
+        // the buffer after next: distance k + 1 leaves it
+        unsigned long long* Lo = p.F[(k + 1) % 3];
+        if (k < st->d) {
+            const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+            for (int64_t r = p.lrow[k + 1] + i0; r < p.lrow[k + 2]; r += step) Lo[p.rkey[r]] = 0ull;
+            for (int64_t r = p.lhrow[k + 1] + i0; r < p.lhrow[k + 2]; r += step) Lo[p.rkey[heavy_row(p, r)]] = 0ull;
+        }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&st->blocks, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last || threadIdx.x != 0) return;
+    st->blocks = 0;
+    st->next = 0;
+    if (k >= 1) st->k = k - 1;
+    loop_continue(ctl, k - 1 >= 2);
 }
 
 // Packed source columns of a batch over a block-diagonal union (device
@@ -785,6 +776,13 @@ struct BcPacking {
     int ncols = 0;
 };
 
+template <typename K>
+static int bc_grid(ga_ctx ctx, K kernel) {
+    int per_sm = 1;
+    GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBcThreads, 0));
+    return ctx->num_sms * std::max(per_sm, 1);
+}
+
 // accumulate: add this batch's scores to d_bc instead of overwriting it.
 static void bc_device(ga_ctx ctx, ga_csr A, const int32_t* d_sources, int64_t nsrc, double* d_bc,
                       bool accumulate = false, const BcPacking* pk = nullptr) {
@@ -797,7 +795,7 @@ static void bc_device(ga_ctx ctx, ga_csr A, const int32_t* d_sources, int64_t ns
     if (!accumulate) GA_CUDA(cudaMemsetAsync(d_bc, 0, sizeof(double) * (m ? m : 1), ctx->stream));
     if (m == 0 || nsrc == 0) return;
     const int ns = pk ? pk->ncols : (int)nsrc;  // source columns
-    const int words = (ns + 31) / 32;
+    const int nblk = (ns + 63) / 64;
     GA_REQUIRE(m * (int64_t)(ns + 1) + nsrc < INT32_MAX, GA_ERR_UNSUPPORTED,
                "BC: m x sources exceeds the int32 entry range");
     ProfScope whole(ctx, "bc");
@@ -813,154 +811,96 @@ static void bc_device(ga_ctx ctx, ga_csr A, const int32_t* d_sources, int64_t ns
         ga_csr Av = unit ? A : Ad;
         if (!symmetric) AT = transpose_csr(ctx, Av);
         ga_csr ATu = symmetric ? Av : AT;
-        DBuf<int> flags(ctx, 2), mark(ctx, (size_t)m);
-        DBuf<int32_t> heavy(ctx, (size_t)m + 1);
-        GA_CUDA(cudaMemsetAsync(flags.p, 0, 2 * sizeof(int), ctx->stream));
-        GA_CUDA(cudaMemsetAsync(mark.p, 0, sizeof(int) * m, ctx->stream));
-        k_bc_scan_vertices<<<grid_for(m, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(Av->rst, Av->col, ATu->rst,
-                                                                                        m, heavy.p, flags.p);
-        post_launch("bc_scan_vertices");
-        k_bc_check_sources<<<grid_for(nsrc, 256, 64), 256, 0, ctx->stream>>>(d_sources, (int)nsrc, m, mark.p,
-                                                                            flags.p);
-        post_launch("bc_check_sources");
-        int hf[2];
-        GA_CUDA(cudaMemcpyAsync(hf, flags.p, sizeof(hf), cudaMemcpyDeviceToHost, ctx->stream));
-        GA_CUDA(cudaStreamSynchronize(ctx->stream));
-        const int f = hf[0];
-        GA_REQUIRE(!(f & 1), GA_ERR_INVALID_ARG, "BC: the graph has self-loops");
-        GA_REQUIRE(!(f & 8), GA_ERR_INVALID_ARG, "BC: source index out of range");
-        GA_REQUIRE(!(f & 16), GA_ERR_INVALID_ARG, "BC: sources must be distinct");
-
-        const int64_t cap_entries = m * (int64_t)ns + nsrc;
-        const int64_t cap_rows = cap_entries;
+        const size_t units = (size_t)m * nblk, pairs = (size_t)m * ns;
+        // pieces of the longer of the two heavy lists: at most nnz / piece full
+        // ones and one more per heavy vertex; a heavy vertex has a row in at
+        // most ns levels, and a level's rows of one vertex are one per block
+        const int piece = A->nnz > (int64_t)kBcDense * m ? kBcPieceDense : kBcPiece;
+        const size_t pieces = (size_t)(2 * (A->nnz / piece) + 1);
+        const size_t hrows = std::min(pairs, (size_t)(A->nnz / piece) * ns) + 1;
+        DBuf<BcState> st(ctx, 1);
+        DBuf<uint32_t> seen(ctx, (size_t)(m + 31) / 32);
+        DBuf<unsigned long long> words(ctx, 4 * units);  // V, F[0], F[1], F[2]
+        DBuf<double> S(ctx, pairs), W(ctx, pairs);
+        DBuf<int32_t> rkey(ctx, pairs);
+        DBuf<unsigned long long> rmask(ctx, pairs);
+        DBuf<int32_t> hfirst(ctx, hrows);
+        DBuf<int2> htask(ctx, pieces * ns);
+        DBuf<int32_t> levels(ctx, 3 * ((size_t)m + 3));
+        DBuf<int4> chunk(ctx, pieces);
+        DBuf<double> part(ctx, pieces * nblk * 64);
+        DBuf<unsigned long long> pmask(ctx, pieces * nblk);
+        DBuf<int32_t> pdone(ctx, pieces * nblk), tlist(ctx, units);
         BcArgs p;
         p.atr = ATu->rst; p.atc = ATu->col; p.atv = unit ? nullptr : static_cast<const double*>(ATu->val);
         p.ar = Av->rst; p.ac = Av->col; p.av = unit ? nullptr : static_cast<const double*>(Av->val);
-        p.m = m; p.ns = ns; p.words = words; p.sources = d_sources;
-        p.nsrc = (int)nsrc; p.scol = pk ? pk->scol : nullptr;
-        DBuf<BcState> st(ctx, 1);
-        DBuf<int32_t> level_rows(ctx, (size_t)m + 2);
-        DBuf<int32_t> cs0(ctx, m), cs1(ctx, m), cl0(ctx, m), cl1(ctx, m), vcnt(ctx, m);
-        DBuf<uint32_t> vbits(ctx, (size_t)m * words), inlvl(ctx, (size_t)(m + 31) / 32);
-        DBuf<int32_t> es(ctx, (size_t)cap_entries);
-        DBuf<double> ev(ctx, (size_t)cap_entries), ed(ctx, (size_t)cap_entries);
-        DBuf<int32_t> rv(ctx, (size_t)cap_rows), rs(ctx, (size_t)cap_rows), rl(ctx, (size_t)cap_rows);
-        DBuf<double> W(ctx, (size_t)m * ns);
-        GA_CUDA(cudaMemsetAsync(cl0.p, 0, sizeof(int32_t) * m, ctx->stream));
-        GA_CUDA(cudaMemsetAsync(cl1.p, 0, sizeof(int32_t) * m, ctx->stream));
-        GA_CUDA(cudaMemsetAsync(vcnt.p, 0, sizeof(int32_t) * m, ctx->stream));
-        GA_CUDA(cudaMemsetAsync(vbits.p, 0, sizeof(uint32_t) * m * words, ctx->stream));
-        GA_CUDA(cudaMemsetAsync(inlvl.p, 0, sizeof(uint32_t) * ((m + 31) / 32), ctx->stream));
-        GA_CUDA(cudaMemsetAsync(W.p, 0, sizeof(double) * m * ns, ctx->stream));
-        p.st = st.p; p.level_rows = level_rows.p;
-        p.cur_start[0] = cs0.p; p.cur_start[1] = cs1.p; p.cur_len[0] = cl0.p; p.cur_len[1] = cl1.p;
-        p.vbits = vbits.p; p.vcnt = vcnt.p;
-        p.es = es.p; p.ev = ev.p; p.ed = ed.p;
-        p.rv = rv.p; p.rs = rs.p; p.rl = rl.p;
-        p.cap_entries = cap_entries; p.cap_rows = cap_rows;
-        p.W = W.p; p.inlvl = inlvl.p; p.bc = d_bc;
-        // vertices whose in-neighbour lists are split over a CTA
-        p.heavy_in = heavy.p;
-        p.nheavy_in = hf[1];
-
-        // push-level state: touched bits, list of reached vertices, marks
-        DBuf<uint32_t> tbits(ctx, (size_t)m * words);
-        DBuf<int32_t> tlist(ctx, (size_t)m), tmark(ctx, (size_t)m), hrows(ctx, (size_t)m);
-        GA_CUDA(cudaMemsetAsync(tbits.p, 0, sizeof(uint32_t) * m * words, ctx->stream));
-        GA_CUDA(cudaMemsetAsync(tmark.p, 0, sizeof(int32_t) * m, ctx->stream));
-        p.hrows = hrows.p; p.tbits = tbits.p; p.tlist = tlist.p; p.tmark = tmark.p;
-        p.nnz = ATu->nnz;
-        k_bc_state_init<<<1, 1, 0, ctx->stream>>>(p);
-        post_launch("bc_state_init");
+        p.m = m; p.nnz = A->nnz; p.ns = ns; p.nblk = nblk; p.piece = piece; p.nsrc = (int)nsrc;
+        p.sources = d_sources; p.scol = pk ? pk->scol : nullptr;
+        p.st = st.p;
+        p.V = words.p;
+        for (int b = 0; b < 3; ++b) p.F[b] = words.p + (size_t)(b + 1) * units;
+        p.S = S.p; p.W = W.p;
+        p.rkey = rkey.p; p.rmask = rmask.p;
+        p.rlast = (int64_t)pairs - 1; p.hfirst = hfirst.p; p.htask = htask.p;
+        p.lrow = levels.p; p.lhrow = levels.p + (m + 3); p.ltask = levels.p + 2 * (m + 3);
+        p.chunk = chunk.p; p.part = part.p; p.pmask = pmask.p; p.pdone = pdone.p; p.tlist = tlist.p;
+        p.bc = d_bc;
+        GA_CUDA(cudaMemsetAsync(st.p, 0, sizeof(BcState), ctx->stream));
+        GA_CUDA(cudaMemsetAsync(seen.p, 0, sizeof(uint32_t) * seen.count, ctx->stream));
+        GA_CUDA(cudaMemsetAsync(words.p, 0, sizeof(unsigned long long) * words.count, ctx->stream));
+        GA_CUDA(cudaMemsetAsync(S.p, 0, sizeof(double) * pairs, ctx->stream));  // push levels add into it
+        GA_CUDA(cudaMemsetAsync(pdone.p, 0, sizeof(int32_t) * pdone.count, ctx->stream));
+        const int grid_v = grid_for(m, 256, ctx->num_sms * 8);
+        k_bc_scan_vertices<<<grid_v, 256, 0, ctx->stream>>>(p);
+        post_launch("bc_scan_vertices");
+        k_bc_check_sources<<<grid_for(nsrc, 256, 64), 256, 0, ctx->stream>>>(p, seen.p);
+        post_launch("bc_check_sources");
         if (pk) {
-            k_bc_previsit<<<grid_for(m, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(p, pk->voff, pk->gsrc,
-                                                                                       pk->count);
+            k_bc_previsit<<<grid_v, 256, 0, ctx->stream>>>(p, pk->voff, pk->gsrc, pk->count);
             post_launch("bc_previsit");
         }
-        k_bc_init<<<grid_for(nsrc, 256, 64), 256, 0, ctx->stream>>>(p);
+        k_bc_init<<<1, kBcThreads, 0, ctx->stream>>>(p);
         post_launch("bc_init");
-
-        const size_t per_warp = (size_t)ns * sizeof(double) + 2 * (size_t)words * sizeof(uint32_t) +
-                                32 * (2 * sizeof(int) + sizeof(double));
-        const size_t smem = kBcWarps * ((per_warp + 15) & ~(size_t)15);
+        // The loops' kernels read the call's parameters from a device copy
+        // and have fixed grids, so the context captures each loop once.
+        const int fslot = unit ? kLoopSlotBcForward : kLoopSlotBcForwardVal;
+        const int bslot = unit ? kLoopSlotBcBackward : kLoopSlotBcBackwardVal;
+        BcArgs* fargs = static_cast<BcArgs*>(cached_loop_args(ctx, fslot, sizeof(BcArgs)));
+        BcArgs* bargs = static_cast<BcArgs*>(cached_loop_args(ctx, bslot, sizeof(BcArgs)));
+        GA_CUDA(cudaMemcpyAsync(fargs, &p, sizeof(BcArgs), cudaMemcpyHostToDevice, ctx->stream));
+        GA_CUDA(cudaMemcpyAsync(bargs, &p, sizeof(BcArgs), cudaMemcpyHostToDevice, ctx->stream));
         auto fwd = unit ? k_bc_forward<true> : k_bc_forward<false>;
-        // The attribute is per kernel, not per call: calls with other source
-        // counts may run concurrently (other contexts, other threads), so it
-        // is always set to the largest size any call launches with.
-        constexpr size_t kMaxWords = (kBcMaxSources + 31) / 32;
-        constexpr size_t max_per_warp = (size_t)kBcMaxSources * sizeof(double) + 2 * kMaxWords * sizeof(uint32_t) +
-                                        32 * (2 * sizeof(int) + sizeof(double));
-        constexpr size_t max_smem = kBcWarps * ((max_per_warp + 15) & ~(size_t)15);
-        GA_CUDA(cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
-        int per_sm = 1;
-        GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fwd, kBcThreads, smem));
-        if (per_sm < 1) per_sm = 1;
-        const int grid_fwd = ctx->num_sms * per_sm;
-        const int grid_rows = ctx->num_sms * 8;
+        auto bwd = unit ? k_bc_backward<true> : k_bc_backward<false>;
+        const int grid_fwd = bc_grid(ctx, fwd), grid_bwd = bc_grid(ctx, bwd), grid_end = ctx->num_sms;
         {
             ProfScope ps(ctx, "bc_forward_loop");
-            auto push = unit ? k_bc_push<true> : k_bc_push<false>;
-            run_device_loop(ctx, [&](const LoopCtl& ctl) {
-                k_bc_level_begin<<<1, 1, 0, ctx->stream>>>(p);
-                post_launch("bc_level_begin");
+            run_cached_loop(ctx, fslot, [ctx, fwd, fargs, grid_fwd, grid_end](const LoopCtl& ctl) {
                 {
-                    ProfScope pk(ctx, "bc_forward_pull");
-                    fwd<<<grid_fwd, kBcThreads, smem, ctx->stream>>>(p);
+                    ProfScope pf(ctx, "bc_forward");
+                    fwd<<<grid_fwd, kBcThreads, 0, ctx->stream>>>(fargs);
                     post_launch("bc_forward");
                 }
-                {
-                    ProfScope pk(ctx, "bc_forward_push");
-                    push<<<grid_rows, kBcThreads, 0, ctx->stream>>>(p);
-                    post_launch("bc_push");
-                    k_bc_push_clear<<<grid_for(m, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(p);
-                    post_launch("bc_push_clear");
-                    k_bc_push_emit<<<grid_rows, kBcThreads, 0, ctx->stream>>>(p);
-                    post_launch("bc_push_emit");
-                }
-                k_bc_forward_finalize<<<1, 32, 0, ctx->stream>>>(p, ctl);
-                post_launch("bc_forward_finalize");
+                k_bc_forward_end<<<grid_end, kBcThreads, 0, ctx->stream>>>(fargs, ctl);
+                post_launch("bc_forward_end");
             }, m + 2);
         }
         {
             ProfScope ps(ctx, "bc_backward_loop");
-            // the bulk form copies whole W rows: 16-byte aligned rows and at
-            // most kBcBulkMaxCols columns (its shared-memory ring)
-            int mode = ctx->bc_backward;
-            if (mode == kBcBwdBulk &&
-                (ns % 2 != 0 || ns > kBcBulkMaxCols || (reinterpret_cast<uintptr_t>(p.W) & 15u) != 0))
-                mode = kBcBwdGather;
-            void (*bwd)(BcArgs) = nullptr;
-            size_t bsmem = 0;
-            if (mode == kBcBwdBulk) {
-                bwd = unit ? k_bc_backward<true, kBcBwdBulk> : k_bc_backward<false, kBcBwdBulk>;
-                bsmem = (size_t)kBcWarps * 2 * kBcHits * ns * sizeof(double) + (size_t)kBcWarps * 2 * sizeof(uint64_t);
-                constexpr size_t max_bsmem = (size_t)kBcWarps * 2 * kBcHits * kBcBulkMaxCols * sizeof(double) +
-                                             (size_t)kBcWarps * 2 * sizeof(uint64_t);
-                GA_CUDA(cudaFuncSetAttribute(bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_bsmem));
-            } else if (mode == kBcBwdSingle) {
-                bwd = unit ? k_bc_backward<true, kBcBwdSingle> : k_bc_backward<false, kBcBwdSingle>;
-            } else {
-                bwd = unit ? k_bc_backward<true, kBcBwdGather> : k_bc_backward<false, kBcBwdGather>;
-            }
-            run_device_loop(ctx, [&](const LoopCtl& ctl) {
-                k_bc_set_w<<<grid_rows, 256, 0, ctx->stream>>>(p, true);
-                post_launch("bc_set_w");
-                {
-                    ProfScope pk(ctx, "bc_backward");
-                    bwd<<<grid_rows, kBcThreads, bsmem, ctx->stream>>>(p);
-                    post_launch("bc_backward");
-                }
-                k_bc_set_w<<<grid_rows, 256, 0, ctx->stream>>>(p, false);
-                post_launch("bc_clear_w");
-                k_bc_backward_finalize<<<1, 32, 0, ctx->stream>>>(p, ctl);
-                post_launch("bc_backward_finalize");
+            GA_CUDA(cudaMemsetAsync(p.F[0], 0, sizeof(unsigned long long) * 3 * units, ctx->stream));
+            k_bc_back_init<<<ctx->num_sms * 4, 256, 0, ctx->stream>>>(bargs);
+            post_launch("bc_back_init");
+            run_cached_loop(ctx, bslot, [ctx, bwd, bargs, grid_bwd](const LoopCtl& ctl) {
+                ProfScope pb(ctx, "bc_backward");
+                bwd<<<grid_bwd, kBcThreads, 0, ctx->stream>>>(bargs, ctl);
+                post_launch("bc_backward");
             }, m + 2);
         }
         BcState hs;
         GA_CUDA(cudaMemcpyAsync(&hs, st.p, sizeof(BcState), cudaMemcpyDeviceToHost, ctx->stream));
         GA_CUDA(cudaStreamSynchronize(ctx->stream));
-        GA_REQUIRE(!hs.overflow, GA_ERR_INVALID_ARG, "BC: entry store overflow");
-        GA_REQUIRE(!hs.stalled, GA_ERR_TIMEOUT, "BC: a bulk copy of the backward sweep did not complete");
+        GA_REQUIRE(!(hs.flags & 1), GA_ERR_INVALID_ARG, "BC: the graph has self-loops");
+        GA_REQUIRE(!(hs.flags & 8), GA_ERR_INVALID_ARG, "BC: source index out of range");
+        GA_REQUIRE(!(hs.flags & 16), GA_ERR_INVALID_ARG, "BC: sources must be distinct");
     } catch (...) {
         csr_destroy(ctx, AT);
         csr_destroy(ctx, Ad);

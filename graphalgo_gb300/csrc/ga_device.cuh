@@ -176,61 +176,6 @@ __device__ __forceinline__ int warp_lower_bound(int32_t key, int32_t x) {
     return lo;
 }
 
-// ------------------------------------------------ bulk copies (sm_90 and up)
-// One thread copies a contiguous global range into shared memory with the
-// tensor memory accelerator's untiled bulk copy; the bytes complete a
-// transaction count on a shared-memory barrier that the consumers wait on.
-// Both addresses must be 16-byte aligned and the size a multiple of 16.
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(arrivals) : "memory");
-}
-
-// Makes barrier initialisation visible to the bulk-copy unit.
-__device__ __forceinline__ void mbar_init_fence() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// One arrival that also announces `bytes` of bulk copies to come.
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-// Orders this thread's earlier shared-memory accesses before later bulk
-// copies into the same memory.
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// Waits until the barrier's phase of parity `parity` has completed, for at
-// most `max_cycles` SM clock cycles; false when the limit ran out.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long max_cycles) {
-    const long long t0 = clock64();
-    while (true) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (clock64() - t0 > max_cycles) return false;
-    }
-}
-
 }  // namespace ga
 
 // value-type dispatch over a ga_dtype

@@ -72,7 +72,6 @@ struct ga_ctx_s {
     int64_t fail_alloc_after = -1;  // fault injection
     bool knn_tiled = false;         // k-NN generator: tiled kernel for every graph
     bool kt_frontier = true;        // GA_TRI k-truss: incremental support after the first listing
-    int bc_backward = 0;            // BC backward sweep: W rows by gathers (0), bulk copies (1), one at a time (2)
     ga::MxmTune tune;               // masked-product schedule
     // profiling
     std::vector<ga::PendingTiming> pending;
@@ -96,7 +95,7 @@ struct ga_ctx_s {
     int64_t bytes_in_use = 0;
     int64_t bytes_peak = 0;
     // device loops captured once and relaunched (run_cached_loop), by slot
-    void* loop_cache[4] = {};
+    void* loop_cache[8] = {};
 };
 
 namespace ga {

@@ -39,6 +39,11 @@ void run_cached_loop(ga_ctx ctx, int slot, const std::function<void(const LoopCt
 // A device buffer of `bytes` kept with the slot's loop for the context's
 // lifetime: where the host writes the call's parameters before the launch.
 void* cached_loop_args(ga_ctx ctx, int slot, size_t bytes);
-enum { kLoopSlotTriFront = 0, kLoopSlotTriFrontBatch = 1 };
+enum {
+    kLoopSlotTriFront = 0, kLoopSlotTriFrontBatch,
+    kLoopSlotBcForward, kLoopSlotBcForwardVal, kLoopSlotBcBackward, kLoopSlotBcBackwardVal,
+    kLoopSlots
+};
+static_assert(kLoopSlots <= sizeof(ga_ctx_s::loop_cache) / sizeof(void*), "a cache entry per slot");
 
 }  // namespace ga

@@ -123,12 +123,8 @@ GA_API int ga_version(int* major, int* minor);
  * triangles once and then, per iteration, only the triangles of the edges it
  * prunes, lowering the supports they touch (same edge sets and iteration
  * counts); 0 lists every triangle again in every iteration.
- * GA_OPT_BC_BACKWARD (0): how BC's backward sweep reads the dependency
- * rows W[w] of a vertex's next-level neighbours: 0 gathers, the rows of
- * four neighbours in flight at once; 1 bulk copies (cp.async.bulk) of whole
- * rows into shared memory, two batches of four rows in flight per warp
- * (used for even source counts up to 128, else 0 runs); 2 one neighbour at
- * a time. Results are the same. */
+ * GA_OPT_BC_BACKWARD (0): 0, 1 or 2; without effect (the backward sweep had
+ * three ways to read its rows and now has one that is faster than each). */
 enum { GA_OPT_DEVICE_LOOPS = 1, GA_OPT_PROFILE = 2, GA_OPT_FAIL_ALLOC_AFTER = 3, GA_OPT_KNN_TILED = 4,
        GA_OPT_MXM_WARP_FLOPS = 5, GA_OPT_MXM_HEAVY_FLOPS = 6, GA_OPT_MXM_CTAS_PER_SM = 7, GA_OPT_DOT_CHUNK = 8,
        GA_OPT_HYBRID_RATIO = 9, GA_OPT_TRI_ORDER = 10, GA_OPT_KT_FRONTIER = 11, GA_OPT_BC_BACKWARD = 12 };
