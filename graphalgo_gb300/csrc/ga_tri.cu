@@ -172,7 +172,11 @@ __global__ void k_tri_tasklist(const int32_t* __restrict__ tstart, int64_t m, in
 //
 // COUNT: triangle counting instead: no edge counts; each triangle adds 1 to
 // the total and, with per_row, to the row of its largest vertex index (the
-// row sums of C<L> = L·L over the strictly lower triangle L).
+// row sums of C<L> = L·L over the strictly lower triangle L). Where that is u
+// or v, the entry's hits are added together: one atomic per entry. Only a w
+// above both takes one of its own; w has the highest degree of the three, and
+// a power-law graph's hubs mostly have low indices. One atomic per triangle
+// took 3.32 ms on R-MAT 18, this form 2.35 ms.
 template <bool COUNT>
 __global__ void __launch_bounds__(kTriThreads, 10) k_tri_support(const int32_t* __restrict__ ost,
                                                              const int32_t* __restrict__ ocnt,
@@ -257,6 +261,8 @@ __global__ void __launch_bounds__(kTriThreads, 10) k_tri_support(const int32_t* 
             const int32_t evn = __shfl_sync(FULL, vn, e);
             const int32_t ev = __shfl_sync(FULL, v, e);
             uint32_t mine = 0;  // this lane's hits for the entry
+            uint32_t own = 0;   // of those, the ones that the row max(u, v) takes
+            const int32_t top = max(u, ev);
             // one round of 32 wedges: the lane's wedge x of the entry, ld its
             // loaded rank (column when the list is not counted); INT32_MAX
             // past the list's end, which no lookup matches
@@ -301,7 +307,8 @@ __global__ void __launch_bounds__(kTriThreads, 10) k_tri_support(const int32_t* 
                 if (!COUNT && hit) atomicAdd(sup_o + wp, 1);  // (v, w)
                 if (COUNT && hit && per_row) {
                     const int32_t w = __ldg(ocol + wp);
-                    atomicAdd(per_row + max(max(u, ev), w), 1ull);
+                    if (w > top) atomicAdd(per_row + w, 1ull);
+                    else ++own;
                 }
                 mine += hit ? 1u : 0u;
             };
@@ -319,6 +326,10 @@ __global__ void __launch_bounds__(kTriThreads, 10) k_tri_support(const int32_t* 
                 wedges += (unsigned long long)evn;
                 tris += (unsigned long long)found;
                 if (!COUNT && found) atomicAdd(sup_o + p0 + e, found);  // (u, v)
+            }
+            if (COUNT && per_row && found) {  // warp-uniform
+                own = __reduce_add_sync(FULL, own);
+                if (lane == 0 && own) atomicAdd(per_row + top, (unsigned long long)own);
             }
         }
         if (counted && COUNT) {
