@@ -362,23 +362,37 @@ void mxm_masked_into(ga_ctx ctx, ga_algo algo, ga_csr A, ga_csr B, ga_csr M, voi
 ga_csr mxm_cmask(ga_ctx ctx, ga_csr A, ga_csr B, ga_csr M);
 // hybrid: room for the hybrid form's inner-product tasks too.
 size_t mxm_scratch_bytes(int64_t m, int64_t n, int64_t mask_nnz, bool hybrid = true);
+// Parts of rows: row i of A / B ends at a_end[i] / b_end[i] (nullptr: the
+// whole row). clip: with mask row ends, B rows are cut to the mask row's span
+// (false where they cannot leave it by much). counted: row starts of the mask
+// that the work counters count (nullptr: the mask as evaluated).
+struct MxmRows {
+    const int32_t* a_end = nullptr;
+    const int32_t* b_end = nullptr;
+    bool clip = true;
+    const int32_t* counted = nullptr;
+};
 // unit_a / unit_b: A's / B's values are all ones (skips value loads).
 // GA_HYBRID: Bt holds B^T (B itself when B is symmetric).
 void mxm_masked_launch(ga_ctx ctx, ga_algo algo, ga_csr A, ga_csr B, ga_csr M, void* d_cvals, void* scratch,
                        int64_t cap_nnz, bool unit_b, const int32_t* mask_row_end = nullptr, bool unit_a = false,
-                       ga_csr Bt = nullptr);
+                       ga_csr Bt = nullptr, const MxmRows& rows = MxmRows());
 // Inner-product masked product (GA_DOT): Bt holds B^T (B itself when B is
 // symmetric); unit: A's and B's values are all ones. Allocates nothing.
 // With mask_row_end, M->rst holds row starts of the mask and
-// mask_row_end - 1 the row partition of M's column array.
+// mask_row_end - 1 the row partition of M's column array. counted: as in
+// MxmRows.
 void mxm_dot_launch(ga_ctx ctx, ga_csr A, ga_csr B, ga_csr Bt, ga_csr M, void* d_cvals, bool unit,
-                    const int32_t* mask_row_end);
+                    const int32_t* mask_row_end, const int32_t* counted = nullptr);
 // True when every stored value of A equals 1 (computed once per handle and
 // cached; synchronises the stream the first time).
 bool csr_unit_values(ga_ctx ctx, ga_csr A);
 // True when A is square and every (i, j, v) has a matching (j, i, v)
 // (synchronises the stream).
 bool csr_is_symmetric(ga_ctx ctx, ga_csr A);
+// Values aligned with the symmetric A's entries: those above the diagonal
+// copied to their mirrors.
+void mirror_values(ga_ctx ctx, ga_csr A, void* vals, ga_dtype dt);
 // Batched BC over the block-diagonal union U of `count` graphs (host vertex
 // offsets voff), graph g with the sources [soff[g], soff[g+1]) of the host
 // array `sources` (indices within graph g); scores of U's rows into d_bc.

@@ -227,6 +227,41 @@ bool csr_is_symmetric(ga_ctx ctx, ga_csr A) {
     return A->sym == 1;
 }
 
+// Values of a symmetric result computed above the diagonal (and on it) copied
+// to their mirrors: v is aligned with the symmetric pattern r / c. Chunks as
+// above; the search is in row j of the entry (i, j), j > i, which for a
+// power-law graph is usually the shorter row.
+template <typename T>
+__global__ void k_mirror_values(const int32_t* __restrict__ r, const int32_t* __restrict__ c, int64_t m, int64_t nnz,
+                                T* v) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t ch = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; ch * kSymChunk < nnz; ch += warps) {
+        const int32_t q0 = (int32_t)(ch * kSymChunk);
+        const int32_t q1 = (int32_t)min(nnz, (int64_t)q0 + kSymChunk);
+        const int i0 = upper_bound_i32(r, (int)m + 1, q0) - 1;
+        const int i1 = upper_bound_i32(r, (int)m + 1, q1 - 1) - 1;
+        for (int32_t q = q0 + lane; q < q1; q += 32) {
+            const int i = i0 + upper_bound_i32(r + i0 + 1, i1 - i0, q);
+            const int32_t j = c[q];
+            if (j <= i) continue;
+            const int32_t jb = r[j], jn = r[j + 1] - jb;
+            const int pos = lower_bound_i32(c + jb, jn, (int32_t)i);
+            if (pos < jn) v[jb + pos] = v[q];
+        }
+    }
+}
+
+void mirror_values(ga_ctx ctx, ga_csr A, void* vals, ga_dtype dt) {
+    if (A->nnz == 0) return;
+    ProfScope ps(ctx, "mirror_values");
+    GA_DISPATCH_DTYPE(dt, T, {
+        k_mirror_values<T><<<grid_for((A->nnz + kSymChunk - 1) / kSymChunk * 32, 256, ctx->num_sms * 16), 256, 0,
+                             ctx->stream>>>(A->rst, A->col, A->m, A->nnz, static_cast<T*>(vals));
+    });
+    post_launch("mirror_values");
+}
+
 template <typename S, typename D>
 __global__ void k_convert(const S* __restrict__ s, D* __restrict__ d, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
