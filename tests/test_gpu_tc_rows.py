@@ -26,3 +26,21 @@ def test_tc_rows_whatever_the_hubs_indices(ctx, flip):
     total, rows = ga.tc("tri", to_device(ctx, G))
     ref_total, ref_rows = oracle.tc_sandia(G)
     assert total == ref_total and np.array_equal(rows, ref_rows)
+
+
+@pytest.mark.parametrize("algo", ["msa", "mca", "heap"])
+@pytest.mark.parametrize("n", [1, 2, 33, 300])
+def test_tc_straight_from_a(ctx, algo, n):
+    """The masked product of the lower parts without extracting them: a pattern
+    that is not symmetric, diagonal entries, rows without a lower part, values
+    that are not ones."""
+    from graphs import dense_to_csr
+    rng = np.random.default_rng(n)
+    D = rng.random((n, n)) < 0.3
+    D[n // 2] = np.arange(n) > n // 2
+    for dtype in (np.int32, np.float64, np.uint8):
+        G = dense_to_csr(D, rng.integers(1, 5, (n, n)), dtype)
+        ref_total, ref_rows = oracle.tc_sandia(oracle.Csr(n, n, G.rst, G.col, np.ones(len(G.col), np.int32)))
+        total, rows = ga.tc(algo, to_device(ctx, G))
+        assert total == ref_total and np.array_equal(rows, ref_rows)
+        assert ga.tc(algo, to_device(ctx, G), per_row=False)[0] == ref_total
