@@ -821,15 +821,13 @@ struct KtSweep {
         int it = 0;
         if (fused) {
             front->run(k);
-            const int64_t kept = front->compact(&it);
+            // the only wait: what follows runs while the caller takes the
+            // result and asks for the next k
+            const int64_t kept = front->result(&it);
             const int64_t m = W->m;
             out = csr_alloc(ctx, m, m, kept, GA_INT32);
             try {
-                GA_CUDA(cudaMemcpyAsync(out->rst, tr.p, sizeof(int32_t) * (size_t)(m + 1), cudaMemcpyDeviceToDevice,
-                                        ctx->stream));
-                if (kept)
-                    GA_CUDA(cudaMemcpyAsync(out->col, tc.p, sizeof(int32_t) * (size_t)kept, cudaMemcpyDeviceToDevice,
-                                            ctx->stream));
+                front->compact(out->rst, out->col);
                 fill_ones(ctx, out->val, kept, GA_INT32);
             } catch (...) {
                 csr_destroy(ctx, out);

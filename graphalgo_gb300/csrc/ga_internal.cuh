@@ -294,9 +294,10 @@ int tri_kt_frontier(ga_ctx ctx, ga_csr C, int k, const int32_t* row_of, const in
 // The same state kept between calls: run(k) iterates for one k (the first
 // call lists the triangles; a later call, one matrix only, takes a larger k
 // and continues from the supports the previous k left, so a sweep k = kmin,
-// kmin + 1, ... lists the triangles once); compact() writes the kept
-// entries, rows in column order, to b.tc / b.tr and returns their number and
-// the iteration count of the last run (one host synchronisation).
+// kmin + 1, ... lists the triangles once); result() gives the number of kept
+// entries and the iteration count of the last run (one host synchronisation);
+// compact() then writes the kept entries, rows in column order (col: as many
+// entries as kept).
 class TriFront {
 public:
     TriFront(ga_ctx ctx, ga_csr C, const int32_t* row_of, const int32_t* mir, const TriKt& t, int64_t cap,
@@ -305,7 +306,8 @@ public:
     TriFront(const TriFront&) = delete;
     TriFront& operator=(const TriFront&) = delete;
     void run(int k);
-    int64_t compact(int* iters);
+    int64_t result(int* iters);
+    void compact(int32_t* rst, int32_t* col);
 
 private:
     struct Impl;

@@ -41,6 +41,8 @@
 #include "ga_loop.cuh"
 
 #include <cstddef>
+#include <map>
+#include <mutex>
 
 namespace ga {
 
@@ -914,7 +916,16 @@ struct TriFrontState {
     int32_t nseg;                // segments of long rows listed this iteration
     uint32_t blocks_done;        // delta kernel: blocks finished
     uint32_t blocks_done_g;      // graph kernel (batches): blocks finished
+    // one-launch loop (k_trif_loop); [4]: by iteration
+    int32_t failed;              // a wait at its barrier ran out
+    int32_t nfront[4];           // frontier
+    int32_t nt[4], nf[4];        // touched vertices, flipped rows
+    unsigned long long nsegs[4]; // segments of the frontier's long rows
+    unsigned long long dd[4];    // change of P
+    unsigned long long dmask[4], dent[4];  // upper entries and entries that left
+    unsigned long long bar;      // arrivals at the barrier
     int32_t live;                // batches: graphs still iterating
+    int32_t diag;                // the matrix has diagonal entries
     unsigned long long prod;     // P_t (batches: summed over the live graphs)
     unsigned long long mask;     // entries (i, j) of C_t with j >= i
     unsigned long long ent;      // entries of C_t
@@ -959,6 +970,12 @@ struct TriFrontArgs {
     int32_t* cntg;          // 2 x ngraphs: frontier elements per graph, by iteration parity
     long long* pg;          // P per graph
     int64_t ngraphs;
+    // one-launch loop: further buffers (used in turn by the iterations), row
+    // lengths of the rows with a diagonal entry
+    int32_t *rd1, *rd2, *rh1, *rh2, *touched1, *touched2, *flip1, *flip2;
+    int32_t* dcur;
+    int2* seg1;
+    int64_t segcap1;        // of seg and seg1
 };
 
 __device__ __forceinline__ void front_push(int32_t* buf, int32_t* cnt, int32_t x) { buf[atomicAdd(cnt, 1)] = x; }
@@ -984,6 +1001,10 @@ __device__ __forceinline__ bool kt_frozen(const TriFrontArgs& a, int32_t i) {
 
 // One support unit less; the edge joins the next frontier when it drops below k - 2.
 __device__ __forceinline__ void lower_support(const TriFrontArgs& a, int32_t f, int32_t* fn, int32_t* cn, int par) {
+    if (!a.gid) {
+        if (atomicSub(a.sup + f, 1) == a.k - 2) front_push(fn, cn, f);
+        return;
+    }
     const int32_t i = a.row_of[f];
     if (atomicSub(a.sup + f, 1) == kt_thr(a, i)) front_add(a, fn, cn, f, i, par);
 }
@@ -1003,6 +1024,11 @@ __global__ void k_trif_init_rows(TriFrontArgs a) {
         a.rd[i] = 0;
         a.rh[i] = 0;
         a.mark[i] = 0;
+        if (a.dcur) {
+            a.rd1[i] = a.rd2[i] = 0;
+            a.rh1[i] = a.rh2[i] = 0;
+            a.dcur[i] = e - b;
+        }
     }
 }
 
@@ -1017,6 +1043,7 @@ __global__ void k_trif_seed(TriFrontArgs a) {
         // one matrix: a record of the first frontier is marked at once
         // (batches mark theirs in k_trif_mark)
         if (i == j) {
+            a.st->diag = 1;
             if (a.deg[i] < kt_thr(a, i)) {
                 front_add(a, a.f0, &a.st->cnt[0], (int32_t)q, i, 0);
                 if (!a.gid) a.state[q] = kDying;
@@ -1116,7 +1143,7 @@ __global__ void k_trif_mark(const TriFrontArgs* __restrict__ ap) {
 
 // Rows of at most this many entries are staged in shared memory (columns
 // and record positions) before the probes search them.
-constexpr int kTrifStage = 512;
+constexpr int kTrifStage = 256;  // (512: 2 % slower sweep, twice the shared memory)
 // An edge whose shorter row has more than kTrifSplit entries is walked in
 // segments of kTrifSeg entries by separate warps (k_trif_lower_seg).
 constexpr int kTrifSplit = 128;
@@ -1134,13 +1161,25 @@ struct TrifEdge {
     int target;
 };
 
-__device__ __forceinline__ TrifEdge trif_edge(const TriFrontArgs& a, int32_t q, int32_t u, int32_t v) {
+// The states of the records as an iteration sees them. The captured loop's
+// kernels mark them between the iterations.
+struct TrifMarked {
+    __device__ __forceinline__ uint8_t operator()(uint8_t s) const { return s; }
+};
+
+// diag: the matrix has diagonal entries.
+template <typename State>
+__device__ __forceinline__ TrifEdge trif_edge(const TriFrontArgs& a, int32_t q, int32_t u, int32_t v,
+                                              const State& now, bool diag) {
     TrifEdge e;
     e.q = q;
     e.u = u;
     e.v = v;
-    const int32_t du = a.dpos[u], dv = a.dpos[v];
-    e.target = a.sup[q] - (du >= 0 && a.state[du] != kGone) - (dv >= 0 && a.state[dv] != kGone);
+    e.target = a.sup[q];
+    if (diag) {
+        const int32_t du = a.dpos[u], dv = a.dpos[v];
+        e.target -= (du >= 0 && now(a.state[du]) != kGone) + (dv >= 0 && now(a.state[dv]) != kGone);
+    }
     const int32_t ub = a.cr[u], ue = a.cr[u + 1], vb = a.cr[v], ve = a.cr[v + 1];
     const bool xu = ue - ub <= ve - vb;  // walk the shorter row
     e.xb = xu ? ub : vb;
@@ -1154,46 +1193,131 @@ __device__ __forceinline__ TrifEdge trif_edge(const TriFrontArgs& a, int32_t q, 
     return e;
 }
 
-// Entry p of row x looked up in row y (scol / soid: y's columns and record
-// positions indexed from yb); loads only, so that a lane's lookups of
-// several entries overlap. A hit is the triangle (u, v, w): f and g are the
-// records of its other two edges (u or v, w) and (y, w), with their states.
+// Row y of an edge as the lookups see it: columns and record positions from
+// yb on, in shared memory (a short row) or in global memory; with shift > 0,
+// shared memory holds every 2^shift-th column, which leaves `shift` dependent
+// loads of a search in global memory (a hub's row took up to 15).
+struct TrifRow {
+    const int32_t* col;
+    const int32_t* oid;
+    const int32_t* fence;  // columns 0, 2^shift, 2 * 2^shift, ...
+    int shift;             // 0: none
+};
+
+// First position >= sb and < se (one of y's parts, sorted) whose column is at
+// least w; se if none.
+__device__ __forceinline__ int32_t trif_search(const TrifRow& y, int32_t sb, int32_t se, int32_t w) {
+    if (y.shift) {
+        // fences inside the part: i0 .. i1 - 1
+        const int32_t up = (1 << y.shift) - 1, i0 = (sb + up) >> y.shift, i1 = (se + up) >> y.shift;
+        const int32_t k = i0 + lower_bound_i32(y.fence + i0, i1 - i0, w);
+        if (k > i0) sb = ((k - 1) << y.shift) + 1;
+        if (k < i1) se = k << y.shift;
+    }
+    return sb + lower_bound_i32(y.col + sb, se - sb, w);
+}
+
+// Entry p of row x looked up in row y; loads only, and the independent ones
+// first, so that they overlap. A hit is the triangle (u, v, w): f and g are
+// the records of its other two edges (u or v, w) and (y, w), with their
+// states.
 struct TrifHit {
-    int32_t f, g;
+    int32_t f, g, w;
     uint8_t sf, sg;
     bool hit;
 };
 
-__device__ __forceinline__ TrifHit trif_find(const TriFrontArgs& a, const TrifEdge& e, int32_t p, const int32_t* scol,
-                                             const int32_t* soid) {
+template <typename State>
+__device__ __forceinline__ TrifHit trif_find(const TriFrontArgs& a, const TrifEdge& e, int32_t p, const TrifRow& y,
+                                             const State& now) {
     TrifHit h;
     h.hit = false;
-    h.f = h.g = 0;
-    h.sf = h.sg = kGone;
-    const int32_t w = a.cc[p];
-    if (w == e.u || w == e.v) return h;
+    h.g = 0;
+    h.sg = kGone;
+    const int32_t w = a.cc[p], rank = a.crank[p];
+    h.w = w;
     h.f = a.oid[p];
-    h.sf = a.state[h.f];
-    if (h.sf == kGone) return h;
+    h.sf = now(a.state[h.f]);
+    if (w == e.u || w == e.v) return h;
     // w ranked above y: (y, w) is in y's oriented part
-    const bool above = a.crank[p] > e.ry;
+    const bool above = rank > e.ry;
     const int32_t sb = above ? 0 : e.yo - e.yb, se = above ? e.yo - e.yb : e.ye - e.yb;
-    const int32_t r = sb + lower_bound_i32(scol + sb, se - sb, w);
-    if (r >= se || scol[r] != w) return h;
-    h.g = soid[r];
-    h.sg = a.state[h.g];
-    h.hit = h.sg != kGone;
+    const int32_t r = trif_search(y, sb, se, w);
+    if (r >= se || y.col[r] != w) return h;
+    h.g = y.oid[r];
+    h.sg = now(a.state[h.g]);
+    h.hit = h.sf != kGone && h.sg != kGone;
     return h;
 }
 
 // A hit lowers the supports of the triangle's other two edges, each once
 // (the frontier edge with the smallest record position owns a triangle with
-// two frontier edges).
-__device__ __forceinline__ void trif_apply_hit(const TriFrontArgs& a, const TrifEdge& e, const TrifHit& h, int32_t* fn,
-                                               int32_t* cn, int np) {
+// two frontier edges): lower(record, length of the row x or y, w).
+template <typename Lower>
+__device__ __forceinline__ void trif_apply_hit(const TrifEdge& e, const TrifHit& h, const Lower& lower) {
     if (!h.hit) return;
-    if (h.sf == kAlive && (h.sg == kAlive || e.q < h.g)) lower_support(a, h.f, fn, cn, np);
-    if (h.sg == kAlive && (h.sf == kAlive || e.q < h.f)) lower_support(a, h.g, fn, cn, np);
+    if (h.sf == kAlive && (h.sg == kAlive || e.q < h.g)) lower(h.f, e.xe - e.xb, h.w);
+    if (h.sg == kAlive && (h.sf == kAlive || e.q < h.f)) lower(h.g, e.ye - e.yb, h.w);
+}
+
+// A warp walks entries [p0, p1) of the edge's shorter row, 32 per pass (two
+// per lane per pass were slower: the later stop wastes more lookups than the
+// overlap gains), stopping once the edge's triangles are found. found: the
+// edge's count, shared by the warps that walk its segments (nullptr: this
+// warp walks the whole row).
+template <typename State, typename Lower>
+__device__ __forceinline__ void trif_walk(const TriFrontArgs& a, const TrifEdge& e, int32_t p0, int32_t p1,
+                                          const TrifRow& y, int32_t* found, const State& now, const Lower& lower,
+                                          unsigned long long& probes, unsigned long long& tris) {
+    const int lane = threadIdx.x & 31;
+    int mine = 0;
+    for (int32_t base = p0; base < p1; base += 32) {
+        const int32_t p = base + lane;
+        TrifHit h;
+        h.hit = false;
+        if (p < p1) {
+            ++probes;
+            h = trif_find(a, e, p, y, now);
+            trif_apply_hit(e, h, lower);
+        }
+        const int hcount = __popc(__ballot_sync(0xffffffffu, h.hit));
+        mine += hcount;
+        if (lane == 0) tris += (unsigned long long)hcount;
+        if (found) {
+            if (lane == 0)
+                mine = hcount ? atomicAdd(found, hcount) + hcount : *(volatile int32_t*)found;
+            mine = __shfl_sync(0xffffffffu, mine, 0);
+        }
+        if (mine >= e.target) break;
+    }
+}
+
+// The edge's other row through the warp's 2 * kTrifStage words of shared
+// memory: copied there (columns and record positions) when it has at most
+// kTrifStage entries, else its fences.
+__device__ __forceinline__ TrifRow trif_stage(const TriFrontArgs& a, const TrifEdge& e, int32_t* buf) {
+    const int lane = threadIdx.x & 31;
+    const int32_t n = e.ye - e.yb;
+    TrifRow y;
+    __syncwarp();  // the previous edge's lookups are done
+    if (n <= kTrifStage) {
+        for (int32_t i = lane; i < n; i += 32) {
+            buf[i] = a.cc[e.yb + i];
+            buf[kTrifStage + i] = a.oid[e.yb + i];
+        }
+        y.col = buf;
+        y.oid = buf + kTrifStage;
+        y.shift = 0;
+    } else {
+        y.shift = 1;
+        while (((n - 1) >> y.shift) >= 2 * kTrifStage) ++y.shift;
+        for (int32_t i = lane; i <= (n - 1) >> y.shift; i += 32) buf[i] = a.cc[e.yb + (i << y.shift)];
+        y.col = a.cc + e.yb;
+        y.oid = a.oid + e.yb;
+    }
+    y.fence = buf;
+    __syncwarp();
+    return y;
 }
 
 // One warp per frontier edge: its triangles in C_t, the supports they lower.
@@ -1204,18 +1328,16 @@ __device__ __forceinline__ void trif_apply_hit(const TriFrontArgs& a, const Trif
 // A row x longer than kTrifSplit is listed as segments for
 // k_trif_lower_seg instead (while the segment list has room).
 __global__ void __launch_bounds__(128, 8) k_trif_lower(const TriFrontArgs* __restrict__ ap) {
-    __shared__ int32_t s_col[4][kTrifStage];
-    __shared__ int32_t s_oid[4][kTrifStage];
+    __shared__ int32_t s_row[4][2 * kTrifStage];
     const TriFrontArgs a = *ap;
     const int lane = threadIdx.x & 31;
-    int32_t* ycol = s_col[threadIdx.x >> 5];
-    int32_t* yoid = s_oid[threadIdx.x >> 5];
     const int t = a.st->t;
     const int32_t n = a.st->cnt[t & 1];
     const int32_t* F = (t & 1) ? a.f1 : a.f0;
     int32_t* fn = (t & 1) ? a.f0 : a.f1;
     int32_t* cn = &a.st->cnt[(t + 1) & 1];
     const int np = (t + 1) & 1;
+    auto lower = [&](int32_t f, int32_t, int32_t) { lower_support(a, f, fn, cn, np); };
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     unsigned long long probes = 0, tris = 0, edges = 0;
     for (int64_t x = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < n; x += warps) {
@@ -1232,7 +1354,7 @@ __global__ void __launch_bounds__(128, 8) k_trif_lower(const TriFrontArgs* __res
             }
             continue;
         }
-        const TrifEdge e = trif_edge(a, q, u, v);
+        const TrifEdge e = trif_edge(a, q, u, v, TrifMarked(), true);
         if (e.target <= 0) continue;
         if (e.xe - e.xb > kTrifSplit) {
             // segments for k_trif_lower_seg: (frontier slot, segment)
@@ -1249,35 +1371,7 @@ __global__ void __launch_bounds__(128, 8) k_trif_lower(const TriFrontArgs* __res
             for (int64_t j = base + lane; j < a.segcap && j < (int64_t)base + nseg; j += 32)
                 a.seg[j] = make_int2(-1, 0);
         }
-        const bool staged = e.ye - e.yb <= kTrifStage;
-        if (staged) {
-            __syncwarp();  // the previous edge's lookups are done
-            for (int32_t i = lane; i < e.ye - e.yb; i += 32) {
-                ycol[i] = a.cc[e.yb + i];
-                yoid[i] = a.oid[e.yb + i];
-            }
-            __syncwarp();
-        }
-        const int32_t* scol = staged ? ycol : a.cc + e.yb;
-        const int32_t* soid = staged ? yoid : a.oid + e.yb;
-        // 32 entries per pass, stopping once the edge's triangles are found
-        // (two entries per lane per pass were slower: the later stop wastes
-        // more lookups than the overlap gains)
-        int found = 0;
-        for (int32_t base = e.xb; base < e.xe; base += 32) {
-            const int32_t p = base + lane;
-            TrifHit h;
-            h.hit = false;
-            if (p < e.xe) {
-                ++probes;
-                h = trif_find(a, e, p, scol, soid);
-                trif_apply_hit(a, e, h, fn, cn, np);
-            }
-            const int hcount = __popc(__ballot_sync(0xffffffffu, h.hit));
-            found += hcount;
-            if (lane == 0) tris += (unsigned long long)hcount;
-            if (found >= e.target) break;
-        }
+        trif_walk(a, e, e.xb, e.xe, trif_stage(a, e, s_row[threadIdx.x >> 5]), nullptr, TrifMarked(), lower, probes, tris);
     }
     probes = warp_sum<unsigned long long>(probes);
     if (lane == 0) {
@@ -1299,6 +1393,7 @@ __global__ void __launch_bounds__(128, 8) k_trif_lower_seg(const TriFrontArgs* _
     int32_t* fn = (t & 1) ? a.f0 : a.f1;
     int32_t* cn = &a.st->cnt[(t + 1) & 1];
     const int np = (t + 1) & 1;
+    auto lower = [&](int32_t f, int32_t, int32_t) { lower_support(a, f, fn, cn, np); };
     const int64_t ns = min((int64_t)a.st->nseg, a.segcap);
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     unsigned long long probes = 0, tris = 0;
@@ -1306,29 +1401,11 @@ __global__ void __launch_bounds__(128, 8) k_trif_lower_seg(const TriFrontArgs* _
         const int2 sg = a.seg[sx];
         if (sg.x < 0) continue;
         const int32_t q = F[sg.x];
-        const TrifEdge e = trif_edge(a, q, a.row_of[q], a.cc[q]);
+        const TrifEdge e = trif_edge(a, q, a.row_of[q], a.cc[q], TrifMarked(), true);
         if (*(volatile int32_t*)(a.efound + sg.x) >= e.target) continue;
         const int32_t s0 = e.xb + sg.y * kTrifSeg, s1 = min(e.xe, s0 + kTrifSeg);
-        const int32_t* scol = a.cc + e.yb;
-        const int32_t* soid = a.oid + e.yb;
-        for (int32_t base = s0; base < s1; base += 32) {
-            const int32_t p = base + lane;
-            TrifHit h;
-            h.hit = false;
-            if (p < s1) {
-                ++probes;
-                h = trif_find(a, e, p, scol, soid);
-                trif_apply_hit(a, e, h, fn, cn, np);
-            }
-            const int hcount = __popc(__ballot_sync(0xffffffffu, h.hit));
-            int before = 0;
-            if (lane == 0) {
-                tris += (unsigned long long)hcount;
-                before = hcount ? atomicAdd(a.efound + sg.x, hcount) : *(volatile int32_t*)(a.efound + sg.x);
-            }
-            before = __shfl_sync(0xffffffffu, before, 0);
-            if (before + hcount >= e.target) break;
-        }
+        const TrifRow y{a.cc + e.yb, a.oid + e.yb, nullptr, 0};
+        trif_walk(a, e, s0, s1, y, a.efound + sg.x, TrifMarked(), lower, probes, tris);
     }
     probes = warp_sum<unsigned long long>(probes);
     if (lane == 0) {
@@ -1493,6 +1570,410 @@ __global__ void __launch_bounds__(256) k_trif_delta(const TriFrontArgs* __restri
     loop_continue(ctl, st->done == 0);
 }
 
+// ------------------------------------------------- the loop in one launch
+// One matrix, device loops: the iterations of a run(k) inside one cooperative
+// launch, one CTA per SM, one grid barrier per iteration. As five kernels per
+// iteration of a captured loop, an iteration with a few hundred frontier edges
+// took 35 us and its loop node 8 more, most of it launches, their tails and
+// chains of dependent loads; here it takes 13 to 16 us, of which the barrier is
+// 2.3 and the rest the longest chain (queue entry, edge, rows, staging, lookup,
+// support, queue). R-MAT 18 sweep, 1,412 iterations: 33.5 ms of 54 in the loop,
+// 56 of 86 before (two barriers per iteration, the parts of an iteration one
+// after the other: 47.5 of 74). Frontiers above 4,096 edges (167 iterations, 12
+// ms) are bound by how many of these chains 32 warps per SM have in flight.
+//
+// What an iteration needs from the one before is only its frontier and the
+// supports, so stage s runs
+//   A(s)    the frontier's triangles lower the supports (k_trif_lower),
+//           queueing and marking the edges that cross k - 2 for s + 1
+//   B(s-1)  the counts of what left in iteration s - 1 (k_trif_apply)
+//   C(s-2)  the rows that lost their last upper entry in iteration s - 2
+//           lower their neighbours' H (k_trif_flip)
+//   D(s-3)  the vertices touched in iteration s - 3 get their new row lengths
+//           and H, and P its change (k_trif_delta); its edges become kGone
+// side by side, and three stages after the last iteration settle the rest.
+// * A queued edge's state is the code 3 + (its iteration mod 5) until D: in
+//   stage s the code of s + 1 means alive, of s dying, of s - 1 .. s - 3 gone,
+//   and the code of s - 4 (that of s + 1) is no longer in use.
+// * Every edge leaves once, so all frontiers of a run share one list, one
+//   after the other; iteration t's counters are slot t mod 4 (reset by the
+//   settling thread when nothing reads them), its buffers t mod 3, and a row
+//   flipped in iteration t has h = 2 + t mod 3 until C.
+// * A diagonal entry joins the next frontier when its row becomes too short,
+//   which B finds: with diagonal entries B(s) runs in stage s, behind a
+//   barrier of its own.
+// * A long row is cut into segments when its edge is queued; while the
+//   frontier is small, so that most warps are idle, from 33 entries on.
+constexpr int kTrifLoopThreads = 1024;
+constexpr int kTrifLoopWarps = kTrifLoopThreads / 32;
+constexpr size_t kTrifLoopSmem = (size_t)kTrifLoopWarps * kTrifStage * 2 * sizeof(int32_t);
+constexpr int kTrifFine = 8;  // warps of the grid per frontier edge from which rows are cut finely
+constexpr long long kTrifWaitCycles = 20000000000ll;  // about ten seconds at 2 GHz
+
+// All CTAs of the launch (cooperative: they are resident together) have
+// arrived `round` times. False when a wait ran out, here or elsewhere.
+__device__ __forceinline__ bool trif_barrier(TriFrontState* st, unsigned long long round) {
+    __shared__ bool s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned long long all = round * gridDim.x;
+        if (atomicAdd(&st->bar, 1ull) + 1ull < all) {
+            const long long t0 = clock64();
+            while (*(volatile unsigned long long*)&st->bar < all) {
+                if (*(volatile int32_t*)&st->failed) break;
+                if (clock64() - t0 > kTrifWaitCycles) {
+                    atomicExch(&st->failed, 1);
+                    break;
+                }
+            }
+        }
+        __threadfence();
+        s_ok = *(volatile int32_t*)&st->failed == 0;
+    }
+    __syncthreads();
+    return s_ok;
+}
+
+__device__ __forceinline__ uint8_t trif_code(int t) { return (uint8_t)(3 + t % 5); }
+
+// The states in stage s.
+struct TrifCoded {
+    uint8_t next, dying;
+    __device__ __forceinline__ explicit TrifCoded(int s) : next(trif_code(s + 1)), dying(trif_code(s)) {}
+    __device__ __forceinline__ uint8_t operator()(uint8_t v) const {
+        return v == kAlive || v == next ? kAlive : v == dying ? kDying : kGone;
+    }
+};
+
+// Segments of the shorter row (len entries) of the edge at place x of the
+// frontier list; efound says whether they were listed.
+__device__ __forceinline__ void trif_cut(const TriFrontArgs& a, int32_t x, int32_t len, bool fine, int2* seg,
+                                         unsigned long long* nsegs) {
+    int32_t listed = -1;
+    if (len > (fine ? 32 : kTrifSplit)) {
+        const int per = fine ? 32 : kTrifSeg, n = (len + per - 1) / per;
+        const int64_t base = (int64_t)atomicAdd(nsegs, (unsigned long long)n);
+        if (base + n <= a.segcap1) listed = 0;
+        for (int64_t j = 0; j < n && base + j < a.segcap1; ++j)
+            seg[base + j] = make_int2(listed < 0 ? -1 : x, (int32_t)(2 * j) | (fine ? 1 : 0));
+    }
+    a.efound[x] = listed;
+}
+
+__global__ void __launch_bounds__(kTrifLoopThreads, 1) k_trif_loop(const __grid_constant__ TriFrontArgs a) {
+    extern __shared__ int32_t s_rows[];
+    TriFrontState* st = a.st;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int32_t* buf = s_rows + (size_t)wid * 2 * kTrifStage;
+    // warps of one CTA lie apart, so that few items spread over the SMs
+    const int64_t warp = (int64_t)wid * gridDim.x + blockIdx.x, warps = (int64_t)gridDim.x * kTrifLoopWarps;
+    const int64_t thread = warp * 32 + lane, threads = warps * 32;
+    // each part of a stage starts at another quarter of the warps: with few
+    // items, the parts run on different warps instead of one after the other
+    auto quarter = [&](int q) {
+        const int64_t w = warp - q * (warps / 4);
+        return w < 0 ? w + warps : w;
+    };
+    const int64_t warp_b = quarter(1), warp_c = quarter(2), thread_d = quarter(3) * 32 + lane;
+    // the thread that keeps the totals: of the warp that gets work last
+    const bool settles = thread == threads - 32;
+    const bool diag = st->diag != 0;
+    const int thr = a.k - 2;
+    int32_t* const F = a.f0;
+    unsigned long long round = 0, probes = 0, tris = 0, edges = 0;
+
+    // P_it (its change by iteration it - 1 is known), the counters of
+    // iteration `it` when it counts, and what left in it. One thread.
+    auto settle = [&](int it, bool count) {
+        if (it > 0) {
+            st->prod += *(volatile unsigned long long*)&st->dd[(it - 1) & 3];
+            st->dd[(it - 1) & 3] = 0;
+        }
+        if (count) trif_count_iteration(a);
+        st->mask -= *(volatile unsigned long long*)&st->dmask[it & 3];
+        st->ent -= *(volatile unsigned long long*)&st->dent[it & 3];
+        st->dmask[it & 3] = 0;
+        st->dent[it & 3] = 0;
+    };
+    // Vertices x (lanes with `is`) newly touched in iteration `it`, listed.
+    auto list_touched = [&](int it, bool is, int32_t x) {
+        const unsigned b = __ballot_sync(FULL, is);
+        if (b == 0u) return;
+        int32_t at = 0;
+        if (lane == 0) at = atomicAdd(&st->nt[it & 3], __popc(b));
+        at = __shfl_sync(FULL, at, 0);
+        const int r = it % 3;
+        int32_t* list = r == 0 ? a.touched : r == 1 ? a.touched1 : a.touched2;
+        if (is) list[at + __popc(b & ((1u << lane) - 1u))] = x;
+    };
+
+    // Queueing for iteration it + 1 from stage `it`: record f, whose edge's
+    // shorter row has len entries (0: a diagonal entry).
+    auto queue = [&](int it, int64_t next_at, bool fine, int32_t f, int32_t len) {
+        const int32_t x = (int32_t)next_at + atomicAdd(&st->nfront[(it + 1) & 3], 1);
+        F[x] = f;
+        a.state[f] = trif_code(it + 1);
+        trif_cut(a, x, len, fine, it & 1 ? a.seg : a.seg1, &st->nsegs[(it + 1) & 3]);
+    };
+
+    // A(s): items [0, n) the frontier, then its segments
+    auto lower_stage = [&](int s, int64_t at, int64_t n, int64_t ns, bool fine) {
+        const TrifCoded now(s);
+        const int64_t next_at = at + n;
+        const int2* seg = s & 1 ? a.seg1 : a.seg;
+        auto lower = [&](int32_t f, int32_t len, int32_t w) {
+            if (atomicSub(a.sup + f, 1) == thr) queue(s, next_at, fine, f, min(len, a.cr[w + 1] - a.cr[w]));
+        };
+        for (int64_t x0 = warp; x0 < n + ns; x0 += warps * 32) {
+            // the warp's next 32 items, one per lane: their chains of loads
+            // overlap
+            const int64_t x = x0 + (int64_t)lane * warps;
+            TrifEdge e = {};
+            int32_t slot = -1, p0 = 0, p1 = 0;
+            bool todo = false;
+            if (x < n) {
+                const int32_t q = F[at + x];
+                const int32_t cut = a.efound[at + x];
+                const int32_t u = a.row_of[q], v = a.cc[q];
+                ++edges;
+                if (u == v) {
+                    e.u = e.v = u;
+                    todo = true;
+                } else if (cut < 0) {
+                    e = trif_edge(a, q, u, v, now, diag);
+                    p0 = e.xb;
+                    p1 = e.xe;
+                    todo = e.target > 0;
+                }
+            } else if (x < n + ns) {
+                const int2 sg = seg[x - n];
+                if (sg.x >= 0) {
+                    slot = sg.x;
+                    const int32_t q = F[slot], per = sg.y & 1 ? 32 : kTrifSeg;
+                    e = trif_edge(a, q, a.row_of[q], a.cc[q], now, diag);
+                    p0 = e.xb + (sg.y >> 1) * per;
+                    p1 = min(e.xe, p0 + per);
+                    todo = *(volatile int32_t*)(a.efound + slot) < e.target;
+                }
+            }
+            for (unsigned set = __ballot_sync(FULL, todo); set; set &= set - 1) {
+                const int l = __ffs(set) - 1;
+                TrifEdge f;
+                f.u = __shfl_sync(FULL, e.u, l);
+                f.v = __shfl_sync(FULL, e.v, l);
+                if (f.u == f.v) {  // a diagonal entry leaves: every other edge of its row loses 1
+                    for (int32_t p = a.cr[f.u] + lane; p < a.cr[f.u + 1]; p += 32) {
+                        const int32_t w = a.cc[p];
+                        if (w == f.u) continue;
+                        const int32_t r = a.oid[p];
+                        if (now(a.state[r]) == kAlive) lower(r, a.cr[f.u + 1] - a.cr[f.u], w);
+                    }
+                    __syncwarp();
+                    continue;
+                }
+                f.q = __shfl_sync(FULL, e.q, l);
+                f.xb = __shfl_sync(FULL, e.xb, l);
+                f.xe = __shfl_sync(FULL, e.xe, l);
+                f.yb = __shfl_sync(FULL, e.yb, l);
+                f.yo = __shfl_sync(FULL, e.yo, l);
+                f.ye = __shfl_sync(FULL, e.ye, l);
+                f.ry = __shfl_sync(FULL, e.ry, l);
+                f.target = __shfl_sync(FULL, e.target, l);
+                const int32_t b = __shfl_sync(FULL, p0, l), c = __shfl_sync(FULL, p1, l);
+                const int32_t sl = __shfl_sync(FULL, slot, l);
+                trif_walk(a, f, b, c, trif_stage(a, f, buf), sl < 0 ? nullptr : a.efound + sl, now, lower, probes, tris);
+            }
+        }
+    };
+    // B(it)
+    auto leave_stage = [&](int it, int64_t at, int64_t n, int64_t next_at) {
+        const int r = it % 3, bit = r;
+        int32_t* rd = r == 0 ? a.rd : r == 1 ? a.rd1 : a.rd2;
+        int32_t* rh = r == 0 ? a.rh : r == 1 ? a.rh1 : a.rh2;
+        int32_t* flip = r == 0 ? a.flip : r == 1 ? a.flip1 : a.flip2;
+        const uint8_t flipping = (uint8_t)(2 + r);
+        unsigned long long mask = 0, ent = 0;
+        for (int64_t x0 = warp_b * 32; x0 < n; x0 += threads) {  // whole warps: they reserve places together
+            int32_t u = -1, v = -1, lo = 0, du = -1, dv = -1;
+            bool tu = false, tv = false, fl = false;  // newly touched, flipped
+            if (x0 + lane < n) {
+                const int32_t q = F[at + x0 + lane];
+                u = a.row_of[q];
+                v = a.cc[q];
+                ++mask;
+                lo = min(u, v);
+                // what is read or returned does not wait for one another
+                const uint8_t su = a.h[u], sv = a.h[v];
+                if (diag && u != v) {
+                    du = a.dpos[u];
+                    dv = a.dpos[v];
+                }
+                const int32_t mu = atomicOr(a.mark + u, 1 << bit);
+                const int32_t mv = u == v ? -1 : atomicOr(a.mark + v, 1 << bit);
+                const int32_t up = atomicSub(a.upc + lo, 1);
+                atomicAdd(rd + u, 1);
+                if (u != v) atomicAdd(rd + v, 1);
+                // h as of the iteration's start: 1, or flipped in it
+                if (u == v || su == 1 || su == flipping) atomicAdd(rh + v, 1);
+                if (u != v && (sv == 1 || sv == flipping)) atomicAdd(rh + u, 1);
+                tu = !(mu >> bit & 1);
+                tv = !(mv >> bit & 1);
+                fl = up == 1;
+                ent += u == v ? 1 : 2;
+            }
+            list_touched(it, tu, u);
+            list_touched(it, tv, v);
+            const unsigned bf = __ballot_sync(FULL, fl);
+            if (bf) {
+                int32_t af = 0;
+                if (lane == 0) af = atomicAdd(&st->nf[it & 3], __popc(bf));
+                af = __shfl_sync(FULL, af, 0);
+                if (fl) {
+                    flip[af + __popc(bf & ((1u << lane) - 1u))] = lo;
+                    a.h[lo] = flipping;
+                }
+            }
+            // a row that lost an entry: its diagonal entry may become too short
+            if (du >= 0 && atomicSub(a.dcur + u, 1) == thr && a.state[du] == kAlive) queue(it, next_at, false, du, 0);
+            if (dv >= 0 && atomicSub(a.dcur + v, 1) == thr && a.state[dv] == kAlive) queue(it, next_at, false, dv, 0);
+            __syncwarp();
+        }
+        mask = warp_sum<unsigned long long>(mask);
+        ent = warp_sum<unsigned long long>(ent);
+        if (lane == 0 && mask) {
+            atomicAdd(&st->dmask[it & 3], mask);
+            atomicAdd(&st->dent[it & 3], ent);
+        }
+    };
+    // C(it), in stage it + 2: the entries present after iteration `it`
+    auto flip_stage = [&](int it) {
+        const int32_t n = *(volatile int32_t*)&st->nf[it & 3];
+        const int r = it % 3;
+        const int32_t* flip = r == 0 ? a.flip : r == 1 ? a.flip1 : a.flip2;
+        int32_t* rh = r == 0 ? a.rh : r == 1 ? a.rh1 : a.rh2;
+        const uint8_t c1 = trif_code(it + 1), c2 = trif_code(it + 2), c3 = trif_code(it + 3);
+        for (int64_t x = warp_c; x < n; x += warps) {
+            const int32_t i = flip[x];
+            if (lane == 0) a.h[i] = 0;
+            const int32_t e = a.cr[i + 1];
+            for (int32_t b = a.cr[i]; b < e; b += 32) {
+                int32_t j = 0;
+                bool is = false;
+                if (b + lane < e) {
+                    j = a.cc[b + lane];
+                    const uint8_t v = a.state[a.oid[b + lane]];
+                    if (v == kAlive || v == c1 || v == c2 || v == c3) {
+                        atomicAdd(rh + j, 1);
+                        is = !(atomicOr(a.mark + j, 1 << r) >> r & 1);
+                    }
+                }
+                list_touched(it, is, j);
+            }
+        }
+    };
+    // D(it), in stage it + 3
+    auto delta_stage = [&](int it, int64_t at, int64_t nleft) {
+        for (int64_t x = thread_d; x < nleft; x += threads) a.state[F[at + x]] = kGone;
+        const int32_t n = *(volatile int32_t*)&st->nt[it & 3];
+        const int r = it % 3;
+        const int32_t* list = r == 0 ? a.touched : r == 1 ? a.touched1 : a.touched2;
+        int32_t* rd = r == 0 ? a.rd : r == 1 ? a.rd1 : a.rd2;
+        int32_t* rh = r == 0 ? a.rh : r == 1 ? a.rh1 : a.rh2;
+        long long d = 0;
+        for (int64_t x = thread_d; x < n; x += threads) {
+            const int32_t j = list[x];
+            const long long od = a.deg[j], oh = a.H[j];
+            const long long nd = od - rd[j], nh = oh - rh[j];
+            d += nd * nh - od * oh;
+            a.deg[j] = (int32_t)nd;
+            a.H[j] = (int32_t)nh;
+            rd[j] = 0;
+            rh[j] = 0;
+            atomicAnd(a.mark + j, ~(1 << r));
+        }
+        d = warp_sum<long long>(d);
+        if (lane == 0 && d) atomicAdd(&st->dd[it & 3], (unsigned long long)d);
+    };
+
+    // the first frontier: its edges get their code and are cut
+    const int64_t n0 = st->cnt[0];
+    bool fine = n0 * kTrifFine < warps;
+    for (int64_t x = thread; x < n0; x += threads) {
+        const int32_t q = F[x], u = a.row_of[q], v = a.cc[q];
+        a.state[q] = trif_code(0);
+        trif_cut(a, (int32_t)x, u == v ? 0 : min(a.cr[u + 1] - a.cr[u], a.cr[v + 1] - a.cr[v]), fine, a.seg,
+                 &st->nsegs[0]);
+    }
+    bool ok = trif_barrier(st, ++round);
+    int64_t n = n0, at = 0;          // this iteration's frontier
+    int64_t n1 = 0, n2 = 0, n3 = 0;  // those of the three before
+    int last = -1;                   // last iteration with a frontier; -1: not known yet
+    int64_t nleft = 0, left_at = 0;  // queued when the bound stopped the loop
+    bool ended = false, bound = false;
+    for (int s = 0; ok; ++s) {
+        if (!ended) {
+            if (s > 0) n = *(volatile int32_t*)&st->nfront[s & 3];
+            if (n == 0) {
+                ended = true;
+                last = s - 1;
+            }
+        } else {
+            n = 0;
+        }
+        if (ended && s > last + 3) break;
+        if (ended && last < 0) break;
+        const int64_t ns = n ? min((int64_t)*(volatile unsigned long long*)&st->nsegs[s & 3], a.segcap1) : 0;
+        fine = n * kTrifFine < warps;
+        if (settles) {
+            if (s >= 3) settle(s - 3, s - 3 <= last || !ended);
+            st->nfront[(s + 2) & 3] = 0;
+            st->nsegs[(s + 2) & 3] = 0;
+            st->nt[s & 3] = 0;
+            st->nf[s & 3] = 0;
+        }
+        if (n) lower_stage(s, at, n, ns, fine);
+        if (n1 && !diag) leave_stage(s - 1, at - n1, n1, 0);
+        if (n2) flip_stage(s - 2);
+        if (n3) delta_stage(s - 3, at - n1 - n2 - n3, n3);
+        if (!(ok = trif_barrier(st, ++round))) break;
+        if (n && diag) {
+            leave_stage(s, at, n, at + n);
+            if (!(ok = trif_barrier(st, ++round))) break;
+        }
+        at += n;
+        n3 = n2;
+        n2 = n1;
+        n1 = n;
+        // the reference's bound: m iterations
+        if (!ended && (int64_t)(s + 1) >= a.m) {
+            ended = bound = true;
+            last = s;
+            nleft = *(volatile int32_t*)&st->nfront[(s + 1) & 3];
+            left_at = at;
+        }
+    }
+    // (present in C while they had their code)
+    for (int64_t x = thread; x < nleft; x += threads) a.state[F[left_at + x]] = kDying;
+    if (ok && settles) {
+        // the iterations not settled yet (the last one that ran is `last`
+        // when the bound stopped the loop, else the empty one after it)
+        const int end = bound ? last : last + 1;
+        for (int it = last < 0 ? 0 : last + 1; it <= last + 1; ++it) settle(it, it <= end);
+        st->iters = bound ? 0 : end + 1;
+        st->t = end;
+        st->done = 1;
+    }
+    probes = warp_sum<unsigned long long>(probes);
+    edges = warp_sum<unsigned long long>(edges);
+    if (lane == 0) {
+        if (edges) atomicAdd(&a.ctr[GA_CTR_FRONT_EDGES], edges);
+        if (probes) atomicAdd(&a.ctr[GA_CTR_FRONT_PROBES], probes);
+        if (tris) atomicAdd(&a.ctr[GA_CTR_FRONT_TRIANGLES], tris);
+    }
+}
+
 // Batches, end of iteration t, one thread per graph: a live graph without
 // frontier elements in this iteration has converged (iteration count t + 1),
 // one that reached its bound stops with count 0 (n_g iterations, as the
@@ -1577,6 +2058,25 @@ __global__ void k_trif_out(TriFrontArgs a, const int32_t* __restrict__ pos, int3
 
 }  // namespace
 
+// One CTA of the one-launch loop fits every SM of the context's device.
+static bool trif_loop_fits(ga_ctx ctx) {
+    static std::mutex mu;
+    static std::map<int, bool> known;  // per device
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find(ctx->device);
+    if (it != known.end()) return it->second;
+    int coop = 0, per_sm = 0;
+    const bool ok =
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) == cudaSuccess && coop &&
+        cudaFuncSetAttribute(k_trif_loop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrifLoopSmem) ==
+            cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trif_loop, kTrifLoopThreads, kTrifLoopSmem) ==
+            cudaSuccess &&
+        per_sm >= 1;
+    cudaGetLastError();
+    return known[ctx->device] = ok;
+}
+
 struct TriFront::Impl {
     ga_ctx ctx;
     ga_csr C;
@@ -1586,6 +2086,8 @@ struct TriFront::Impl {
     const KtBatch* batch;
     int64_t ng;
     DBuf<int32_t> deg, upc, H, rd, rh, mark, touched, flip;
+    bool one_launch;                   // the loop in one cooperative launch
+    DBuf<int32_t> rd1, rd2, rh1, rh2, flip2, dcur;
     DBuf<uint8_t> h;
     DBuf<TriFrontState> st;
     DBuf<int32_t> cntg;
@@ -1600,7 +2102,12 @@ struct TriFront::Impl {
         : ctx(ctx_), C(C_), t(t_), cap(cap_), b(b_), batch(batch_), ng(batch_ ? batch_->ngraphs : 0),
           deg(ctx_, (size_t)C_->m + 1), upc(ctx_, (size_t)C_->m + 1), H(ctx_, (size_t)C_->m + 1),
           rd(ctx_, (size_t)C_->m + 1), rh(ctx_, (size_t)C_->m + 1), mark(ctx_, (size_t)C_->m + 1),
-          touched(ctx_, (size_t)C_->m + 1), flip(ctx_, (size_t)C_->m + 1), h(ctx_, (size_t)C_->m + 1),
+          touched(ctx_, (size_t)C_->m + 1), flip(ctx_, (size_t)C_->m + 1),
+          one_launch(!batch_ && ctx_->device_loops && trif_loop_fits(ctx_)),
+          rd1(ctx_, one_launch ? (size_t)C_->m + 1 : 1), rd2(ctx_, one_launch ? (size_t)C_->m + 1 : 1),
+          rh1(ctx_, one_launch ? (size_t)C_->m + 1 : 1), rh2(ctx_, one_launch ? (size_t)C_->m + 1 : 1),
+          flip2(ctx_, one_launch ? (size_t)C_->m + 1 : 1), dcur(ctx_, one_launch ? (size_t)C_->m + 1 : 1),
+          h(ctx_, (size_t)C_->m + 1),
           st(ctx_, 1), cntg(ctx_, batch_ ? (size_t)(2 * batch_->ngraphs) : 1),
           pg(ctx_, batch_ ? (size_t)batch_->ngraphs : 1),
           seg(ctx_, (size_t)std::max<int64_t>(cap_ / 8, 4096)), efound(ctx_, (size_t)cap_) {
@@ -1646,6 +2153,20 @@ struct TriFront::Impl {
         a.cntg = batch ? cntg.p : nullptr;
         a.pg = batch ? pg.p : nullptr;
         a.ngraphs = ng;
+        // one-launch loop: its frontiers share f0, so f1 holds segments; b.tc,
+        // b.flag and b.tr are free until compact() (touched vertices have
+        // entries, so they are at most cap)
+        a.rd1 = rd1.p;
+        a.rd2 = rd2.p;
+        a.rh1 = rh1.p;
+        a.rh2 = rh2.p;
+        a.touched1 = b.tc;
+        a.touched2 = b.flag;
+        a.flip1 = b.tr;
+        a.flip2 = flip2.p;
+        a.dcur = one_launch ? dcur.p : nullptr;
+        a.seg1 = reinterpret_cast<int2*>(b.f1);
+        a.segcap1 = std::min<int64_t>(a.segcap, cap / 2);
     }
 
     void run(int k) {
@@ -1675,6 +2196,19 @@ struct TriFront::Impl {
                 k_trif_reseed<<<grid_ent, 256, 0, ctx->stream>>>(a);
                 post_launch("trif_reseed");
             }
+        }
+        if (one_launch) {
+            ProfScope ps(ctx, "ktruss_loop");
+            void* args[] = {&a};
+            if (cudaLaunchCooperativeKernel((const void*)k_trif_loop, dim3(ctx->num_sms), dim3(kTrifLoopThreads), args,
+                                            kTrifLoopSmem, ctx->stream) == cudaSuccess) {
+                post_launch("trif_loop");
+                return;
+            }
+            // the device cannot hold the whole grid at once (part of it is set
+            // aside): the captured loop serves
+            cudaGetLastError();
+            one_launch = false;
         }
         if (!batch) {
             k_trif_begin<<<1, 32, 0, ctx->stream>>>(a);
@@ -1724,22 +2258,25 @@ struct TriFront::Impl {
         run_cached_loop(ctx, slot, body, m + 1);
     }
 
-    int64_t compact(int* iters) {
+    // Entries kept and iteration count of the last run (one synchronisation).
+    int64_t result(int* iters) {
+        TriFrontState hs;
+        GA_CUDA(cudaMemcpyAsync(&hs, st.p, sizeof(TriFrontState), cudaMemcpyDeviceToHost, ctx->stream));
+        GA_CUDA(cudaStreamSynchronize(ctx->stream));
+        GA_REQUIRE(!hs.failed, GA_ERR_TIMEOUT, "k-truss: a wait inside the loop ran out");
+        if (iters) *iters = hs.iters;
+        return (int64_t)hs.ent;
+    }
+
+    // The kept entries' row starts and columns, rows in column order.
+    void compact(int32_t* rst, int32_t* col) {
         const int64_t m = a.m, nnz = a.nnz;
         ProfScope ps(ctx, "trif_compact");
         k_trif_keep<<<grid_for(cap, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(a, cap, b.flag);
         post_launch("trif_keep");
         scan_exclusive_i32_scratch(ctx, b.flag, b.flag, cap, b.scan_scr);
-        k_trif_out<<<grid_for(nnz > m ? nnz : m + 1, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a, b.flag, b.tc,
-                                                                                                 b.tr);
+        k_trif_out<<<grid_for(nnz > m ? nnz : m + 1, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a, b.flag, col, rst);
         post_launch("trif_out");
-        TriFrontState hs;
-        int32_t kept = 0;
-        GA_CUDA(cudaMemcpyAsync(&hs, st.p, sizeof(TriFrontState), cudaMemcpyDeviceToHost, ctx->stream));
-        GA_CUDA(cudaMemcpyAsync(&kept, b.tr + m, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-        GA_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (iters) *iters = hs.iters;
-        return kept;
     }
 };
 
@@ -1751,14 +2288,17 @@ TriFront::~TriFront() { delete impl_; }
 
 void TriFront::run(int k) { impl_->run(k); }
 
-int64_t TriFront::compact(int* iters) { return impl_->compact(iters); }
+int64_t TriFront::result(int* iters) { return impl_->result(iters); }
+
+void TriFront::compact(int32_t* rst, int32_t* col) { impl_->compact(rst, col); }
 
 int tri_kt_frontier(ga_ctx ctx, ga_csr C, int k, const int32_t* row_of, const int32_t* mir, const TriKt& t,
                     int64_t cap, const TriFrontBufs& b, const KtBatch* batch) {
     TriFront f(ctx, C, row_of, mir, t, cap, b, batch);
     f.run(k);
     int iters = 0;
-    const int64_t kept = f.compact(&iters);
+    const int64_t kept = f.result(&iters);
+    f.compact(b.tr, b.tc);
     const int64_t m = C->m;
     GA_CUDA(cudaMemcpyAsync(C->rst, b.tr, sizeof(int32_t) * (size_t)(m + 1), cudaMemcpyDeviceToDevice, ctx->stream));
     if (kept) GA_CUDA(cudaMemcpyAsync(C->col, b.tc, sizeof(int32_t) * (size_t)kept, cudaMemcpyDeviceToDevice,
