@@ -204,6 +204,19 @@ int csr_check_bits(ga_ctx ctx, const int32_t* rst, const int32_t* col, int64_t m
 // merge-path merges). nnz: entries of the whole matrix.
 void sort_rows_by_key(ga_ctx ctx, const int32_t* rst, int64_t m, int32_t* key, int32_t* pay, int64_t nnz);
 
+// Stable sort of n keys of `bits` bits, with a payload (or nullptr), between
+// the two buffers; true when the result is in tkeys / tpay.
+bool radix_sort_u64(ga_ctx ctx, uint64_t* keys, uint64_t* tkeys, int32_t* pay, int32_t* tpay, int64_t n, int bits);
+bool radix_sort_u32(ga_ctx ctx, uint32_t* keys, uint32_t* tkeys, int32_t* pay, int32_t* tpay, int64_t n, int bits);
+// Bits of the integers 0 .. n - 1.
+inline int bits_for(int64_t n) {
+    int b = 0;
+    while (((int64_t)1 << b) < n) ++b;
+    return b;
+}
+// Row starts of sorted keys row << shift | ...: rst[i] = keys below row i.
+void rows_of_keys(ga_ctx ctx, const uint64_t* keys, int64_t n, int shift, int64_t m, int32_t* rst);
+
 // k-truss on a single matrix (batch == nullptr) or on a block-diagonal union
 // of graphs with per-graph convergence (see ga_batch_ktruss).
 struct KtBatch {

@@ -297,28 +297,24 @@ ga_csr copy_csr(ga_ctx ctx, ga_csr A, ga_dtype to) {
     return C;
 }
 
-// ================================================================ transpose
-__global__ void k_count_cols(const int32_t* __restrict__ col, int64_t nnz, int32_t* __restrict__ cnt) {
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd(&cnt[col[q]], 1);
-}
-
-// Scatter: entry (i, j) goes to AT row j at an atomically reserved position;
-// the row index is recorded with the source entry index for the sort.
-__global__ void k_transpose_scatter(const int32_t* __restrict__ rst, const int32_t* __restrict__ col, int64_t m,
-                                    int32_t* __restrict__ cursor, int32_t* __restrict__ trow,
-                                    int32_t* __restrict__ tsrc) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += warps) {
-        for (int32_t q = rst[i] + lane; q < rst[i + 1]; q += 32) {
-            int32_t p = atomicAdd(&cursor[col[q]], 1);
-            trow[p] = (int32_t)i;
-            tsrc[p] = q;
+__global__ void k_rows_of_keys(const uint64_t* __restrict__ key, int64_t n, int shift, int64_t m,
+                               int32_t* __restrict__ rst) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= m; i += (int64_t)gridDim.x * blockDim.x) {
+        int64_t lo = 0, hi = n;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if ((int64_t)(key[mid] >> shift) < i) lo = mid + 1; else hi = mid;
         }
+        rst[i] = (int32_t)lo;
     }
 }
 
+void rows_of_keys(ga_ctx ctx, const uint64_t* keys, int64_t n, int shift, int64_t m, int32_t* rst) {
+    k_rows_of_keys<<<grid_for(m + 1, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(keys, n, shift, m, rst);
+    post_launch("rows_of_keys");
+}
+
+// ================================================================ transpose
 // Sort every row segment by key with a block-wide bitonic sort in shared
 // memory; the payload follows its key. Rows longer than kSortCap are listed
 // in long_rows (count in *nlong) for k_sort_long_rows.
@@ -552,36 +548,60 @@ void sort_rows_by_key(ga_ctx ctx, const int32_t* rst, int64_t m, int32_t* key, i
     GA_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 
+// Transpose by a stable sort of the columns: the entries keep their rows'
+// order inside every column, so the result's rows come sorted. R-MAT 18's
+// lower triangle (3.8M entries) in 210 us; counted and scattered with atomics
+// and sorted row by row it took 1,310 us (10,500 entries: 49 and 86 us).
+__global__ void k_sorted_rst(const uint32_t* __restrict__ key, int64_t nnz, int64_t n, int32_t* __restrict__ rst) {
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j <= n; j += (int64_t)gridDim.x * blockDim.x) {
+        int64_t lo = 0, hi = nnz;  // keys below j
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if ((int64_t)key[mid] < j) lo = mid + 1; else hi = mid;
+        }
+        rst[j] = (int32_t)lo;
+    }
+}
+
+__global__ void k_iota(int32_t* __restrict__ v, int64_t n) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        v[i] = (int32_t)i;
+}
+
 template <typename T>
-__global__ void k_gather_vals(const int32_t* __restrict__ src, const T* __restrict__ v, T* __restrict__ out,
-                              int64_t n) {
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x)
-        out[q] = v[src[q]];
+__global__ void k_transpose_gather(const int32_t* __restrict__ src, const int32_t* __restrict__ row_of,
+                                   const T* __restrict__ v, int64_t nnz, int32_t* __restrict__ col,
+                                   T* __restrict__ val) {
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t s = src[q];
+        col[q] = row_of[s];
+        val[q] = v[s];
+    }
 }
 
 ga_csr transpose_csr(ga_ctx ctx, ga_csr A) {
     ProfScope ps(ctx, "transpose");
-    ga_csr T = csr_alloc(ctx, A->n, A->m, A->nnz, A->dtype);
+    const int64_t nnz = A->nnz;
+    ga_csr T = csr_alloc(ctx, A->n, A->m, nnz, A->dtype);
     try {
-        DBuf<int32_t> cnt(ctx, (size_t)A->n + 1);
-        GA_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int32_t) * (A->n + 1), ctx->stream));
-        if (A->nnz) {
-            k_count_cols<<<grid_for(A->nnz, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(A->col, A->nnz, cnt.p);
-            post_launch("transpose_count");
+        DBuf<uint32_t> key(ctx, (size_t)nnz), tkey(ctx, (size_t)nnz);
+        DBuf<int32_t> src(ctx, (size_t)nnz), tsrc(ctx, (size_t)nnz), row_of(ctx, (size_t)nnz);
+        const int grid = grid_for(nnz, 256, ctx->num_sms * 8);
+        if (nnz) {
+            GA_CUDA(cudaMemcpyAsync(key.p, A->col, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, ctx->stream));
+            k_iota<<<grid, 256, 0, ctx->stream>>>(src.p, nnz);
+            post_launch("iota");
+            expand_rows(ctx, A, row_of.p);
         }
-        scan_exclusive_i32(ctx, cnt.p, T->rst, A->n);
-        if (A->nnz) {
-            DBuf<int32_t> cursor(ctx, (size_t)A->n + 1);
-            DBuf<int32_t> src(ctx, (size_t)A->nnz);
-            GA_CUDA(cudaMemcpyAsync(cursor.p, T->rst, sizeof(int32_t) * (A->n + 1), cudaMemcpyDeviceToDevice,
-                                    ctx->stream));
-            k_transpose_scatter<<<grid_for(A->m * 32, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-                A->rst, A->col, A->m, cursor.p, T->col, src.p);
-            post_launch("transpose_scatter");
-            sort_rows_by_key(ctx, T->rst, T->m, T->col, src.p, A->nnz);
+        const bool other = radix_sort_u32(ctx, key.p, tkey.p, src.p, tsrc.p, nnz, bits_for(A->n));
+        k_sorted_rst<<<grid_for(A->n + 1, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(other ? tkey.p : key.p, nnz,
+                                                                                        A->n, T->rst);
+        post_launch("transpose_rst");
+        if (nnz) {
             GA_DISPATCH_DTYPE(A->dtype, V, {
-                k_gather_vals<V><<<grid_for(A->nnz, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
-                    src.p, static_cast<const V*>(A->val), static_cast<V*>(T->val), A->nnz);
+                k_transpose_gather<V><<<grid, 256, 0, ctx->stream>>>(other ? tsrc.p : src.p, row_of.p,
+                                                                     static_cast<const V*>(A->val), nnz, T->col,
+                                                                     static_cast<V*>(T->val));
             });
             post_launch("transpose_gather");
         }
@@ -611,17 +631,24 @@ __global__ void k_tri_count(const int32_t* __restrict__ rst, const int32_t* __re
     }
 }
 
+// One warp per chunk of consecutive output entries (balanced whatever the row
+// lengths: one warp per row took 175 us on R-MAT 18, this form 35 us).
 template <typename T>
 __global__ void k_tri_copy(const int32_t* __restrict__ first, const int32_t* __restrict__ orst,
-                           const int32_t* __restrict__ col, const T* __restrict__ val, int64_t m,
+                           const int32_t* __restrict__ col, const T* __restrict__ val, int64_t m, int64_t nnz,
                            int32_t* __restrict__ ocol, T* __restrict__ oval) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += warps) {
-        int32_t s = first[i], o = orst[i], len = orst[i + 1] - orst[i];
-        for (int32_t t = lane; t < len; t += 32) {
-            ocol[o + t] = col[s + t];
-            oval[o + t] = val[s + t];
+    for (int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c * kSymChunk < nnz; c += warps) {
+        const int32_t q0 = (int32_t)(c * kSymChunk);
+        const int32_t q1 = (int32_t)min(nnz, (int64_t)q0 + kSymChunk);
+        const int i0 = upper_bound_i32(orst, (int)m + 1, q0) - 1;
+        const int i1 = upper_bound_i32(orst, (int)m + 1, q1 - 1) - 1;
+        for (int32_t q = q0 + lane; q < q1; q += 32) {
+            const int i = i0 + upper_bound_i32(orst + i0 + 1, i1 - i0, q);
+            const int32_t s = first[i] + (q - orst[i]);
+            ocol[q] = col[s];
+            oval[q] = val[s];
         }
     }
 }
@@ -639,8 +666,9 @@ ga_csr extract_tri(ga_ctx ctx, ga_csr A, bool lower) {
         GA_CUDA(cudaMemcpyAsync(L->rst, rst.p, sizeof(int32_t) * (A->m + 1), cudaMemcpyDeviceToDevice, ctx->stream));
         if (nnz) {
             GA_DISPATCH_DTYPE(A->dtype, T, {
-                k_tri_copy<T><<<grid_for(A->m * 32, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-                    first.p, rst.p, A->col, static_cast<const T*>(A->val), A->m, L->col, static_cast<T*>(L->val));
+                k_tri_copy<T><<<grid_for((nnz / kSymChunk + 1) * 32, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+                    first.p, rst.p, A->col, static_cast<const T*>(A->val), A->m, nnz, L->col,
+                    static_cast<T*>(L->val));
             });
             post_launch("tri_copy");
         }
@@ -656,28 +684,36 @@ ga_csr extract_tri(ga_ctx ctx, ga_csr A, bool lower) {
 // comes first (the tie rule of build_symm_from_lower and add_nointersect,
 // include/matrix.h:713-720, include/matrix_la.h:351-357). Every element finds
 // its output position by a binary search in the other row.
+// One warp per chunk of kSymChunk consecutive entries of X, then of Y
+// (balanced whatever the row lengths: one warp per row took 778 us for the
+// R-MAT 18 lower triangle and its transpose, this form 100 us).
 template <typename T>
 __global__ void k_merge_rows(const int32_t* __restrict__ xr, const int32_t* __restrict__ xc,
                              const T* __restrict__ xv, const int32_t* __restrict__ yr,
-                             const int32_t* __restrict__ yc, const T* __restrict__ yv, int64_t m,
-                             const int32_t* __restrict__ cr, int32_t* __restrict__ cc, T* __restrict__ cv) {
+                             const int32_t* __restrict__ yc, const T* __restrict__ yv, int64_t m, int64_t xnnz,
+                             int64_t ynnz, const int32_t* __restrict__ cr, int32_t* __restrict__ cc,
+                             T* __restrict__ cv) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < m; i += warps) {
-        int32_t xb = xr[i], xn = xr[i + 1] - xb;
-        int32_t yb = yr[i], yn = yr[i + 1] - yb;
-        int32_t o = cr[i];
-        for (int32_t t = lane; t < xn; t += 32) {
-            int32_t c = xc[xb + t];
-            int p = upper_bound_i32(yc + yb, yn, c);
-            cc[o + t + p] = c;
-            cv[o + t + p] = xv[xb + t];
-        }
-        for (int32_t t = lane; t < yn; t += 32) {
-            int32_t c = yc[yb + t];
-            int p = lower_bound_i32(xc + xb, xn, c);
-            cc[o + t + p] = c;
-            cv[o + t + p] = yv[yb + t];
+    const int64_t xch = (xnnz + kSymChunk - 1) / kSymChunk, ych = (ynnz + kSymChunk - 1) / kSymChunk;
+    for (int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < xch + ych; c += warps) {
+        const bool x = c < xch;
+        const int32_t* r = x ? xr : yr;
+        const int32_t* own = x ? xc : yc;
+        const int32_t* other_r = x ? yr : xr;
+        const int32_t* other = x ? yc : xc;
+        const T* val = x ? xv : yv;
+        const int32_t q0 = (int32_t)((x ? c : c - xch) * kSymChunk);
+        const int32_t q1 = (int32_t)min(x ? xnnz : ynnz, (int64_t)q0 + kSymChunk);
+        const int i0 = upper_bound_i32(r, (int)m + 1, q0) - 1;
+        const int i1 = upper_bound_i32(r, (int)m + 1, q1 - 1) - 1;
+        for (int32_t q = q0 + lane; q < q1; q += 32) {
+            const int i = i0 + upper_bound_i32(r + i0 + 1, i1 - i0, q);
+            const int32_t col = own[q], ob = other_r[i], on = other_r[i + 1] - ob;
+            const int p = x ? upper_bound_i32(other + ob, on, col) : lower_bound_i32(other + ob, on, col);
+            const int32_t o = cr[i] + (q - r[i]) + p;
+            cc[o] = col;
+            cv[o] = val[q];
         }
     }
 }
@@ -695,9 +731,9 @@ static ga_csr merge_csr(ga_ctx ctx, ga_csr X, ga_csr Y) {
         post_launch("add_rst");
         if (C->nnz) {
             GA_DISPATCH_DTYPE(X->dtype, T, {
-                k_merge_rows<T><<<grid_for(X->m * 32, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+                k_merge_rows<T><<<grid_for((C->nnz / kSymChunk + 2) * 32, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
                     X->rst, X->col, static_cast<const T*>(X->val), Y->rst, Y->col, static_cast<const T*>(Y->val),
-                    X->m, C->rst, C->col, static_cast<T*>(C->val));
+                    X->m, X->nnz, Y->nnz, C->rst, C->col, static_cast<T*>(C->val));
             });
             post_launch("merge_rows");
         }
