@@ -11,18 +11,22 @@
 //     drains the CTA queue, then every warp drains the warp queue. The
 //     accumulator is indexed by mask slot and lives in shared memory.
 //     Column -> slot lookup per variant:
-//       GA_MSA  : a dense bitmap of the window's mask columns in shared memory
-//                 (the reference MSA keeps a dense state array over the
+//       GA_MSA, : a dense bitmap of the window's mask columns in shared memory
+//       GA_MCA    (the reference MSA keeps a dense state array over the
 //                 columns, matrix_la.h:681-749); a set bit is resolved to its
 //                 slot as the word's first slot plus a popcount (the
 //                 slot base is kept per 32-column word). Warp rows use a
-//                 4096-bit hashed filter and a 512-entry hash table.
-//       GA_MCA  : binary search of the sorted mask row in shared memory (the
-//                 reference MCA walks the mask row, matrix_la.h:625-632),
-//                 after a membership test that rejects the columns outside
-//                 the mask (most products of a k-truss support miss it): a
-//                 bitmap over the window (CTA items) or the 4096-bit hashed
-//                 filter (warp rows);
+//                 4096-bit hashed filter and a 512-entry hash table. The
+//                 accumulator is the mask row's entries, which is MCA's too:
+//                 the reference MCA finds the entry by walking the mask row
+//                 (matrix_la.h:625-632), here the rank of the set bit is it.
+//                 A binary search of the mask row behind the same filters
+//                 was slower at every size tried: a 50,021 x 40,009 product of
+//                 1e8 products under 24-entry mask rows 914 us against 631 in
+//                 FP64 and 721 against 417 in int32, 1,000 x 1,000 with 10
+//                 entries per row 141 against 128, R-MAT 16 support 2,764
+//                 against 1,162, 32-entry rows under 2-entry masks 1,947
+//                 against 945;
 //       GA_HEAP : sorted merge of each B row against the mask row
 //                 (replaces the priority-queue merge,
 //                 matrix_la.h:1030-1084): lanes take 32 A entries; a B row
@@ -273,17 +277,16 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
 }
 
 // ------------------------------------------------------------------ lookups
-// MODE: how a product's column finds its mask slot.
-// MD_BSEARCH: CTA items (window bitmap, then search); MD_BSEARCH_F: warp
-// rows (hashed filter, then search).
-enum { MD_DENSE = 0, MD_HASHED = 1, MD_BSEARCH = 2, MD_MERGE = 3, MD_BSEARCH_F = 4 };
+// How a product's column finds its mask slot: MD_DENSE in CTA items, MD_HASHED
+// in warp rows; MD_MERGE merges whole B rows instead.
+enum { MD_DENSE = 0, MD_HASHED = 1, MD_MERGE = 2 };
 
 // The mask columns of one work item, staged in shared memory.
 struct SlotView {
-    const int32_t* mcol;    // MD_BSEARCH(_F) / MD_MERGE: sorted mask columns
-    const uint32_t* bits;   // MD_DENSE, MD_BSEARCH: bitmap over [lo, lo + kWinCols)
+    const int32_t* mcol;    // MD_MERGE: sorted mask columns
+    const uint32_t* bits;   // MD_DENSE: bitmap over [lo, lo + kWinCols)
     const uint16_t* wbase;  // MD_DENSE: slot of the first mask column of each bitmap word
-    const uint32_t* filt;   // MD_HASHED, MD_BSEARCH_F: 4096-bit filter of hashed columns
+    const uint32_t* filt;   // MD_HASHED: 4096-bit filter of hashed columns
     const int32_t* hkeys;   // MD_HASHED: open-addressing table (2^kWarpTblBits)
     const uint8_t* hslot;
     int ns;
@@ -301,7 +304,7 @@ __device__ __forceinline__ int slot_of(const SlotView& v, int32_t c) {
         const uint32_t b = d & 31;
         if (!((w >> b) & 1u)) return -1;
         return (int)v.wbase[d >> 5] + __popc(w & ((1u << b) - 1u));
-    } else if (MD == MD_HASHED) {
+    } else {
         const uint32_t h = hash_col(c);
         const uint32_t f = h >> (32 - kFilterBits);
         if (!((v.filt[f >> 5] >> (f & 31)) & 1u)) return -1;
@@ -313,17 +316,6 @@ __device__ __forceinline__ int slot_of(const SlotView& v, int32_t c) {
             if (key == kEmpty) return -1;
             pos = (pos + 1) & mask;
         }
-    } else {
-        if (c < v.lo || c > v.hi) return -1;
-        if (MD == MD_BSEARCH) {
-            const uint32_t d = (uint32_t)(c - v.lo);
-            if (!((v.bits[d >> 5] >> (d & 31)) & 1u)) return -1;
-        } else if (MD == MD_BSEARCH_F) {
-            const uint32_t f = hash_col(c) >> (32 - kFilterBits);
-            if (!((v.filt[f >> 5] >> (f & 31)) & 1u)) return -1;
-        }
-        const int pos = lower_bound_i32(v.mcol, v.ns, c);
-        return (pos < v.ns && v.mcol[pos] == c) ? pos : -1;
     }
 }
 
@@ -711,25 +703,22 @@ __device__ __forceinline__ int64_t merge_group(const MxmArgs<T, A>& p, int32_t t
 template <int MD, typename A>
 struct MxmSmem {
     static constexpr bool dense = MD == MD_DENSE;
-    static constexpr bool filt = MD == MD_BSEARCH;  // bitmap / hashed filter in front of the search
     // CTA phase
     static constexpr size_t off_acc = 0;
     static constexpr size_t off_lbs = off_acc + (size_t)kCtaSlots * sizeof(A);
     static constexpr size_t off_lend = off_lbs + (size_t)kLongCap * 4;
     static constexpr size_t off_lchunk = off_lend + (size_t)kLongCap * 4;
     static constexpr size_t off_la = off_lchunk + (size_t)(kLongCap + 8) * 4;
-    static constexpr size_t off_key = off_la + (size_t)kLongCap * sizeof(A);  // bits+wbase, bits+mcol or mcol
+    static constexpr size_t off_key = off_la + (size_t)kLongCap * sizeof(A);  // bits and wbase, or mcol
     static constexpr size_t off_wbase = off_key + (size_t)kWinWords * 4;
-    static constexpr size_t off_fcol = off_key + (size_t)kWinWords * 4;  // MCA: mcol after the bitmap
-    static constexpr size_t cta_bytes = dense  ? off_wbase + (size_t)kWinWords * 2
-                                        : filt ? off_fcol + (size_t)kCtaSlots * 4
-                                               : off_key + (size_t)kCtaSlots * 4;
-    // warp phase (per warp): acc, hashed filter + table (MSA) or mcol (others)
+    static constexpr size_t cta_bytes =
+        dense ? off_wbase + (size_t)kWinWords * 2 : off_key + (size_t)kCtaSlots * 4;
+    // warp phase (per warp): acc, hashed filter and table, or mcol
     static constexpr size_t w_acc = 0;
     static constexpr size_t w_filt = w_acc + (size_t)kWarpSlots * sizeof(A);
     static constexpr size_t w_hkeys = w_filt + (size_t)(1 << kFilterBits) / 8;
     static constexpr size_t w_hslot = w_hkeys + (size_t)(1 << kWarpTblBits) * 4;
-    static constexpr size_t w_mcol = filt ? w_filt + (size_t)(1 << kFilterBits) / 8 : w_filt;
+    static constexpr size_t w_mcol = w_filt;
     static constexpr size_t warp_one =
         dense ? w_hslot + (size_t)(1 << kWarpTblBits) : w_mcol + (size_t)kWarpSlots * 4;
     static constexpr size_t warp_bytes = warp_one * kMxmWarps;
@@ -744,9 +733,7 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
     extern __shared__ __align__(16) unsigned char smem[];
     using SM = MxmSmem<MD, A>;
     constexpr bool DENSE = MD == MD_DENSE;
-    constexpr bool FILT = MD == MD_BSEARCH;   // MCA: membership filters in front of the search
-    constexpr bool BITS = DENSE || FILT;      // CTA items keep a window bitmap
-    constexpr int WMD = DENSE ? MD_HASHED : FILT ? MD_BSEARCH_F : MD;  // warp-row lookup
+    constexpr int WMD = DENSE ? MD_HASHED : MD;  // warp-row lookup
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned char* scr = smem + SM::region;
@@ -765,8 +752,8 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
         A* la = reinterpret_cast<A*>(smem + SM::off_la);
         uint32_t* bits = reinterpret_cast<uint32_t*>(smem + SM::off_key);
         uint16_t* wbase = reinterpret_cast<uint16_t*>(smem + SM::off_wbase);
-        int32_t* mcol = reinterpret_cast<int32_t*>(smem + (FILT ? SM::off_fcol : SM::off_key));
-        if (BITS)
+        int32_t* mcol = reinterpret_cast<int32_t*>(smem + SM::off_key);
+        if (DENSE)
             for (int t = threadIdx.x; t < kWinWords; t += blockDim.x) bits[t] = 0u;
         const int nheavy = p.q->heavy_count;
         const int ncta = nheavy + p.q->normal_count;
@@ -796,10 +783,6 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
                     if (s == 0 || ((uint32_t)(__ldg(gcol + s - 1) - v.lo) >> 5) != (d >> 5)) wbase[d >> 5] = (uint16_t)s;
                 } else {
                     mcol[s] = c;
-                    if (FILT) {
-                        const uint32_t d = (uint32_t)(c - v.lo);
-                        atomicOr(&bits[d >> 5], 1u << (d & 31));
-                    }
                 }
             }
             __syncthreads();
@@ -863,7 +846,7 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
             __syncthreads();
             for (int s = threadIdx.x; s < ns; s += blockDim.x) {
                 p.cv[mb + s0 + s] = from_acc<T, A>(acc[s]);
-                if (BITS) bits[(uint32_t)(__ldg(gcol + s) - v.lo) >> 5] = 0u;
+                if (DENSE) bits[(uint32_t)(__ldg(gcol + s) - v.lo) >> 5] = 0u;
             }
             __syncthreads();
         }
@@ -879,7 +862,7 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
         int32_t* mcol = reinterpret_cast<int32_t*>(base + SM::w_mcol);
         constexpr int FW = (1 << kFilterBits) / 32;
         constexpr int TBL = 1 << kWarpTblBits;
-        if (DENSE || FILT)
+        if (DENSE)
             for (int t = lane; t < FW; t += 32) filt[t] = 0u;
         if (DENSE)
             for (int t = lane; t < TBL; t += 32) hkeys[t] = kEmpty;
@@ -908,10 +891,6 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
                     hash_insert<uint8_t>(hkeys, hslot, kWarpTblBits, c, (uint8_t)s);
                 } else {
                     mcol[s] = c;
-                    if (FILT) {
-                        const uint32_t f = hash_col(c) >> (32 - kFilterBits);
-                        atomicOr(&filt[f >> 5], 1u << (f & 31));
-                    }
                 }
             }
             __syncwarp();
@@ -927,7 +906,7 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
             }
             __syncwarp();
             for (int s = lane; s < mi; s += 32) p.cv[mb + s] = from_acc<T, A>(acc[s]);
-            if (DENSE || FILT)
+            if (DENSE)
                 for (int t = lane; t < FW; t += 32) filt[t] = 0u;
             if (DENSE)
                 for (int t = lane; t < TBL; t += 32) hkeys[t] = kEmpty;
@@ -948,7 +927,7 @@ static int64_t cta_item_cap(int64_t m, int64_t n, int64_t mask_nnz) {
 // Launch the masked product for one value type and lookup variant.
 template <int LK, int VM, typename T>
 static void launch_masked(ga_ctx ctx, ga_csr A_, ga_csr B_, ga_csr M_, T* cv, MxmQueue* q, int32_t* warp_rows,
-                          int4* cta_items, int32_t cta_cap, const int32_t* mre, const MxmRows& rows,
+                          int4* cta_items, int32_t cta_cap, const int32_t* mre, const MxmRows& rows, const char* name,
                           const int32_t* btr = nullptr, int2* dot_tasks = nullptr) {
     using Ac = typename Acc<T>::type;
     MxmArgs<T, Ac> p;
@@ -982,7 +961,6 @@ static void launch_masked(ga_ctx ctx, ga_csr A_, ga_csr B_, ga_csr M_, T* cv, Mx
     GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMxmThreads, smem));
     if (per_sm < 1) per_sm = 1;
     if (ctx->tune.ctas_per_sm > 0 && ctx->tune.ctas_per_sm < per_sm) per_sm = ctx->tune.ctas_per_sm;
-    const char* name = LK == MD_DENSE ? "mxm_msa" : LK == MD_BSEARCH ? "mxm_mca" : "mxm_heap_merge";
     ProfScope ps(ctx, name);
     kern<<<ctx->num_sms * per_sm, kMxmThreads, smem, ctx->stream>>>(p);
     post_launch(name);
@@ -1286,23 +1264,25 @@ void mxm_masked_launch(ga_ctx ctx, ga_algo algo, ga_csr A, ga_csr B, ga_csr M, v
             const int32_t* btr = Bt->rst;
             if (ones)
                 launch_masked<MD_DENSE, 2, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows,
-                                              btr, dot_tasks);
+                                              "mxm_msa", btr, dot_tasks);
             else if (unit_b)
                 launch_masked<MD_DENSE, 1, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows,
-                                              btr, dot_tasks);
+                                              "mxm_msa", btr, dot_tasks);
             else
                 launch_masked<MD_DENSE, 0, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows,
-                                              btr, dot_tasks);
+                                              "mxm_msa", btr, dot_tasks);
             launch_dot_t<T>(ctx, A, B, Bt, M, cv, unit_a && unit_b, mask_row_end, rows.counted, dot_tasks, q);
-        } else if (algo == GA_MSA) {
-            if (ones) launch_masked<MD_DENSE, 2, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows);
-            else if (unit_b) launch_masked<MD_DENSE, 1, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows);
-            else launch_masked<MD_DENSE, 0, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows);
-        } else if (algo == GA_MCA) {
-            if (unit_b) launch_masked<MD_BSEARCH, 1, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows);
-            else launch_masked<MD_BSEARCH, 0, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows);
+        } else if (algo == GA_MSA || algo == GA_MCA) {
+            const char* name = algo == GA_MSA ? "mxm_msa" : "mxm_mca";
+            if (ones)
+                launch_masked<MD_DENSE, 2, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows, name);
+            else if (unit_b)
+                launch_masked<MD_DENSE, 1, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows, name);
+            else
+                launch_masked<MD_DENSE, 0, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows, name);
         } else {
-            launch_masked<MD_MERGE, 0, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows);
+            launch_masked<MD_MERGE, 0, T>(ctx, A, B, M, cv, q, warp_rows, cta_items, c32, mask_row_end, rows,
+                                          "mxm_heap_merge");
         }
     });
 }

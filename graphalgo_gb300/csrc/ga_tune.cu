@@ -58,9 +58,9 @@ std::vector<Cand> product_candidates(bool dot_ok, int only, bool tri_ok = false)
         c.push_back({GA_MSA, tune_of(32768, 1, 8)});
         c.push_back({GA_MSA, tune_of(131072, 1, 8)});
     }
-    if (only < 0 || only == GA_MCA) {
+    if (only == GA_MCA) {  // runs MSA's kernel: no candidate of its own among the others
         c.push_back({GA_MCA, MxmTune()});
-        if (only == GA_MCA) c.push_back({GA_MCA, tune_of(131072, 0, 8)});
+        c.push_back({GA_MCA, tune_of(131072, 0, 8)});
     }
     if (dot_ok && (only < 0 || only == GA_DOT))
         for (int chunk : {4, 8, 16}) c.push_back({GA_DOT, tune_of(32768, 0, chunk)});
