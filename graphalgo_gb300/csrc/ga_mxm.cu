@@ -53,10 +53,15 @@ namespace ga {
 
 constexpr int kMxmThreads = 512;
 constexpr int kMxmWarps = kMxmThreads / 32;
-constexpr int kCtaSlots = 4096;            // mask slots per CTA work item
+// Mask slots per CTA work item and per warp row. Half as many of 8 bytes: the
+// third CTA fits on an SM then (75 KB each instead of 90), FP64 products of
+// 200,000 x 200,000 under 8-entry mask rows 1,695 -> 1,484 us, 50,021 x
+// 40,009 under 32-entry rows 2,195 -> 2,104.
+template <typename A> constexpr int kCtaSlots = sizeof(A) == 8 ? 2048 : 4096;
+template <typename A> constexpr int kWarpSlots = sizeof(A) == 8 ? 128 : 256;
+constexpr int kLeastCtaSlots = 2048;
 constexpr int kWinCols = 1 << 17;          // column span of a CTA work item
 constexpr int kWinWords = kWinCols / 32;   // dense bitmap words
-constexpr int kWarpSlots = 256;            // mask slots per warp row
 constexpr int kWarpTblBits = 9;            // warp-row hash table: 512 entries
 constexpr int kFilterBits = 12;            // warp-row filter: 4096 bits
 constexpr int kDotTask = 8;                // hybrid form: mask entries per inner-product task
@@ -226,7 +231,7 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
             }
         }
         // warp rows
-        const bool short_row = todo && mi <= kWarpSlots && f <= p.warp_max_flops;
+        const bool short_row = todo && mi <= kWarpSlots<A> && f <= p.warp_max_flops;
         unsigned set = __ballot_sync(FULL, short_row);
         if (set) {
             int pos = 0;
@@ -238,7 +243,7 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
         const bool cta_row = todo && !short_row;
         const int32_t* mcol = p.mc + mb;
         const bool heavy = f >= p.heavy_flops;
-        const bool one = cta_row && mi <= kCtaSlots && mcol[mi - 1] - mcol[0] < kWinCols;
+        const bool one = cta_row && mi <= kCtaSlots<A> && mcol[mi - 1] - mcol[0] < kWinCols;
         for (int h = 0; h < 2; ++h) {
             const bool in = one && heavy == (h == 0);
             set = __ballot_sync(FULL, in);
@@ -251,7 +256,7 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
         if (cta_row && !one) {
             int s0 = 0;
             while (s0 < mi) {
-                int s1 = min(mi, s0 + kCtaSlots);
+                int s1 = min(mi, s0 + kCtaSlots<A>);
                 const int32_t c0 = mcol[s0];
                 if (mcol[s1 - 1] - c0 >= kWinCols) {
                     const int64_t lim = (int64_t)c0 + (kWinCols - 1);
@@ -721,22 +726,22 @@ struct MxmSmem {
     static constexpr bool dense = MD == MD_DENSE;
     // CTA phase
     static constexpr size_t off_acc = 0;
-    static constexpr size_t off_lbs = off_acc + (size_t)kCtaSlots * sizeof(A);
+    static constexpr size_t off_lbs = off_acc + (size_t)kCtaSlots<A> * sizeof(A);
     static constexpr size_t off_lend = off_lbs + (size_t)kLongCap * 4;
     static constexpr size_t off_lchunk = off_lend + (size_t)kLongCap * 4;
     static constexpr size_t off_la = off_lchunk + (size_t)(kLongCap + 8) * 4;
     static constexpr size_t off_key = off_la + (size_t)kLongCap * sizeof(A);  // bits and wbase, or mcol
     static constexpr size_t off_wbase = off_key + (size_t)kWinWords * 4;
     static constexpr size_t cta_bytes =
-        dense ? off_wbase + (size_t)kWinWords * 2 : off_key + (size_t)kCtaSlots * 4;
+        dense ? off_wbase + (size_t)kWinWords * 2 : off_key + (size_t)kCtaSlots<A> * 4;
     // warp phase (per warp): acc, hashed filter and table, or mcol
     static constexpr size_t w_acc = 0;
-    static constexpr size_t w_filt = w_acc + (size_t)kWarpSlots * sizeof(A);
+    static constexpr size_t w_filt = w_acc + (size_t)kWarpSlots<A> * sizeof(A);
     static constexpr size_t w_hkeys = w_filt + (size_t)(1 << kFilterBits) / 8;
     static constexpr size_t w_hslot = w_hkeys + (size_t)(1 << kWarpTblBits) * 4;
     static constexpr size_t w_mcol = w_filt;
     static constexpr size_t warp_one =
-        dense ? w_hslot + (size_t)(1 << kWarpTblBits) : w_mcol + (size_t)kWarpSlots * 4;
+        dense ? w_hslot + (size_t)(1 << kWarpTblBits) : w_mcol + (size_t)kWarpSlots<A> * 4;
     static constexpr size_t warp_bytes = warp_one * kMxmWarps;
     static constexpr size_t region = cta_bytes > warp_bytes ? cta_bytes : warp_bytes;
     // per-warp flattening scratch (both phases)
@@ -933,9 +938,9 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
 }
 
 static int64_t cta_item_cap(int64_t m, int64_t n, int64_t mask_nnz) {
-    // windows per row <= ceil(m_i / kCtaSlots) + ceil(n / kWinCols), and <= m_i
+    // windows per row <= ceil(m_i / kLeastCtaSlots) + ceil(n / kWinCols), and <= m_i
     const int64_t per_row = 1 + (n + kWinCols - 1) / kWinCols;
-    int64_t cap = m * per_row + mask_nnz / kCtaSlots + 1;
+    int64_t cap = m * per_row + mask_nnz / kLeastCtaSlots + 1;
     if (cap > mask_nnz + 1) cap = mask_nnz + 1;
     return cap;
 }
