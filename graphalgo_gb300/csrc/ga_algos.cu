@@ -573,6 +573,12 @@ ga_csr ktruss_impl(ga_ctx ctx, ga_algo algo, ga_csr A, int k, int* iters_out, co
                    algo == GA_HYBRID || algo == GA_TRI,
                GA_ERR_INVALID_ARG, "k-truss: unknown algorithm");
     const int64_t m = A->m;
+    if (algo == GA_TRI && ctx->kt_frontier && m > 0 && csr_unit_values(ctx, A) && csr_is_symmetric(ctx, A)) {
+        // one listing, then only the triangles of the pruned edges
+        TriFront front(ctx, A, batch);
+        front.run(k);
+        return front.result(iters_out);
+    }
     // C = A (a copy; its pattern shrinks in place)
     ga_csr C = copy_csr(ctx, A, GA_INT32);
     try {
@@ -618,17 +624,7 @@ ga_csr ktruss_impl(ga_ctx ctx, ga_algo algo, ga_csr A, int k, int* iters_out, co
             post_launch("kt_expand_rows");
             if (tri) {
                 // rows partitioned [ranked above the row | the rest] for the whole loop
-                tri_kt_setup(ctx, C, row_of.p, mir.p, tc.p, eflag.p, tk, cap, batch);
-                if (ctx->kt_frontier) {
-                    // one listing, then only the triangles of the pruned edges
-                    const TriFrontBufs fb{sup.p, eflag.p, tr.p, tc.p, pos_new.p, trow.p, mir_new.p,
-                                          reinterpret_cast<uint8_t*>(tk.tcrank), scan_scr.p};
-                    const int it = tri_kt_frontier(ctx, C, k, row_of.p, mir.p, tk, cap, fb, batch);
-                    C->unit = 1;
-                    C->sym = 1;
-                    if (iters_out) *iters_out = it;
-                    return C;
-                }
+                tri_kt_setup(ctx, C, row_of.p, mir.p, tc.p, tk, batch);
             } else {
                 k_mirror_index<<<grid_ent, 256, 0, ctx->stream>>>(C->rst, C->col, row_of.p, C->nnz, mir.p);
                 post_launch("kt_mirror_index");
@@ -737,12 +733,7 @@ struct KtSweep {
     bool finished = false;
     ga_csr cur = nullptr;  // stage by stage: the next k's input
     bool fused = false;
-    ga_csr W = nullptr;    // fused: A's copy, rows partitioned for the whole sweep
-    int64_t cap = 0;
-    DBuf<int32_t> sup, eflag, tr, tc, row_of, mir, oid, f0, f1;
-    DBuf<uint8_t> state;
-    DBuf<unsigned char> scan_scr, tri_scr;
-    TriKt tk{};
+    ga_csr W = nullptr;    // fused: the matrix that the frontier state reads
     std::unique_ptr<TriFront> front;
 
     ~KtSweep() {
@@ -769,32 +760,7 @@ struct KtSweep {
             return;
         }
         W = copy_csr(ctx, A, GA_INT32);
-        cap = W->nnz;
-        sup = DBuf<int32_t>(ctx, (size_t)cap);
-        eflag = DBuf<int32_t>(ctx, (size_t)cap + 1);
-        tr = DBuf<int32_t>(ctx, (size_t)m + 1);
-        tc = DBuf<int32_t>(ctx, (size_t)cap);
-        row_of = DBuf<int32_t>(ctx, (size_t)cap);
-        mir = DBuf<int32_t>(ctx, (size_t)cap);
-        oid = DBuf<int32_t>(ctx, (size_t)cap);
-        f0 = DBuf<int32_t>(ctx, (size_t)cap);
-        f1 = DBuf<int32_t>(ctx, (size_t)cap);
-        state = DBuf<uint8_t>(ctx, (size_t)cap);
-        scan_scr = DBuf<unsigned char>(ctx, scan_scratch_bytes(cap + 1));
-        tri_scr = DBuf<unsigned char>(ctx, tri_kt_bytes(m, cap));
-        setup_front();
-    }
-
-    // The frontier state on W (its rows partitioned by rank, its mirror
-    // index; the first run lists W's triangles). The buffers keep the size
-    // of the sweep's first matrix; a rebuilt W is smaller.
-    void setup_front() {
-        cap = W->nnz;
-        tri_kt_carve(tri_scr.p, W->m, cap, &tk);
-        expand_rows(ctx, W, row_of.p);
-        tri_kt_setup(ctx, W, row_of.p, mir.p, tc.p, eflag.p, tk, cap, nullptr);
-        const TriFrontBufs fb{sup.p, eflag.p, tr.p, tc.p, oid.p, f0.p, f1.p, state.p, scan_scr.p};
-        front.reset(new TriFront(ctx, W, row_of.p, mir.p, tk, cap, fb, nullptr));
+        front.reset(new TriFront(ctx, W, nullptr));
     }
 
     // Entries never move inside the state, so once a k-truss keeps at most
@@ -809,7 +775,7 @@ struct KtSweep {
         nw->sym = 1;
         csr_destroy(ctx, W);
         W = nw;
-        setup_front();
+        front.reset(new TriFront(ctx, W, nullptr));
     }
 
     // The next C_k (owned by the caller), or nullptr after the empty one.
@@ -821,20 +787,9 @@ struct KtSweep {
         int it = 0;
         if (fused) {
             front->run(k);
-            // the only wait: what follows runs while the caller takes the
+            // the only wait: what follows it runs while the caller takes the
             // result and asks for the next k
-            const int64_t kept = front->result(&it);
-            const int64_t m = W->m;
-            out = csr_alloc(ctx, m, m, kept, GA_INT32);
-            try {
-                front->compact(out->rst, out->col);
-                fill_ones(ctx, out->val, kept, GA_INT32);
-            } catch (...) {
-                csr_destroy(ctx, out);
-                throw;
-            }
-            out->unit = 1;
-            out->sym = 1;
+            out = front->result(&it);
             maybe_rebuild(out);
         } else {
             ga_csr res = ktruss_impl(ctx, algo, cur, k, &it, nullptr);

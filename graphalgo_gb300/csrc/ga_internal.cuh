@@ -253,16 +253,19 @@ struct TriKt {
     int32_t* tstart;    // m + 2: tasks per row, scanned into task starts
     int32_t* task_row;  // cap / 16 + m + 1: row of each task
     int32_t* dpos;      // m + 1: position of each row's diagonal entry, -1 if none
+    int32_t* rank;      // m + 1: rank of each vertex
+    uint32_t* bits;     // cap / 32 + 1: flags, one bit per entry
+    int32_t* pre;       // cap / 32 + 2: flags before each word
     void* scan_scr;
 };
 size_t tri_kt_bytes(int64_t m, int64_t cap);
 void tri_kt_carve(void* scratch, int64_t m, int64_t cap, TriKt* t);
 // Before the loop: ranks (with `batch`, among each graph's vertices), the
-// partition of every row (tmp_col: cap entries, tmp_flag: cap + 1), the
-// mirror index in that layout, diagonal positions, tasks per row. row_of must
-// hold every entry's row.
-void tri_kt_setup(ga_ctx ctx, ga_csr C, const int32_t* row_of, int32_t* mir, int32_t* tmp_col, int32_t* tmp_flag,
-                  const TriKt& t, int64_t cap, const KtBatch* batch);
+// partition of every row (tmp_col: cap entries), the mirror index in that
+// layout, diagonal positions, tasks per row. row_of must hold every entry's
+// row.
+void tri_kt_setup(ga_ctx ctx, ga_csr C, const int32_t* row_of, int32_t* mir, int32_t* tmp_col, const TriKt& t,
+                  const KtBatch* batch);
 // One support evaluation: counts at the oriented entries of sup (cap).
 void tri_kt_support(ga_ctx ctx, ga_csr C, int32_t* sup, const TriKt& t, int64_t cap);
 // Keep flags from the support (k, or the batch's per-graph k / finished
@@ -282,45 +285,25 @@ void tri_kt_copyback(ga_ctx ctx, ga_csr C, const KtState* st, const int32_t* tr,
 // After the loop: every row back in column order.
 void tri_kt_finish(ga_ctx ctx, ga_csr C, const int32_t* row_of, const TriKt& t, int32_t* tmp_col);
 
-// Frontier form of the triangle-listing k-truss of one matrix (symmetric,
-// values 1), after tri_kt_setup: the triangles are listed once, then every
-// iteration prunes the edges whose support is below k - 2 and lowers the
-// supports of the edges that shared a triangle with them. Buffers: sup, oid,
-// f0, f1, tc (cap each), flag (cap + 1), state (cap bytes), tr (m + 1), scan
-// scratch. Leaves C pruned with its rows in column order; returns the
-// reference's iteration count.
-struct TriFrontBufs {
-    int32_t* sup;
-    int32_t* flag;
-    int32_t* tr;
-    int32_t* tc;
-    int32_t* oid;
-    int32_t* f0;
-    int32_t* f1;
-    uint8_t* state;
-    void* scan_scr;
-};
-// With `batch`: every graph of the union with its own k, iteration count
-// (batch->iters_g) and iteration bound; the loop runs while a graph iterates.
-int tri_kt_frontier(ga_ctx ctx, ga_csr C, int k, const int32_t* row_of, const int32_t* mir, const TriKt& t,
-                    int64_t cap, const TriFrontBufs& b, const KtBatch* batch);
-// The same state kept between calls: run(k) iterates for one k (the first
-// call lists the triangles; a later call, one matrix only, takes a larger k
-// and continues from the supports the previous k left, so a sweep k = kmin,
-// kmin + 1, ... lists the triangles once); result() gives the number of kept
-// entries and the iteration count of the last run (one host synchronisation);
-// compact() then writes the kept entries, rows in column order (col: as many
-// entries as kept).
+// Frontier form of the triangle-listing k-truss of a symmetric matrix with
+// values one: the triangles are listed once, then every iteration prunes the
+// edges whose support is below k - 2 and lowers the supports of the edges
+// that shared a triangle with them. run(k) iterates for one k: the first call
+// lists the triangles; a later call, one matrix only, takes a larger k and
+// continues from the supports the previous k left, so a sweep k = kmin,
+// kmin + 1, ... lists the triangles once. result() gives the entries the last
+// run kept as a matrix of their own, and the iteration count (one host wait).
+// A is read until the object is gone. With `batch`: every graph of the union
+// with its own k, iteration count (batch->iters_g) and iteration bound; the
+// loop runs while a graph iterates.
 class TriFront {
 public:
-    TriFront(ga_ctx ctx, ga_csr C, const int32_t* row_of, const int32_t* mir, const TriKt& t, int64_t cap,
-             const TriFrontBufs& b, const KtBatch* batch);
+    TriFront(ga_ctx ctx, ga_csr A, const KtBatch* batch);
     ~TriFront();
     TriFront(const TriFront&) = delete;
     TriFront& operator=(const TriFront&) = delete;
     void run(int k);
-    int64_t result(int* iters);
-    void compact(int32_t* rst, int32_t* col);
+    ga_csr result(int* iters);
 
 private:
     struct Impl;

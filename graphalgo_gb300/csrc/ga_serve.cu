@@ -38,8 +38,9 @@ static int64_t bound_tc(int64_t m, int64_t nnz, int64_t sval) {
 }
 
 static int64_t bound_ktruss(int64_t m, int64_t nnz) {
-    // copy of C, support, compaction, SpGEMM scratch, mirror index arrays
-    return 56 * (m + 2) + 60 * (nnz + 1) + (1 << 20);
+    // products: copy of C, support, compaction, SpGEMM scratch, mirror index
+    // arrays; triangle listing: the frontier state and the result
+    return std::max(56 * (m + 2) + 60 * (nnz + 1), 96 * (m + 2) + 52 * (nnz + 1)) + (1 << 20);
 }
 
 static int64_t bound_bc(int64_t m, int64_t nnz, int64_t ns) {

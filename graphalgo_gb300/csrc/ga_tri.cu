@@ -40,7 +40,9 @@
 #include "ga_device.cuh"
 #include "ga_loop.cuh"
 
+#include <algorithm>
 #include <cstddef>
+#include <cstring>
 #include <map>
 #include <mutex>
 
@@ -556,45 +558,70 @@ void tri_masked_into(ga_ctx ctx, ga_csr A, int32_t* sup) {
 }
 
 // =============================================== resident orientation (k-truss)
+// Ranks of flagged entries. A flag takes one bit of a 32-entry word, and the
+// words' counts are scanned, not the entries: a 32nd of the scan's work, and
+// a rank is read from two small arrays (R-MAT 18, 7.6M entries: flags, scan
+// and placing 124 us with an int per entry, 92 with words).
+struct WordRanks {
+    uint32_t* bits;  // word w: entries 32 w ..
+    int32_t* pre;    // flags before word w; the last word's next holds their number
+};
+// Flagged entries before entry q (q: up to the number of entries).
+__device__ __forceinline__ int32_t word_rank(const WordRanks& r, int64_t q) {
+    return r.pre[q >> 5] + __popc(r.bits[q >> 5] & ((1u << (q & 31)) - 1u));
+}
+__device__ __forceinline__ bool word_flag(const WordRanks& r, int64_t q) { return r.bits[q >> 5] >> (q & 31) & 1u; }
+// Words that word_rank reads for q <= entries.
+static int64_t rank_words(int64_t entries) { return entries / 32 + 1; }
+
 // Entry q of the unpartitioned C (column order) goes to the oriented part of
-// its row when its column is ranked above the row.
-__global__ void k_trikt_part_flags(const int32_t* __restrict__ cr, const int32_t* __restrict__ cc,
-                                   const int32_t* __restrict__ row_of, const int32_t* __restrict__ rank, int64_t m,
-                                   int64_t cap, int32_t* __restrict__ flag) {
-    const int64_t cur = cr[m];
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < cap; q += (int64_t)gridDim.x * blockDim.x) {
-        int32_t f = 0;
-        if (q < cur) {
+// its row when its column is ranked above the row. One warp per word.
+__global__ void k_trikt_part_flags(const int32_t* __restrict__ cc, const int32_t* __restrict__ row_of,
+                                   const int32_t* __restrict__ rank, int64_t nnz, WordRanks r) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5), words = nnz / 32 + 1;
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += warps) {
+        const int64_t q = w * 32 + lane;
+        bool f = false;
+        if (q < nnz) {
             const int32_t i = row_of[q], j = cc[q];
             f = i != j && rank[j] > rank[i];
         }
-        flag[q] = f;
+        const unsigned b = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) {
+            r.bits[w] = b;
+            r.pre[w] = __popc(b);
+        }
     }
 }
 
-// After the flags' scan: stable partition of every row (oriented part, then
-// the rest), the rank of every placed column, and per row its oriented count
-// and tasks.
+// Place of entry q of row [rb, re) in the stable partition of the row.
+__device__ __forceinline__ int32_t part_place(const WordRanks& r, int64_t q, int32_t rb, int32_t oc, bool* oriented) {
+    const int32_t before = word_rank(r, q) - word_rank(r, rb);  // oriented entries before q in its row
+    *oriented = word_flag(r, q);
+    return *oriented ? rb + before : rb + oc + (int32_t)(q - rb) - before;
+}
+
+// After the scan: the partition of every row (oriented part, then the rest),
+// the rank of every placed column, and per row its oriented count and tasks
+// (its diagonal position comes later).
 __global__ void k_trikt_part_place(const int32_t* __restrict__ cr, const int32_t* __restrict__ cc,
-                                   const int32_t* __restrict__ row_of, const int32_t* __restrict__ rank,
-                                   const int32_t* __restrict__ pos, int64_t m, int32_t* __restrict__ out_col,
+                                   const int32_t* __restrict__ row_of, const int32_t* __restrict__ rank, WordRanks r,
+                                   int64_t m, int64_t nnz, int32_t* __restrict__ out_col,
                                    int32_t* __restrict__ crank, int32_t* __restrict__ ocount,
-                                   int32_t* __restrict__ ntask) {
-    const int64_t cur = cr[m];
+                                   int32_t* __restrict__ ntask, int32_t* __restrict__ dpos) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < cur || q < m; q += stride) {
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nnz || q < m; q += stride) {
         if (q < m) {
-            const int32_t oc = pos[cr[q + 1]] - pos[cr[q]];
+            dpos[q] = -1;
+            const int32_t oc = word_rank(r, cr[q + 1]) - word_rank(r, cr[q]);
             ocount[q] = oc;
             ntask[q] = (oc + kTriTask - 1) / kTriTask;
         }
-        if (q < cur) {
-            const int32_t i = row_of[q], rb = cr[i];
-            const int32_t before = pos[q] - pos[rb];            // oriented entries before q in its row
-            const int32_t oc = pos[cr[i + 1]] - pos[rb];
-            const bool o = pos[q + 1] != pos[q];
-            const int32_t np = o ? rb + before : rb + oc + (int32_t)(q - rb) - before;
-            const int32_t j = cc[q];
+        if (q < nnz) {
+            const int32_t i = row_of[q], rb = cr[i], j = cc[q];
+            bool o;
+            const int32_t np = part_place(r, q, rb, word_rank(r, cr[i + 1]) - word_rank(r, rb), &o);
             out_col[np] = j;
             crank[np] = rank[j];
         }
@@ -766,6 +793,9 @@ size_t trikt_carve(void* scratch, int64_t m, int64_t cap, TriKt* t) {
     s.tstart = take(r);
     s.task_row = take(task_cap(m, cap));
     s.dpos = take(r);
+    s.rank = take(r);
+    s.bits = reinterpret_cast<uint32_t*>(take((size_t)rank_words(cap)));
+    s.pre = take((size_t)rank_words(cap) + 1);
     s.scan_scr = base ? base + off : nullptr;
     off += align256(scan_scratch_bytes((cap > m ? cap : m) + 2));
     if (t) *t = s;
@@ -777,11 +807,10 @@ size_t tri_kt_bytes(int64_t m, int64_t cap) { return trikt_carve(nullptr, m, cap
 
 void tri_kt_carve(void* scratch, int64_t m, int64_t cap, TriKt* t) { trikt_carve(scratch, m, cap, t); }
 
-void tri_kt_setup(ga_ctx ctx, ga_csr C, const int32_t* row_of, int32_t* mir, int32_t* tmp_col, int32_t* tmp_flag,
-                  const TriKt& t, int64_t cap, const KtBatch* batch) {
-    const int64_t m = C->m, nnz = C->nnz;
-    // ranks by degree (or index) into task_row, which the loop fills later
-    int32_t* rank = t.task_row;
+// Ranks, and the stable partition of every row of (rst, col) into out_col.
+static void trikt_partition(ga_ctx ctx, const int32_t* rst, const int32_t* col, int64_t m, int64_t nnz,
+                            const int32_t* row_of, const TriKt& t, const KtBatch* batch, int32_t* out_col) {
+    int32_t* rank = t.rank;  // by degree (or index)
     const int grid_v = grid_for(m, 256, ctx->num_sms * 8);
     if (ctx->tune.tri_order == 1) {
         k_tri_iota<<<grid_v, 256, 0, ctx->stream>>>(m, rank);
@@ -793,29 +822,36 @@ void tri_kt_setup(ga_ctx ctx, ga_csr C, const int32_t* row_of, int32_t* mir, int
         // graphs of up to 4,096 vertices (46M entries): the listing takes
         // 3.40 ms, 6.61 ms with the union's ranks.
         GA_CUDA(cudaMemsetAsync(t.tstart, 0, sizeof(int32_t) * (size_t)(m + 2), ctx->stream));
-        k_tri_graph_deg_count<<<grid_v, 256, 0, ctx->stream>>>(C->rst, m, batch->gid, batch->voff, t.tstart);
+        k_tri_graph_deg_count<<<grid_v, 256, 0, ctx->stream>>>(rst, m, batch->gid, batch->voff, t.tstart);
         post_launch("tri_deg_count");
         scan_exclusive_i32_scratch(ctx, t.tstart, t.tstart, m, t.scan_scr);
-        k_tri_graph_rank<<<grid_v, 256, 0, ctx->stream>>>(C->rst, m, batch->gid, batch->voff, t.tstart, rank);
+        k_tri_graph_rank<<<grid_v, 256, 0, ctx->stream>>>(rst, m, batch->gid, batch->voff, t.tstart, rank);
         post_launch("tri_rank");
     } else {
         GA_CUDA(cudaMemsetAsync(t.tstart, 0, sizeof(int32_t) * (size_t)(m + 2), ctx->stream));
-        k_tri_deg_count<<<grid_v, 256, 0, ctx->stream>>>(C->rst, m, t.tstart);
+        k_tri_deg_count<<<grid_v, 256, 0, ctx->stream>>>(rst, m, t.tstart);
         post_launch("tri_deg_count");
         scan_exclusive_i32_scratch(ctx, t.tstart, t.tstart, m + 1, t.scan_scr);
-        k_tri_rank<<<grid_v, 256, 0, ctx->stream>>>(C->rst, m, t.tstart, rank);
+        k_tri_rank<<<grid_v, 256, 0, ctx->stream>>>(rst, m, t.tstart, rank);
         post_launch("tri_rank");
     }
-    const int grid_ent = grid_for(cap, 256, ctx->num_sms * 16);
-    k_trikt_part_flags<<<grid_ent, 256, 0, ctx->stream>>>(C->rst, C->col, row_of, rank, m, cap, tmp_flag);
+    const WordRanks r{t.bits, t.pre};
+    const int64_t words = rank_words(nnz);
+    k_trikt_part_flags<<<grid_for(words * 32, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(col, row_of, rank, nnz,
+                                                                                            r);
     post_launch("trikt_part_flags");
-    scan_exclusive_i32_scratch(ctx, tmp_flag, tmp_flag, cap, t.scan_scr);
-    k_trikt_part_place<<<grid_for(m + cap, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
-        C->rst, C->col, row_of, rank, tmp_flag, m, tmp_col, t.crank, t.ocount, t.tstart);
+    scan_exclusive_i32_scratch(ctx, t.pre, t.pre, words, t.scan_scr);
+    k_trikt_part_place<<<grid_for(nnz > m ? nnz : m, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+        rst, col, row_of, rank, r, m, nnz, out_col, t.crank, t.ocount, t.tstart, t.dpos);
     post_launch("trikt_part_place");
+}
+
+void tri_kt_setup(ga_ctx ctx, ga_csr C, const int32_t* row_of, int32_t* mir, int32_t* tmp_col, const TriKt& t,
+                  const KtBatch* batch) {
+    const int64_t m = C->m, nnz = C->nnz;
+    trikt_partition(ctx, C->rst, C->col, m, nnz, row_of, t, batch, tmp_col);
     if (nnz) GA_CUDA(cudaMemcpyAsync(C->col, tmp_col, sizeof(int32_t) * (size_t)nnz, cudaMemcpyDeviceToDevice,
                                      ctx->stream));
-    GA_CUDA(cudaMemsetAsync(t.dpos, 0xff, sizeof(int32_t) * (size_t)m, ctx->stream));
     if (nnz) {
         k_trikt_part_mirror<<<grid_for(nnz, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
             C->rst, C->col, row_of, t.crank, t.ocount, nnz, mir, t.dpos);
@@ -909,7 +945,6 @@ enum : uint8_t { kAlive = 0, kDying = 1, kGone = 2 };
 struct TriFrontState {
     int32_t cnt[2];              // frontier sizes; the current one is cnt[t & 1]
     int32_t t;                   // iteration
-    int32_t iters;               // reported iteration count
     int32_t done;
     int32_t ntouch;              // vertices whose terms of P change this iteration
     int32_t nflip;               // rows that lost their last upper entry
@@ -917,29 +952,39 @@ struct TriFrontState {
     uint32_t blocks_done;        // delta kernel: blocks finished
     uint32_t blocks_done_g;      // graph kernel (batches): blocks finished
     // one-launch loop (k_trif_loop); [4]: by iteration
-    int32_t failed;              // a wait at its barrier ran out
     int32_t nfront[4];           // frontier
     int32_t nt[4], nf[4];        // touched vertices, flipped rows
     unsigned long long nsegs[4]; // segments of the frontier's long rows
     unsigned long long dd[4];    // change of P
     unsigned long long dmask[4], dent[4];  // upper entries and entries that left
     unsigned long long bar;      // arrivals at the barrier
-    int32_t live;                // batches: graphs still iterating
+    // iters .. ent are read back together
+    int32_t iters;               // reported iteration count
+    int32_t failed;              // a wait at the one-launch loop's barrier ran out
+    int32_t live;                // batches: graphs still iterating (from here on kept from one k to the next)
     int32_t diag;                // the matrix has diagonal entries
+    unsigned long long ent;      // entries of C_t
     unsigned long long prod;     // P_t (batches: summed over the live graphs)
     unsigned long long mask;     // entries (i, j) of C_t with j >= i
-    unsigned long long ent;      // entries of C_t
 };
+struct TriFrontResult {
+    int32_t iters, failed, live, diag;
+    unsigned long long ent;
+};
+static_assert(offsetof(TriFrontState, ent) - offsetof(TriFrontState, iters) == offsetof(TriFrontResult, ent),
+              "the part of the state that is read back");
 
 struct TriFrontArgs {
     const int32_t* cr;      // row starts (fixed during the loop)
     const int32_t* cc;      // columns, every row as [oriented part | rest]
+    const int32_t* ac;      // columns, rows in column order
     const int32_t* row_of;
-    const int32_t* mir;
     const int32_t* crank;   // rank of each entry's column
+    const int32_t* rank;    // of each vertex
     const int32_t* ocount;
     const int32_t* dpos;    // position of each row's diagonal entry, -1 if none
-    int32_t* oid;           // entry -> position of its edge's record
+    int32_t* oid;           // entry (of cc) -> position of its edge's record
+    int32_t* orec;          // the same for the entries in column order (of ac)
     int32_t* sup;           // supports at the records
     uint8_t* state;         // states at the records
     int32_t* deg;           // entries of each row still in C
@@ -1015,47 +1060,118 @@ __device__ __forceinline__ void touch(const TriFrontArgs& a, int32_t x) {
 
 __global__ void k_trif_init_rows(TriFrontArgs a) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.m; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t b = a.cr[i], e = a.cr[i + 1], oc = a.ocount[i];
-        const int32_t up = (oc - lower_bound_i32(a.cc + b, oc, (int32_t)i)) +
-                           (e - b - oc - lower_bound_i32(a.cc + b + oc, e - b - oc, (int32_t)i));
-        a.deg[i] = e - b;
+        const int32_t b = a.cr[i], n = a.cr[i + 1] - b;
+        const int32_t up = n - lower_bound_i32(a.ac + b, n, (int32_t)i);
+        a.deg[i] = n;
         a.upc[i] = up;
         a.h[i] = up > 0;
+        a.H[i] = 0;
         a.rd[i] = 0;
         a.rh[i] = 0;
         a.mark[i] = 0;
         if (a.dcur) {
             a.rd1[i] = a.rd2[i] = 0;
             a.rh1[i] = a.rh2[i] = 0;
-            a.dcur[i] = e - b;
+            a.dcur[i] = n;
         }
     }
 }
 
-// Records of the edges (the oriented entry; a diagonal entry is its own),
-// states, the diagonal terms of the listed supports, and the first frontier.
-__global__ void k_trif_seed(TriFrontArgs a) {
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < a.nnz; q += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t i = a.row_of[q], j = a.cc[q];
-        const bool rec = i == j || (int64_t)q - a.cr[i] < a.ocount[i];
-        a.oid[q] = rec ? (int32_t)q : a.mir[q];
-        a.state[q] = kAlive;
-        // one matrix: a record of the first frontier is marked at once
-        // (batches mark theirs in k_trif_mark)
-        if (i == j) {
-            a.st->diag = 1;
-            if (a.deg[i] < kt_thr(a, i)) {
-                front_add(a, a.f0, &a.st->cnt[0], (int32_t)q, i, 0);
-                if (!a.gid) a.state[q] = kDying;
+// The states, every entry's record (the oriented entry of its edge; a diagonal entry is
+// its own), for the entries as the loop stores them and in column order, the
+// diagonal positions, and H. An oriented entry is its own record, the other
+// entry of the edge searches the row ranked below for it, in the short
+// oriented part. (A mirror found for both, each by its own search, then a
+// pass to make records of them, and H by a warp per row, where a hub's row
+// keeps one warp busy: 389 us together at R-MAT 18 and 1,190 us for 512
+// nearest-neighbour graphs of 46M entries.)
+__global__ void k_trif_records(TriFrontArgs a, WordRanks r, int32_t* __restrict__ dpos) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t threads = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~(int64_t)31; p0 < a.nnz; p0 += threads) {
+        const int64_t p = p0 + lane;
+        int32_t i = -1;
+        bool hj = false;
+        if (p < a.nnz) {
+            i = a.row_of[p];
+            const int32_t j = a.ac[p];
+            bool o;
+            const int32_t np = part_place(r, p, a.cr[i], a.ocount[i], &o);
+            int32_t rec = np;
+            if (i == j) {
+                dpos[i] = np;
+                a.st->diag = 1;
+            } else if (!o) {
+                const int32_t jb = a.cr[j];
+                rec = jb + lower_bound_i32(a.cc + jb, a.ocount[j], i);
             }
-        } else if (rec) {
-            const int32_t s = a.sup[q] + (a.dpos[i] >= 0) + (a.dpos[j] >= 0);
-            a.sup[q] = s;
-            if (s < kt_thr(a, i)) {
-                front_add(a, a.f0, &a.st->cnt[0], (int32_t)q, i, 0);
-                if (!a.gid) a.state[q] = kDying;
-            }
+            a.orec[p] = rec;
+            a.oid[np] = rec;
+            a.state[p] = kAlive;
+            hj = a.h[j] != 0;
         }
+        // entries of each row among the warp's
+        const int32_t before = __shfl_up_sync(FULL, i, 1);
+        const unsigned heads = __ballot_sync(FULL, lane == 0 || before != i), set = __ballot_sync(FULL, hj);
+        if (i >= 0 && (heads >> lane & 1u)) {
+            const unsigned later = heads & ~((2u << lane) - 1u);
+            const unsigned upto = later ? (1u << (__ffs(later) - 1)) - 1u : FULL;
+            const int c = __popc(set & upto & ~((1u << lane) - 1u));
+            if (c) atomicAdd(a.H + i, c);
+        }
+    }
+}
+
+// A warp's records of the first frontier, kSeedWords words of 32 entries from
+// q0 on (is: bit w for the lane's entry of word w): they take their places
+// together, since all places come from one counter (R-MAT 18's 4-truss, half
+// of the records in the first frontier: an atomic per word 52 us, per four
+// words 30). One matrix: the records are marked at once; batches mark
+// theirs in k_trif_mark and count them for their graphs.
+constexpr int kSeedWords = 4;
+__device__ __forceinline__ void front_first(const TriFrontArgs& a, unsigned is, int64_t q0) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int mine = __popc(is), incl = warp_incl_scan(mine), total = __shfl_sync(FULL, incl, 31);
+    if (!total) return;
+    int32_t at = 0;
+    if (lane == 0) at = atomicAdd(&a.st->cnt[0], total);
+    at = __shfl_sync(FULL, at, 0) + incl - mine;
+    for (; is; is &= is - 1) {
+        const int32_t q = (int32_t)q0 + (__ffs(is) - 1) * 32 + lane;
+        a.f0[at++] = q;
+        if (a.gid) atomicAdd(a.cntg + a.gid[a.row_of[q]], 1);
+        else a.state[q] = kDying;
+    }
+}
+
+// The diagonal terms of the listed supports, and the first frontier. (The
+// states are alive.)
+__global__ void k_trif_seed(TriFrontArgs a) {
+    const bool diag = a.st->diag != 0;
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5) * kSeedWords * 32;
+    for (int64_t q0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kSeedWords * 32; q0 < a.nnz;
+         q0 += step) {
+        unsigned is = 0;
+#pragma unroll
+        for (int w = 0; w < kSeedWords; ++w) {
+            const int64_t q = q0 + w * 32 + lane;
+            if (q >= a.nnz || a.oid[q] != (int32_t)q) continue;
+            int32_t s = a.sup[q];
+            if (diag) {
+                const int32_t i = a.row_of[q], j = a.cc[q];
+                if (i == j) {
+                    s = a.deg[i];
+                } else {
+                    s += (a.dpos[i] >= 0) + (a.dpos[j] >= 0);
+                    a.sup[q] = s;
+                }
+            }
+            is |= (unsigned)(s < (a.kg ? kt_thr(a, a.row_of[q]) : a.k - 2)) << w;
+        }
+        front_first(a, is, q0);
     }
 }
 
@@ -1063,35 +1179,49 @@ __global__ void k_trif_seed(TriFrontArgs a) {
 // exact supports in C, so the first frontier of the new k is the live
 // records below the new k - 2 (a diagonal record: its row's length).
 __global__ void k_trif_reseed(TriFrontArgs a) {
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < a.nnz; q += (int64_t)gridDim.x * blockDim.x) {
-        if (a.oid[q] != (int32_t)q || a.state[q] != kAlive) continue;
-        const int32_t i = a.row_of[q];
-        const int32_t s = a.cc[q] == i ? a.deg[i] : a.sup[q];
-        if (s < kt_thr(a, i)) {
-            front_push(a.f0, &a.st->cnt[0], (int32_t)q);
-            a.state[q] = kDying;
+    const bool diag = a.st->diag != 0;
+    const int lane = threadIdx.x & 31;
+    const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5) * kSeedWords * 32;
+    for (int64_t q0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kSeedWords * 32; q0 < a.nnz;
+         q0 += step) {
+        unsigned is = 0;
+#pragma unroll
+        for (int w = 0; w < kSeedWords; ++w) {
+            const int64_t q = q0 + w * 32 + lane;
+            if (q >= a.nnz || a.oid[q] != (int32_t)q || a.state[q] != kAlive) continue;
+            const int32_t s = diag && a.cc[q] == a.row_of[q] ? a.deg[a.row_of[q]] : a.sup[q];
+            is |= (unsigned)(s < a.k - 2) << w;
         }
+        front_first(a, is, q0);
     }
 }
 
-// H, and P_0, the upper entries and the entries of C_0; one warp per row.
+// P_0, the upper entries and the entries of C_0; one thread per row.
 __global__ void k_trif_init_counts(TriFrontArgs a) {
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int64_t threads = (int64_t)gridDim.x * blockDim.x;
     unsigned long long prod = 0, mask = 0, ent = 0;
-    for (int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < a.m; j += warps) {
-        int hs = 0;
-        for (int32_t p = a.cr[j] + lane; p < a.cr[j + 1]; p += 32) hs += a.h[a.cc[p]];
-        hs = warp_sum<int>(hs);
-        if (lane == 0) {
-            a.H[j] = hs;
-            const unsigned long long pj = (unsigned long long)a.deg[j] * (unsigned long long)hs;
-            prod += pj;
-            if (a.gid && pj) atomicAdd(reinterpret_cast<unsigned long long*>(a.pg + a.gid[j]), pj);
+    for (int64_t j0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~(int64_t)31; j0 < a.m; j0 += threads) {
+        const int64_t j = j0 + lane;
+        unsigned long long pj = 0;
+        if (j < a.m) {
+            pj = (unsigned long long)a.deg[j] * (unsigned long long)a.H[j];
             mask += (unsigned long long)a.upc[j];
             ent += (unsigned long long)a.deg[j];
         }
+        prod += pj;
+        if (a.gid) {
+            // most warps lie inside one graph
+            const int32_t g = a.gid[min(j, a.m - 1)], g0 = __shfl_sync(FULL, g, 0);
+            const bool one = __all_sync(FULL, g == g0);
+            if (one) pj = warp_sum<unsigned long long>(pj);
+            if (pj && (!one || lane == 0)) atomicAdd(reinterpret_cast<unsigned long long*>(a.pg + g), pj);
+        }
     }
+    prod = warp_sum<unsigned long long>(prod);
+    mask = warp_sum<unsigned long long>(mask);
+    ent = warp_sum<unsigned long long>(ent);
     if (lane == 0) {
         if (prod) atomicAdd(&a.st->prod, prod);
         if (mask) atomicAdd(&a.st->mask, mask);
@@ -1188,8 +1318,7 @@ __device__ __forceinline__ TrifEdge trif_edge(const TriFrontArgs& a, int32_t q, 
     e.yb = xu ? vb : ub;
     e.ye = xu ? ve : ue;
     e.yo = e.yb + a.ocount[y];
-    // rank of y: the entry (u, v) holds rank(v), its mirror rank(u)
-    e.ry = xu ? a.crank[q] : a.crank[a.mir[q]];
+    e.ry = a.rank[y];
     return e;
 }
 
@@ -2031,27 +2160,33 @@ __global__ void __launch_bounds__(256) k_trif_graphs(const TriFrontArgs* __restr
     loop_continue(ctl, st->done == 0);
 }
 
-__global__ void k_trif_keep(TriFrontArgs a, int64_t cap, int32_t* __restrict__ flag) {
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < cap; q += (int64_t)gridDim.x * blockDim.x)
-        flag[q] = q < a.nnz && a.state[a.oid[q]] != kGone;
+// Keep flags of the entries in column order. One warp per word.
+__global__ void k_trif_keep(TriFrontArgs a, WordRanks r) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5), words = a.nnz / 32 + 1;
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += warps) {
+        const int64_t p = w * 32 + lane;
+        const unsigned b = __ballot_sync(0xffffffffu, p < a.nnz && a.state[a.orec[p]] != kGone);
+        if (lane == 0) {
+            r.bits[w] = b;
+            r.pre[w] = __popc(b);
+        }
+    }
 }
 
-// After the keep flags' scan (pos): kept entries written in column order (an
-// entry's place: kept entries before it in its part, plus kept entries of
-// the other part with smaller columns), new row starts.
-__global__ void k_trif_out(TriFrontArgs a, const int32_t* __restrict__ pos, int32_t* __restrict__ tc,
-                           int32_t* __restrict__ tr) {
+// After the scan: the kept entries' columns, ones, and the new row starts.
+// (Kept entries in the loop's order, each placed by a search of its row's
+// other part, with an int per entry as flag and position: flags, scan and
+// this 145 us at R-MAT 18.)
+__global__ void k_trif_out(TriFrontArgs a, WordRanks r, int32_t* __restrict__ col, int32_t* __restrict__ val,
+                           int32_t* __restrict__ rst) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < a.nnz || q <= a.m; q += stride) {
-        if (q <= a.m) tr[q] = pos[a.cr[q]];
-        if (q < a.nnz && pos[q + 1] != pos[q]) {
-            const int32_t i = a.row_of[q], rb = a.cr[i], re = a.cr[i + 1], ro = rb + a.ocount[i];
-            const bool o = q < ro;
-            const int32_t pb = o ? rb : ro;
-            const int32_t ob = o ? ro : rb, oe = o ? re : ro;
-            const int32_t j = a.cc[q];
-            const int32_t t = ob + lower_bound_i32(a.cc + ob, oe - ob, j);
-            tc[pos[rb] + (pos[q] - pos[pb]) + (pos[t] - pos[ob])] = j;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < a.nnz || p <= a.m; p += stride) {
+        if (p <= a.m) rst[p] = word_rank(r, a.cr[p]);
+        if (p < a.nnz && word_flag(r, p)) {
+            const int32_t d = word_rank(r, p);
+            col[d] = a.ac[p];
+            val[d] = 1;
         }
     }
 }
@@ -2079,121 +2214,163 @@ static bool trif_loop_fits(ga_ctx ctx) {
 
 struct TriFront::Impl {
     ga_ctx ctx;
-    ga_csr C;
-    TriKt t;
-    int64_t cap;
-    TriFrontBufs b;
+    int64_t m, nnz, cap;
     const KtBatch* batch;
     int64_t ng;
-    DBuf<int32_t> deg, upc, H, rd, rh, mark, touched, flip;
     bool one_launch;                   // the loop in one cooperative launch
-    DBuf<int32_t> rd1, rd2, rh1, rh2, flip2, dcur;
-    DBuf<uint8_t> h;
-    DBuf<TriFrontState> st;
-    DBuf<int32_t> cntg;
-    DBuf<long long> pg;
-    DBuf<int2> seg;
-    DBuf<int32_t> efound;
+    DBuf<unsigned char> mem;           // everything below (as thirty allocations 35 us of host time)
+    int32_t *row_of, *pcol, *oid, *orec, *sup, *f0, *f1, *efound;                            // per entry
+    int32_t *deg, *upc, *H, *rd, *rh, *mark, *touched, *flip;                                // per row
+    int32_t *rd1, *rd2, *rh1, *rh2, *touched1, *touched2, *flip1, *flip2, *dcur;             // (one-launch loop)
+    uint8_t *h, *state;
+    TriFrontState* st;
+    int32_t* cntg;
+    long long* pg;
+    int2* seg;
+    int64_t nseg;
+    void* kt_scr;
+    TriKt t;
+    WordRanks words;
+    ga_csr_s W;                        // the matrix with partitioned rows
     TriFrontArgs a;
+    cudaEvent_t ready = nullptr;       // the result has been copied
     bool first = true;
 
-    Impl(ga_ctx ctx_, ga_csr C_, const int32_t* row_of, const int32_t* mir, const TriKt& t_, int64_t cap_,
-         const TriFrontBufs& b_, const KtBatch* batch_)
-        : ctx(ctx_), C(C_), t(t_), cap(cap_), b(b_), batch(batch_), ng(batch_ ? batch_->ngraphs : 0),
-          deg(ctx_, (size_t)C_->m + 1), upc(ctx_, (size_t)C_->m + 1), H(ctx_, (size_t)C_->m + 1),
-          rd(ctx_, (size_t)C_->m + 1), rh(ctx_, (size_t)C_->m + 1), mark(ctx_, (size_t)C_->m + 1),
-          touched(ctx_, (size_t)C_->m + 1), flip(ctx_, (size_t)C_->m + 1),
-          one_launch(!batch_ && ctx_->device_loops && trif_loop_fits(ctx_)),
-          rd1(ctx_, one_launch ? (size_t)C_->m + 1 : 1), rd2(ctx_, one_launch ? (size_t)C_->m + 1 : 1),
-          rh1(ctx_, one_launch ? (size_t)C_->m + 1 : 1), rh2(ctx_, one_launch ? (size_t)C_->m + 1 : 1),
-          flip2(ctx_, one_launch ? (size_t)C_->m + 1 : 1), dcur(ctx_, one_launch ? (size_t)C_->m + 1 : 1),
-          h(ctx_, (size_t)C_->m + 1),
-          st(ctx_, 1), cntg(ctx_, batch_ ? (size_t)(2 * batch_->ngraphs) : 1),
-          pg(ctx_, batch_ ? (size_t)batch_->ngraphs : 1),
-          seg(ctx_, (size_t)std::max<int64_t>(cap_ / 8, 4096)), efound(ctx_, (size_t)cap_) {
-        GA_CUDA(cudaMemsetAsync(st.p, 0, sizeof(TriFrontState), ctx->stream));
+    Impl(ga_ctx ctx_, ga_csr A, const KtBatch* batch_)
+        : ctx(ctx_), m(A->m), nnz(A->nnz), cap(std::max<int64_t>(A->nnz, 1)), batch(batch_),
+          ng(batch_ ? batch_->ngraphs : 0), one_launch(!batch_ && ctx_->device_loops && trif_loop_fits(ctx_)),
+          nseg(std::max<int64_t>(cap / 8, 4096)) {
+        mem = DBuf<unsigned char>(ctx, carve(nullptr));
+        carve(mem.p);
+        tri_kt_carve(kt_scr, m, cap, &t);
+        words = WordRanks{t.bits, t.pre};
+        W.m = W.n = m;
+        W.nnz = nnz;
+        W.rst = A->rst;
+        W.col = pcol;
+        W.dtype = GA_INT32;
+        GA_CUDA(cudaMemsetAsync(st, 0, sizeof(TriFrontState), ctx->stream));
         if (batch) {
-            GA_CUDA(cudaMemsetAsync(cntg.p, 0, sizeof(int32_t) * (size_t)(2 * ng), ctx->stream));
-            GA_CUDA(cudaMemsetAsync(pg.p, 0, sizeof(long long) * (size_t)ng, ctx->stream));
+            GA_CUDA(cudaMemsetAsync(cntg, 0, sizeof(int32_t) * (size_t)(2 * ng), ctx->stream));
+            GA_CUDA(cudaMemsetAsync(pg, 0, sizeof(long long) * (size_t)ng, ctx->stream));
         }
-        a.cr = C->rst;
-        a.cc = C->col;
+        a.cr = A->rst;
+        a.cc = pcol;
+        a.ac = A->col;
         a.row_of = row_of;
-        a.mir = mir;
         a.crank = t.crank;
+        a.rank = t.rank;
         a.ocount = t.ocount;
         a.dpos = t.dpos;
-        a.oid = b.oid;
-        a.sup = b.sup;
-        a.state = b.state;
-        a.deg = deg.p;
-        a.upc = upc.p;
-        a.h = h.p;
-        a.H = H.p;
-        a.rd = rd.p;
-        a.rh = rh.p;
-        a.mark = mark.p;
-        a.touched = touched.p;
-        a.flip = flip.p;
-        a.f0 = b.f0;
-        a.f1 = b.f1;
-        a.seg = seg.p;
-        a.efound = efound.p;
-        a.segcap = (int64_t)seg.count;
-        a.st = st.p;
+        a.oid = oid;
+        a.orec = orec;
+        a.sup = sup;
+        a.state = state;
+        a.deg = deg;
+        a.upc = upc;
+        a.h = h;
+        a.H = H;
+        a.rd = rd;
+        a.rh = rh;
+        a.mark = mark;
+        a.touched = touched;
+        a.flip = flip;
+        a.f0 = f0;
+        a.f1 = f1;
+        a.seg = seg;
+        a.efound = efound;
+        a.segcap = nseg;
+        a.st = st;
         a.ctr = ctx->d_counters;
-        a.m = C->m;
-        a.nnz = C->nnz;
+        a.m = m;
+        a.nnz = nnz;
         a.k = 0;
         a.gid = batch ? batch->gid : nullptr;
         a.kg = batch ? batch->kg : nullptr;
         a.nvert = batch ? batch->nvert : nullptr;
         a.done_g = batch ? batch->done_g : nullptr;
         a.iters_g = batch ? batch->iters_g : nullptr;
-        a.cntg = batch ? cntg.p : nullptr;
-        a.pg = batch ? pg.p : nullptr;
+        a.cntg = batch ? cntg : nullptr;
+        a.pg = batch ? pg : nullptr;
         a.ngraphs = ng;
-        // one-launch loop: its frontiers share f0, so f1 holds segments; b.tc,
-        // b.flag and b.tr are free until compact() (touched vertices have
-        // entries, so they are at most cap)
-        a.rd1 = rd1.p;
-        a.rd2 = rd2.p;
-        a.rh1 = rh1.p;
-        a.rh2 = rh2.p;
-        a.touched1 = b.tc;
-        a.touched2 = b.flag;
-        a.flip1 = b.tr;
-        a.flip2 = flip2.p;
-        a.dcur = one_launch ? dcur.p : nullptr;
-        a.seg1 = reinterpret_cast<int2*>(b.f1);
+        // one-launch loop: its frontiers share f0, so f1 holds segments
+        a.rd1 = rd1;
+        a.rd2 = rd2;
+        a.rh1 = rh1;
+        a.rh2 = rh2;
+        a.touched1 = touched1;
+        a.touched2 = touched2;
+        a.flip1 = flip1;
+        a.flip2 = flip2;
+        a.dcur = one_launch ? dcur : nullptr;
+        a.seg1 = reinterpret_cast<int2*>(f1);
         a.segcap1 = std::min<int64_t>(a.segcap, cap / 2);
+        GA_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+    }
+
+    // Places of the arrays from `base` on; the bytes they take.
+    size_t carve(unsigned char* base) {
+        size_t off = 0;
+        auto take = [&](auto** p, int64_t count) {
+            using E = std::remove_reference_t<decltype(**p)>;
+            *p = reinterpret_cast<E*>(base + off);
+            off += align256(sizeof(E) * (size_t)count);
+        };
+        for (int32_t** p : {&row_of, &pcol, &oid, &orec, &sup, &f0, &f1, &efound}) take(p, cap);
+        for (int32_t** p : {&deg, &upc, &H, &rd, &rh, &mark, &touched, &flip}) take(p, m + 1);
+        for (int32_t** p : {&rd1, &rd2, &rh1, &rh2, &touched1, &touched2, &flip1, &flip2, &dcur})
+            take(p, one_launch ? m + 1 : 1);
+        take(&h, m + 1);
+        take(&state, cap);
+        take(&st, 1);
+        take(&cntg, batch ? 2 * ng : 1);
+        take(&pg, batch ? ng : 1);
+        take(&seg, nseg);
+        kt_scr = base + off;
+        return off + tri_kt_bytes(m, cap);
+    }
+
+    ~Impl() {
+        if (ready) cudaEventDestroy(ready);
+    }
+
+    // The matrix as the loop stores it, its records and the counts of C_0;
+    // iteration 0's supports by one listing of every triangle; the first
+    // frontier.
+    void begin() {
+        const int grid_ent = grid_for(cap, 256, ctx->num_sms * 16);
+        ga_csr_s A = W;
+        A.col = const_cast<int32_t*>(a.ac);
+        expand_rows(ctx, &A, row_of);
+        trikt_partition(ctx, a.cr, a.ac, m, nnz, row_of, t, batch, pcol);
+            k_trif_init_rows<<<grid_for(m, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a);
+        post_launch("trif_init_rows");
+        if (nnz) {
+            k_trif_records<<<grid_ent, 256, 0, ctx->stream>>>(a, words, t.dpos);
+            post_launch("trif_records");
+        }
+        k_trif_init_counts<<<grid_for(std::max<int64_t>(m, ng), 256, ctx->num_sms * 2), 256, 0, ctx->stream>>>(a);
+        post_launch("trif_init_counts");
+        tri_kt_support(ctx, &W, sup, t, cap);
+        if (nnz) {
+            ProfScope ps(ctx, "trif_seed");
+            k_trif_seed<<<grid_for((cap + kSeedWords - 1) / kSeedWords, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a);
+            post_launch("trif_seed");
+        }
     }
 
     void run(int k) {
-        const int64_t m = a.m, nnz = a.nnz;
         a.k = k;
-        const int grid_ent = grid_for(nnz > 0 ? nnz : 1, 256, ctx->num_sms * 16);
         if (first) {
             first = false;
-            // iteration 0's supports: one listing of every triangle
-            tri_kt_support(ctx, C, b.sup, t, cap);
-            ProfScope ps(ctx, "trif_seed");
-            k_trif_init_rows<<<grid_for(m, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a);
-            post_launch("trif_init_rows");
-            if (nnz) {
-                k_trif_seed<<<grid_ent, 256, 0, ctx->stream>>>(a);
-                post_launch("trif_seed");
-            }
-            k_trif_init_counts<<<grid_for(std::max<int64_t>(m * 32, ng), 256, ctx->num_sms * 16), 256, 0,
-                                 ctx->stream>>>(a);
-            post_launch("trif_init_counts");
+            begin();
         } else {
             GA_REQUIRE(!batch, GA_ERR_INVALID_ARG, "a batched frontier k-truss runs one k");
             // a new k: the loop state restarts (the running work totals stay)
             ProfScope ps(ctx, "trif_seed");
-            GA_CUDA(cudaMemsetAsync(st.p, 0, offsetof(TriFrontState, live), ctx->stream));
+            GA_CUDA(cudaMemsetAsync(st, 0, offsetof(TriFrontState, live), ctx->stream));
             if (nnz) {
-                k_trif_reseed<<<grid_ent, 256, 0, ctx->stream>>>(a);
+                k_trif_reseed<<<grid_for((cap + kSeedWords - 1) / kSeedWords, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a);
                 post_launch("trif_reseed");
             }
         }
@@ -2258,53 +2435,55 @@ struct TriFront::Impl {
         run_cached_loop(ctx, slot, body, m + 1);
     }
 
-    // Entries kept and iteration count of the last run (one synchronisation).
+    // Entries kept and iteration count of the last run (one wait, during
+    // which the device goes on to the kept entries' places).
     int64_t result(int* iters) {
-        TriFrontState hs;
-        GA_CUDA(cudaMemcpyAsync(&hs, st.p, sizeof(TriFrontState), cudaMemcpyDeviceToHost, ctx->stream));
-        GA_CUDA(cudaStreamSynchronize(ctx->stream));
-        GA_REQUIRE(!hs.failed, GA_ERR_TIMEOUT, "k-truss: a wait inside the loop ran out");
-        if (iters) *iters = hs.iters;
-        return (int64_t)hs.ent;
+        static_assert(sizeof(TriFrontResult) <= 64, "the context's pinned words");
+        GA_CUDA(cudaMemcpyAsync(ctx->h_pinned, &st->iters, sizeof(TriFrontResult), cudaMemcpyDeviceToHost,
+                                ctx->stream));
+        GA_CUDA(cudaEventRecord(ready, ctx->stream));
+        {
+            ProfScope ps(ctx, "trif_compact");
+            const int64_t nw = rank_words(nnz);
+            k_trif_keep<<<grid_for(nw * 32, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(a, words);
+            post_launch("trif_keep");
+            scan_exclusive_i32_scratch(ctx, t.pre, t.pre, nw, t.scan_scr);
+        }
+        GA_CUDA(cudaEventSynchronize(ready));
+        TriFrontResult r;
+        std::memcpy(&r, ctx->h_pinned, sizeof(r));
+        GA_REQUIRE(!r.failed, GA_ERR_TIMEOUT, "k-truss: a wait inside the loop ran out");
+        if (iters) *iters = r.iters;
+        return (int64_t)r.ent;
     }
 
-    // The kept entries' row starts and columns, rows in column order.
-    void compact(int32_t* rst, int32_t* col) {
-        const int64_t m = a.m, nnz = a.nnz;
+    // After result(): the kept entries, values one, rows in column order.
+    void compact(int32_t* rst, int32_t* col, int32_t* val) {
         ProfScope ps(ctx, "trif_compact");
-        k_trif_keep<<<grid_for(cap, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(a, cap, b.flag);
-        post_launch("trif_keep");
-        scan_exclusive_i32_scratch(ctx, b.flag, b.flag, cap, b.scan_scr);
-        k_trif_out<<<grid_for(nnz > m ? nnz : m + 1, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a, b.flag, col, rst);
+        k_trif_out<<<grid_for(nnz > m ? nnz : m + 1, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(a, words, col, val,
+                                                                                                  rst);
         post_launch("trif_out");
     }
 };
 
-TriFront::TriFront(ga_ctx ctx, ga_csr C, const int32_t* row_of, const int32_t* mir, const TriKt& t, int64_t cap,
-                   const TriFrontBufs& b, const KtBatch* batch)
-    : impl_(new Impl(ctx, C, row_of, mir, t, cap, b, batch)) {}
+TriFront::TriFront(ga_ctx ctx, ga_csr A, const KtBatch* batch) : impl_(new Impl(ctx, A, batch)) {}
 
 TriFront::~TriFront() { delete impl_; }
 
 void TriFront::run(int k) { impl_->run(k); }
 
-int64_t TriFront::result(int* iters) { return impl_->result(iters); }
-
-void TriFront::compact(int32_t* rst, int32_t* col) { impl_->compact(rst, col); }
-
-int tri_kt_frontier(ga_ctx ctx, ga_csr C, int k, const int32_t* row_of, const int32_t* mir, const TriKt& t,
-                    int64_t cap, const TriFrontBufs& b, const KtBatch* batch) {
-    TriFront f(ctx, C, row_of, mir, t, cap, b, batch);
-    f.run(k);
-    int iters = 0;
-    const int64_t kept = f.result(&iters);
-    f.compact(b.tr, b.tc);
-    const int64_t m = C->m;
-    GA_CUDA(cudaMemcpyAsync(C->rst, b.tr, sizeof(int32_t) * (size_t)(m + 1), cudaMemcpyDeviceToDevice, ctx->stream));
-    if (kept) GA_CUDA(cudaMemcpyAsync(C->col, b.tc, sizeof(int32_t) * (size_t)kept, cudaMemcpyDeviceToDevice,
-                                      ctx->stream));
-    C->nnz = kept;
-    return iters;
+ga_csr TriFront::result(int* iters) {
+    const int64_t kept = impl_->result(iters);
+    ga_csr C = csr_alloc(impl_->ctx, impl_->m, impl_->m, kept, GA_INT32);
+    try {
+        impl_->compact(C->rst, C->col, static_cast<int32_t*>(C->val));
+    } catch (...) {
+        csr_destroy(impl_->ctx, C);
+        throw;
+    }
+    C->unit = 1;
+    C->sym = 1;
+    return C;
 }
 
 }  // namespace ga
