@@ -104,6 +104,7 @@ struct MxmArgs {
     int32_t cta_cap;
     unsigned long long* ctr;  // context work counters (GA_CTR_*)
     int64_t warp_max_flops, heavy_flops;
+    bool small;               // warp_max_flops is only a bound (warp_limit)
     // hybrid form: rows whose inner-product work (sum over mask entries of
     // min(|A_i|, |B^T_j|)) times hybrid_ratio is below their Gustavson work
     // are listed in dot_tasks (row, first mask entry; count in the queue),
@@ -121,6 +122,8 @@ __global__ void k_reset_queue(MxmQueue* q) {
 }
 
 // ------------------------------------------------------------------ binning
+constexpr int kBinThreads = 256;
+
 // Products of A entries [t0, t1) at stride `step`, this thread's share.
 template <typename T, typename A>
 __device__ __forceinline__ long long bin_products(const MxmArgs<T, A>& p, int32_t t0, int32_t t1, int32_t step) {
@@ -133,6 +136,47 @@ __device__ __forceinline__ long long bin_products(const MxmArgs<T, A>& p, int32_
     return f;
 }
 
+// Products up to which a short row is a warp's, in a product that is small for
+// the device. A warp takes about 1.6 ns per product; a CTA 0.1 ns, but 5 us per
+// row, and rows wait when there are more of them than CTAs. With the rows of f
+// products or more sent to CTAs, at most total / f of them, the slowest on
+// either side is fastest near f = kWarpShare * sqrt(total). Every CTA estimates
+// the total from the same kSamples of A's entries, which takes 2 us (support of
+// 1,000 vertices with 20 neighbours, all rows alike: 31 -> 33 us). With 32,768
+// at every size, and so: supports of R-MAT 9, 10, 12, 13 (0.27M to 19M
+// products) 64 / 168 / 273 / 398 and 34 / 49 / 109 / 114 us, of 1,000 vertices
+// with 180 neighbours 314 and 123, MSA k-truss of R-MAT 11 960 and 402. With
+// kWarpShare 2.6 and 4.0 R-MAT 13 takes 136 and 197, with 1.1 5,000 vertices
+// with 80 neighbours take 219 instead of 171.
+constexpr int kSamples = 4 * kBinThreads;
+constexpr float kWarpShare = 1.6f;
+constexpr long long kWarpLeast = 1024;
+
+template <typename T, typename A>
+__device__ __forceinline__ long long warp_limit(const MxmArgs<T, A>& p) {
+    if (!p.small) return p.warp_max_flops;
+    __shared__ long long part[kBinThreads / 32];
+    const int64_t first = p.ar[0], nnz = (int64_t)p.ar[p.m] - first;
+    const int64_t count = nnz < kSamples ? nnz : kSamples;
+    long long f = 0;
+#pragma unroll
+    for (int x = 0; x < kSamples / kBinThreads; ++x) {
+        const int64_t t = x * kBinThreads + threadIdx.x;
+        if (t < count) {
+            const int32_t k = __ldg(p.ac + first + t * nnz / count);
+            f += __ldg(p.bre + k) - __ldg(p.br + k);
+        }
+    }
+    f = warp_sum<long long>(f);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = f;
+    __syncthreads();
+    f = 0;
+    for (int w = 0; w < kBinThreads / 32; ++w) f += part[w];
+    const float total = count ? (float)f * ((float)nnz / (float)count) : 0.0f;
+    const long long share = max(kWarpLeast, (long long)(kWarpShare * sqrtf(total)));
+    return share < p.warp_max_flops ? share : p.warp_max_flops;
+}
+
 // The bins of `take` rows per warp at a time (up to 32; fewer when the matrix
 // has not that many rows for every resident warp). Queue places are reserved
 // for the rows together: with one atomic per row, a union of a million short rows
@@ -141,7 +185,6 @@ __device__ __forceinline__ long long bin_products(const MxmArgs<T, A>& p, int32_
 // (a power-law graph's hubs sit together or a power of two apart), and rows
 // of more than kBinLong entries are summed by the whole CTA (R-MAT 18
 // support: 236 -> 69 us).
-constexpr int kBinThreads = 256;
 constexpr int kBinLong = 1024;
 
 template <typename T, typename A>
@@ -152,6 +195,7 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
     __shared__ int s_nlong;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long warp_max = warp_limit(p);
     unsigned long long my_flops = 0, my_mask = 0, my_entries = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(&p.ctr[GA_CTR_LAUNCHES], 1ull);
@@ -231,7 +275,7 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
             }
         }
         // warp rows
-        const bool short_row = todo && mi <= kWarpSlots<A> && f <= p.warp_max_flops;
+        const bool short_row = todo && mi <= kWarpSlots<A> && f <= warp_max;
         unsigned set = __ballot_sync(FULL, short_row);
         if (set) {
             int pos = 0;
@@ -963,8 +1007,12 @@ static void launch_masked(ga_ctx ctx, ga_csr A_, ga_csr B_, ga_csr M_, T* cv, Mx
     p.clip = mre != nullptr && rows.clip;
     p.cv = cv; p.m = M_->m; p.q = q; p.warp_rows = warp_rows; p.cta_items = cta_items; p.cta_cap = cta_cap;
     p.ctr = ctx->d_counters;
-    p.warp_max_flops = ctx->tune.warp_max_flops;
     p.heavy_flops = ctx->tune.heavy_flops;
+    p.warp_max_flops = ctx->tune.warp_max_flops;
+    // the limit reaches the option's default at (32,768 / kWarpShare)^2
+    // products; rows of mean length give a lower bound of their number
+    const double most = (double)MxmTune().warp_max_flops / kWarpShare;
+    p.small = p.m > 0 && (double)A_->nnz * (double)B_->nnz < most * most * (double)B_->m;
     p.btr = btr;
     p.dot_tasks = dot_tasks;
     p.hybrid_ratio = ctx->tune.hybrid_ratio;

@@ -111,7 +111,8 @@ GA_API int ga_version(int* major, int* minor);
  * the autotuner chooses; results do not depend on it):
  * GA_OPT_MXM_WARP_FLOPS (32768): output rows with at most this many
  * Gustavson products (and at most 256 mask entries) are computed by one
- * warp, larger rows by CTAs; GA_OPT_MXM_HEAVY_FLOPS (2^20): CTA work of rows
+ * warp, larger rows by CTAs (fewer in a product that is small for the device:
+ * an upper bound then); GA_OPT_MXM_HEAVY_FLOPS (2^20): CTA work of rows
  * with at least this many products is scheduled first;
  * GA_OPT_MXM_CTAS_PER_SM (0 = as many as fit): persistent grid size;
  * GA_OPT_DOT_CHUNK (8): mask entries per warp task of the inner-product form;
