@@ -141,38 +141,46 @@ __device__ __forceinline__ long long bin_products(const MxmArgs<T, A>& p, int32_
 // row, and rows wait when there are more of them than CTAs. With the rows of f
 // products or more sent to CTAs, at most total / f of them, the slowest on
 // either side is fastest near f = kWarpShare * sqrt(total). Every CTA estimates
-// the total from the same kSamples of A's entries, which takes 2 us (support of
-// 1,000 vertices with 20 neighbours, all rows alike: 31 -> 33 us). With 32,768
-// at every size, and so: supports of R-MAT 9, 10, 12, 13 (0.27M to 19M
+// the total from the same kSamples of A's entries, while it reads its first rows
+// (where all rows are alike, it is 0.5 to 2 us lost; with four times as many
+// samples 2 to 5). With 32,768 at every size, and so: supports of R-MAT 9, 10, 12, 13 (0.27M to 19M
 // products) 64 / 168 / 273 / 398 and 34 / 49 / 109 / 114 us, of 1,000 vertices
 // with 180 neighbours 314 and 123, MSA k-truss of R-MAT 11 960 and 402. With
 // kWarpShare 2.6 and 4.0 R-MAT 13 takes 136 and 197, with 1.1 5,000 vertices
 // with 80 neighbours take 219 instead of 171.
-constexpr int kSamples = 4 * kBinThreads;
+constexpr int kSamples = kBinThreads;
 constexpr float kWarpShare = 1.6f;
 constexpr long long kWarpLeast = 1024;
 
+// This thread's sample: the loads are under way while the first rows are read.
+struct BinSample {
+    int32_t b = 0, e = 0;
+    int64_t nnz, count;
+};
 template <typename T, typename A>
-__device__ __forceinline__ long long warp_limit(const MxmArgs<T, A>& p) {
-    if (!p.small) return p.warp_max_flops;
-    __shared__ long long part[kBinThreads / 32];
-    const int64_t first = p.ar[0], nnz = (int64_t)p.ar[p.m] - first;
-    const int64_t count = nnz < kSamples ? nnz : kSamples;
-    long long f = 0;
-#pragma unroll
-    for (int x = 0; x < kSamples / kBinThreads; ++x) {
-        const int64_t t = x * kBinThreads + threadIdx.x;
-        if (t < count) {
-            const int32_t k = __ldg(p.ac + first + t * nnz / count);
-            f += __ldg(p.bre + k) - __ldg(p.br + k);
-        }
+__device__ __forceinline__ BinSample bin_sample(const MxmArgs<T, A>& p) {
+    BinSample s;
+    const int64_t first = p.ar[0];
+    s.nnz = (int64_t)p.ar[p.m] - first;
+    s.count = s.nnz < kSamples ? s.nnz : kSamples;
+    if (threadIdx.x < s.count) {
+        const int32_t k = __ldg(p.ac + first + threadIdx.x * s.nnz / s.count);
+        s.b = __ldg(p.br + k);
+        s.e = __ldg(p.bre + k);
     }
-    f = warp_sum<long long>(f);
+    return s;
+}
+
+// All threads of the CTA.
+template <typename T, typename A>
+__device__ __forceinline__ long long warp_limit(const MxmArgs<T, A>& p, const BinSample& s) {
+    __shared__ long long part[kBinThreads / 32];
+    long long f = warp_sum<long long>(s.e - s.b);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = f;
     __syncthreads();
     f = 0;
     for (int w = 0; w < kBinThreads / 32; ++w) f += part[w];
-    const float total = count ? (float)f * ((float)nnz / (float)count) : 0.0f;
+    const float total = s.count ? (float)f * ((float)s.nnz / (float)s.count) : 0.0f;
     const long long share = max(kWarpLeast, (long long)(kWarpShare * sqrtf(total)));
     return share < p.warp_max_flops ? share : p.warp_max_flops;
 }
@@ -195,7 +203,9 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
     __shared__ int s_nlong;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const long long warp_max = warp_limit(p);
+    long long warp_max = p.small ? -1 : p.warp_max_flops;
+    BinSample sample;
+    if (p.small) sample = bin_sample(p);
     unsigned long long my_flops = 0, my_mask = 0, my_entries = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(&p.ctr[GA_CTR_LAUNCHES], 1ull);
@@ -240,6 +250,7 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
             const long long fr = warp_sum<long long>(bin_products(p, b + lane, e, 32));
             if (lane == r) f = fr;
         }
+        if (warp_max < 0) warp_max = warp_limit(p, sample);
         // rows without products: explicit zeros
         for (unsigned rows = __ballot_sync(FULL, live && f == 0); rows; rows &= rows - 1) {
             const int r = __ffs(rows) - 1;
