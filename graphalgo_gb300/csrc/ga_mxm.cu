@@ -82,7 +82,13 @@ struct MxmQueue {
     int32_t warp_next;
     int32_t cta_next;
     int32_t dot_count;     // hybrid form: inner-product tasks listed
-    unsigned long long flops;
+    int32_t split_count;   // windows that heavy rows were split into
+};
+
+// Shares of the whole that a row is split into, and the products it has at least.
+struct BinSplit {
+    float shares;
+    long long least;
 };
 
 template <typename T, typename A>
@@ -104,7 +110,8 @@ struct MxmArgs {
     int32_t cta_cap;
     unsigned long long* ctr;  // context work counters (GA_CTR_*)
     int64_t warp_max_flops, heavy_flops;
-    bool small;               // warp_max_flops is only a bound (warp_limit)
+    bool small;               // warp_max_flops is only a bound, and heavy rows are split
+    BinSplit split;
     // hybrid form: rows whose inner-product work (sum over mask entries of
     // min(|A_i|, |B^T_j|)) times hybrid_ratio is below their Gustavson work
     // are listed in dot_tasks (row, first mask entry; count in the queue),
@@ -117,7 +124,7 @@ struct MxmArgs {
 __global__ void k_reset_queue(MxmQueue* q) {
     if (threadIdx.x == 0) {
         q->warp_count = 0; q->heavy_count = 0; q->normal_count = 0;
-        q->warp_next = 0; q->cta_next = 0; q->dot_count = 0; q->flops = 0ull;
+        q->warp_next = 0; q->cta_next = 0; q->dot_count = 0; q->split_count = 0;
     }
 }
 
@@ -171,19 +178,32 @@ __device__ __forceinline__ BinSample bin_sample(const MxmArgs<T, A>& p) {
     return s;
 }
 
-// All threads of the CTA.
-template <typename T, typename A>
-__device__ __forceinline__ long long warp_limit(const MxmArgs<T, A>& p, const BinSample& s) {
+// Products of the whole, estimated. All threads of the CTA.
+__device__ __forceinline__ float bin_total(const BinSample& s) {
     __shared__ long long part[kBinThreads / 32];
     long long f = warp_sum<long long>(s.e - s.b);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = f;
     __syncthreads();
     f = 0;
     for (int w = 0; w < kBinThreads / 32; ++w) f += part[w];
-    const float total = s.count ? (float)f * ((float)s.nnz / (float)s.count) : 0.0f;
-    const long long share = max(kWarpLeast, (long long)(kWarpShare * sqrtf(total)));
-    return share < p.warp_max_flops ? share : p.warp_max_flops;
+    return s.count ? (float)f * ((float)s.nnz / (float)s.count) : 0.0f;
 }
+
+// A row of more products than its share of the whole is cut into as many
+// windows as it holds shares, each of them an item that meets only the part of
+// the B rows inside it: as one item, the heaviest row of R-MAT 16 (1.4M
+// products) keeps a CTA busy for nearly as long as the rest takes the whole
+// device. Items of half a share and more start first. Support of R-MAT 14, 15,
+// 17 by MSA 353 / 584 / 1,012 and 331 / 559 / 938 us, of R-MAT 12, 14, 16 (4 per
+// vertex) by merging 322 / 1,143 / 1,014 and 224 / 742 / 545; MSA k-truss of
+// R-MAT 16 6.5 and 5.7 ms. MSA rows of fewer than kSplitLeast products are not
+// worth another look at A's row (R-MAT 12 from 32,768 on: 98 and 111 us). Of
+// 608, 912, 1,216 and 1,824 shares MSA is best with 912 (R-MAT 14: 314, 331,
+// 332, 355; R-MAT 16: 993, 988, 955, 965), merging, which takes three times as
+// long per product, with 1,824 (R-MAT 15: 1,459, 1,472, 1,397, 1,257).
+constexpr BinSplit kSplit = {912.0f, 131072}, kSplitMerge = {1824.0f, 32768};
+constexpr int kSplitSlots = 32;             // mask slots that a window has at least
+constexpr int kSplitItems = 4096;           // windows of all split rows together
 
 // The bins of `take` rows per warp at a time (up to 32; fewer when the matrix
 // has not that many rows for every resident warp). Queue places are reserved
@@ -200,10 +220,13 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
     __shared__ int32_t s_long[kBinThreads];           // the CTA's long rows: thread that holds each
     __shared__ long long s_sum[kBinThreads];          // products of the row held by each thread
     __shared__ int2 s_range[kBinThreads];
-    __shared__ int s_nlong;
+    __shared__ int s_nlong, s_at;
+    __shared__ int s_short[kBinThreads / 32];
+    __shared__ unsigned long long s_work[3];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    long long warp_max = p.small ? -1 : p.warp_max_flops;
+    if (threadIdx.x < 3) s_work[threadIdx.x] = 0;
+    long long warp_max = p.small ? -1 : p.warp_max_flops, split = INT64_MAX, heavy_min = p.heavy_flops;
     BinSample sample;
     if (p.small) sample = bin_sample(p);
     unsigned long long my_flops = 0, my_mask = 0, my_entries = 0;
@@ -215,7 +238,8 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
     const int64_t step = (int64_t)gridDim.x * (kBinThreads / 32);
     for (int64_t g0 = (int64_t)blockIdx.x * (kBinThreads / 32); g0 < groups; g0 += step) {
         const int64_t g = g0 + wid;
-        const int64_t i = g < groups && lane < take ? (g + 1571ll * lane) % groups + (int64_t)lane * groups : p.m;
+        int64_t i = p.m;
+        if (g < groups && lane < take) i = take == 1 ? g : (g + 1571ll * lane) % groups + (int64_t)lane * groups;
         int32_t mb = 0, me = 0, ab = 0, ae = 0, count = 0;
         if (i < p.m) {
             mb = p.mr[i];
@@ -250,7 +274,12 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
             const long long fr = warp_sum<long long>(bin_products(p, b + lane, e, 32));
             if (lane == r) f = fr;
         }
-        if (warp_max < 0) warp_max = warp_limit(p, sample);
+        if (warp_max < 0) {
+            const float total = bin_total(sample);
+            warp_max = min((long long)p.warp_max_flops, max(kWarpLeast, (long long)(kWarpShare * sqrtf(total))));
+            split = max(p.split.least, (long long)(total / p.split.shares));
+            heavy_min = min(heavy_min, split / 2);
+        }
         // rows without products: explicit zeros
         for (unsigned rows = __ballot_sync(FULL, live && f == 0); rows; rows &= rows - 1) {
             const int r = __ffs(rows) - 1;
@@ -288,17 +317,20 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
         // warp rows
         const bool short_row = todo && mi <= kWarpSlots<A> && f <= warp_max;
         unsigned set = __ballot_sync(FULL, short_row);
-        if (set) {
-            int pos = 0;
-            if (lane == 0) pos = atomicAdd(&p.q->warp_count, __popc(set));
-            pos = __shfl_sync(FULL, pos, 0);
-            if (short_row) p.warp_rows[pos + __popc(set & ((1u << lane) - 1u))] = (int32_t)i;
+        if (lane == 0) s_short[wid] = __popc(set);
+        __syncthreads();
+        if (wid == 0) {
+            const int mine = lane < kBinThreads / 32 ? s_short[lane] : 0, incl = warp_incl_scan(mine);
+            if (lane < kBinThreads / 32) s_short[lane] = incl - mine;
+            if (lane == 31 && incl) s_at = atomicAdd(&p.q->warp_count, incl);
         }
+        __syncthreads();
+        if (short_row) p.warp_rows[s_at + s_short[wid] + __popc(set & ((1u << lane) - 1u))] = (int32_t)i;
         // CTA items: rows of one window together, the others window by window
         const bool cta_row = todo && !short_row;
         const int32_t* mcol = p.mc + mb;
-        const bool heavy = f >= p.heavy_flops;
-        const bool one = cta_row && mi <= kCtaSlots<A> && mcol[mi - 1] - mcol[0] < kWinCols;
+        const bool heavy = f >= heavy_min;
+        const bool one = cta_row && mi <= kCtaSlots<A> && f <= split && mcol[mi - 1] - mcol[0] < kWinCols;
         for (int h = 0; h < 2; ++h) {
             const bool in = one && heavy == (h == 0);
             set = __ballot_sync(FULL, in);
@@ -309,9 +341,14 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
             if (in) p.cta_items[h == 0 ? pos : p.cta_cap - 1 - pos] = make_int4((int)i, 0, mi, 0);
         }
         if (cta_row && !one) {
-            int s0 = 0;
+            int s0 = 0, slots = kCtaSlots<A>;
+            if (f > split) {
+                const int windows = (int)min(f / split + 1, (long long)(mi + kSplitSlots - 1) / kSplitSlots);
+                const int each = (mi + windows - 1) / windows;
+                if (each < slots && atomicAdd(&p.q->split_count, windows) + windows <= kSplitItems) slots = each;
+            }
             while (s0 < mi) {
-                int s1 = min(mi, s0 + kCtaSlots<A>);
+                int s1 = min(mi, s0 + slots);
                 const int32_t c0 = mcol[s0];
                 if (mcol[s1 - 1] - c0 >= kWinCols) {
                     const int64_t lim = (int64_t)c0 + (kWinCols - 1);
@@ -325,15 +362,20 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
             }
         }
     }
+    // one addition per CTA and counter, as for the warp rows' places: with the
+    // warps' own, 4,786 rows took 14 us instead of 7.4
     my_flops = warp_sum<unsigned long long>(my_flops);
     my_mask = warp_sum<unsigned long long>(my_mask);
     my_entries = warp_sum<unsigned long long>(my_entries);
-    if (lane == 0 && my_entries) atomicAdd(&p.ctr[GA_CTR_A_ENTRIES], my_entries);
-    if (lane == 0 && my_flops) {
-        atomicAdd(&p.q->flops, my_flops);
-        atomicAdd(&p.ctr[GA_CTR_PRODUCTS], my_flops);
+    if (lane == 0) {
+        if (my_flops) atomicAdd(&s_work[0], my_flops);
+        if (my_mask) atomicAdd(&s_work[1], my_mask);
+        if (my_entries) atomicAdd(&s_work[2], my_entries);
     }
-    if (lane == 0 && my_mask) atomicAdd(&p.ctr[GA_CTR_MASK_ENTRIES], my_mask);
+    __syncthreads();
+    if (threadIdx.x < 3 && s_work[threadIdx.x])
+        atomicAdd(&p.ctr[threadIdx.x == 0 ? GA_CTR_PRODUCTS : threadIdx.x == 1 ? GA_CTR_MASK_ENTRIES : GA_CTR_A_ENTRIES],
+                  s_work[threadIdx.x]);
 }
 
 // ------------------------------------------------------------------ lookups
@@ -1002,9 +1044,10 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
 }
 
 static int64_t cta_item_cap(int64_t m, int64_t n, int64_t mask_nnz) {
-    // windows per row <= ceil(m_i / kLeastCtaSlots) + ceil(n / kWinCols), and <= m_i
+    // windows per row <= ceil(m_i / kLeastCtaSlots) + ceil(n / kWinCols), and <= m_i;
+    // kSplitItems for the split rows
     const int64_t per_row = 1 + (n + kWinCols - 1) / kWinCols;
-    int64_t cap = m * per_row + mask_nnz / kLeastCtaSlots + 1;
+    int64_t cap = m * per_row + mask_nnz / kLeastCtaSlots + 1 + kSplitItems;
     if (cap > mask_nnz + 1) cap = mask_nnz + 1;
     return cap;
 }
@@ -1028,6 +1071,7 @@ static void launch_masked(ga_ctx ctx, ga_csr A_, ga_csr B_, ga_csr M_, T* cv, Mx
     p.cv = cv; p.m = M_->m; p.q = q; p.warp_rows = warp_rows; p.cta_items = cta_items; p.cta_cap = cta_cap;
     p.ctr = ctx->d_counters;
     p.heavy_flops = ctx->tune.heavy_flops;
+    p.split = LK == MD_MERGE ? kSplitMerge : kSplit;
     p.warp_max_flops = ctx->tune.warp_max_flops;
     // the limit reaches the option's default at (32,768 / kWarpShare)^2
     // products; rows of mean length give a lower bound of their number

@@ -13,12 +13,24 @@
 // contexts, which this entry point does not have.
 #include "ga_device.cuh"
 
+#include <algorithm>
 #include <mutex>
 
 namespace ga {
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = (size_t)16 << 20;  // 16 MiB
+// A shape is accepted when its queues, at 4,096 mask slots per CTA work item,
+// take at most 16 MiB. Items of 8-byte accumulators hold half as many slots
+// (at most 2^31 / 4,096 items more, of 16 bytes), and the windows of split rows
+// add up to 4,096 items.
+constexpr size_t kNoAllocShapeBytes = (size_t)16 << 20;
+constexpr size_t kNoAllocScratchBytes = kNoAllocShapeBytes + ((size_t)8 << 20) + ((size_t)128 << 10);
+
+size_t shape_bytes(int64_t m, int64_t n, int64_t mask_nnz) {
+    const int64_t windows = 1 + (n + (1 << 17) - 1) / (1 << 17);
+    const int64_t items = std::min(m * windows + mask_nnz / 4096 + 1, mask_nnz + 1);
+    return 256 + sizeof(int32_t) * (size_t)(m + 1) + 16 + sizeof(int4) * (size_t)items;
+}
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 __device__ unsigned long long g_noalloc_counters[GA_CTR_COUNT];
@@ -76,6 +88,7 @@ extern "C" int ga_mxm_masked_noalloc(void* stream, ga_algo algo, int64_t m, int6
     // the sorted merge (GA_HEAP) always reads B's values
     if ((!b_unit || algo == GA_HEAP) && !b_val) return GA_ERR_INVALID_ARG;
     // the scratch needed for this shape must fit the fixed array
+    if (shape_bytes(m, n, mask_nnz) > kNoAllocShapeBytes) return GA_ERR_INVALID_ARG;
     if (mxm_scratch_bytes(m, n, mask_nnz, false) > kNoAllocScratchBytes) return GA_ERR_INVALID_ARG;
     try {
         const NoAllocDevice& d = noalloc_setup();
