@@ -1,12 +1,13 @@
 // Masked SpGEMM C<M> = A*B (structural mask, C has M's pattern).
 //
 // Design (one pass, no symbolic phase: the output pattern is M's):
-//  1. k_row_bin: one warp per output row computes the mask length m_i and the
-//     Gustavson product count P_i = sum_{k in A_i} nnz(B_k). Rows with an
+//  1. k_row_bin computes each output row's mask length m_i and Gustavson
+//     product count P_i = sum_{k in A_i} nnz(B_k). Rows with an
 //     empty mask are skipped, rows without products get explicit zeros, short
-//     light rows (m_i <= kWarpSlots, P_i <= warp_max_flops) go to a warp
-//     queue, all others to a CTA queue as windows of at most kCtaSlots mask
-//     slots spanning fewer than kWinCols columns (heavy rows first).
+//     light rows (m_i <= kWarpSlots, P_i <= warp_max_flops or a limit of the
+//     product's own) go to a warp queue, all others to a CTA queue as windows
+//     of at most kCtaSlots mask slots spanning fewer than kWinCols columns
+//     (heavy rows first, the heaviest in more windows).
 //  2. k_mxm_masked: a persistent kernel (one wave of CTAs sized by occupancy)
 //     drains the CTA queue, then every warp drains the warp queue. The
 //     accumulator is indexed by mask slot and lives in shared memory.
@@ -196,7 +197,7 @@ __device__ __forceinline__ float bin_total(const BinSample& s) {
 // device. Items of half a share and more start first. Support of R-MAT 14, 15,
 // 17 by MSA 353 / 584 / 1,012 and 331 / 559 / 938 us, of R-MAT 12, 14, 16 (4 per
 // vertex) by merging 322 / 1,143 / 1,014 and 224 / 742 / 545; MSA k-truss of
-// R-MAT 16 6.5 and 5.7 ms. MSA rows of fewer than kSplitLeast products are not
+// R-MAT 16 6.5 and 5.7 ms. MSA rows of fewer than 131,072 products are not
 // worth another look at A's row (R-MAT 12 from 32,768 on: 98 and 111 us). Of
 // 608, 912, 1,216 and 1,824 shares MSA is best with 912 (R-MAT 14: 314, 331,
 // 332, 355; R-MAT 16: 993, 988, 955, 965), merging, which takes three times as

