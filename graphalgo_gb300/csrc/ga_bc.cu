@@ -407,11 +407,15 @@ __device__ __forceinline__ int bc_take(int64_t items, int most) {
     return n < 1 ? 1 : n > most ? most : (int)n;
 }
 
-// The warp's next task of the level.
+// The warp's first task of a level, dealt out by its number (neighbouring tasks
+// to different CTAs), and its next one. With the first from the counter too,
+// all the grid's warps take one, most of a small level's to find none (32
+// sources, 10,000 vertices: 445 us, so 429).
+__device__ __forceinline__ int32_t bc_first() { return blockIdx.x + (threadIdx.x >> 5) * gridDim.x; }
 __device__ __forceinline__ int32_t bc_next(const BcArgs& p) {
     int32_t t = 0;
     if ((threadIdx.x & 31) == 0) t = atomicAdd(&p.st->next, 1);
-    return __shfl_sync(0xffffffffu, t, 0);
+    return gridDim.x * kBcWarps + __shfl_sync(0xffffffffu, t, 0);
 }
 
 // Push: the row (unit key with columns mask) of vertex u and its
@@ -457,7 +461,7 @@ __global__ void __launch_bounds__(kBcThreads, 4) k_bc_forward(const BcArgs* __re
     if (st->mode != 0) {
         const int32_t task0 = p.ltask[d], ntask = p.ltask[d + 1] - task0;
         const int32_t row0 = p.lrow[d], nrow = p.lrow[d + 1] - row0;
-        for (int32_t t = bc_next(p); t < ntask + nrow; t = bc_next(p)) {
+        for (int32_t t = bc_first(); t < ntask + nrow; t = bc_next(p)) {
             int32_t u;
             if (t < ntask) {
                 const int2 task = p.htask[task0 + t];
@@ -478,7 +482,7 @@ __global__ void __launch_bounds__(kBcThreads, 4) k_bc_forward(const BcArgs* __re
         const int64_t units = p.m * p.nblk, nheavy = (int64_t)nchunk * p.nblk;
         const int take = bc_take(units, kBcUnits);
         const int64_t ntake = (units + take - 1) / take;
-        for (int64_t t = bc_next(p); t < nheavy + ntake; t = bc_next(p)) {
+        for (int64_t t = bc_first(); t < nheavy + ntake; t = bc_next(p)) {
             if (t < nheavy) {
                 const int blk = (int)(t / nchunk);
                 const int64_t off = (int64_t)blk * nchunk;
@@ -681,7 +685,7 @@ __global__ void __launch_bounds__(kBcThreads, 4) k_bc_backward(const BcArgs* __r
         const int32_t row0 = p.lrow[k - 1], row1 = p.lrow[k];
         const int take = bc_take(row1 - row0, kBcRows);
         const int32_t ntake = (row1 - row0 + take - 1) / take;
-        for (int32_t t = bc_next(p); t < ntask + ntake; t = bc_next(p)) {
+        for (int32_t t = bc_first(); t < ntask + ntake; t = bc_next(p)) {
             if (t < ntask) {  // a piece of a heavy row
                 const int2 task = p.htask[task0 + t];
                 const int64_t hr = heavy_row(p, task.x);
