@@ -355,6 +355,7 @@ static void tc_device(ga_ctx ctx, ga_algo algo, ga_csr A, int64_t* d_total, int6
         k_row_sums<<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(A->rst, end.p, cv.p, m, d_per_row,
                                                                                     tot);
         post_launch("row_sums");
+        settle_reads(ctx, A);
         return;
     }
     ga_csr L0 = extract_tri(ctx, A, true);
@@ -577,7 +578,9 @@ ga_csr ktruss_impl(ga_ctx ctx, ga_algo algo, ga_csr A, int k, int* iters_out, co
         // one listing, then only the triangles of the pruned edges
         TriFront front(ctx, A, batch);
         front.run(k);
-        return front.result(iters_out);
+        ga_csr C = front.result(iters_out);
+        settle_reads(ctx, A);
+        return C;
     }
     // C = A (a copy; its pattern shrinks in place)
     ga_csr C = copy_csr(ctx, A, GA_INT32);
@@ -786,11 +789,17 @@ struct KtSweep {
         ga_csr out = nullptr;
         int it = 0;
         if (fused) {
+            GA_REQUIRE(front != nullptr, GA_ERR_OOM, "k-truss sweep: an earlier call ran out of memory");
             front->run(k);
             // the only wait: what follows it runs while the caller takes the
             // result and asks for the next k
             out = front->result(&it);
-            maybe_rebuild(out);
+            try {
+                maybe_rebuild(out);
+            } catch (...) {
+                csr_destroy(ctx, out);
+                throw;
+            }
         } else {
             ga_csr res = ktruss_impl(ctx, algo, cur, k, &it, nullptr);
             csr_destroy(ctx, cur);

@@ -99,6 +99,13 @@ ga_csr csr_alloc(ga_ctx ctx, int64_t m, int64_t n, int64_t nnz, ga_dtype dt) {
     return A;
 }
 
+void settle_reads(ga_ctx ctx, ga_csr A) {
+    if (ctx->live.count(A->rst)) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GA_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+    if (cap == cudaStreamCaptureStatusNone) GA_CUDA(cudaStreamSynchronize(ctx->stream));
+}
+
 void csr_destroy(ga_ctx ctx, ga_csr A) {
     if (!A) return;
     if (A->copied) cudaEventDestroy(A->copied);

@@ -191,6 +191,10 @@ size_t scan_scratch_bytes(int64_t n);
 
 // Fills `count` values of type `dt` with 1.
 void fill_ones(ga_ctx ctx, void* vals, int64_t count, ga_dtype dt);
+// Before a call returns with kernels that read A still under way: when A's
+// memory is another context's, whose frees this context's stream does not
+// order, waits for them (not inside a stream capture).
+void settle_reads(ga_ctx ctx, ga_csr A);
 
 // Validates a device CSR; throws GA_ERR_INVALID_CSR when malformed.
 void validate_csr(ga_ctx ctx, const int32_t* rst, const int32_t* col, int64_t m, int64_t n, int64_t nnz);
