@@ -738,6 +738,7 @@ struct KtSweep {
     bool fused = false;
     ga_csr W = nullptr;    // fused: the matrix that the frontier state reads
     std::unique_ptr<TriFront> front;
+    int broken = GA_OK;    // fused, front gone: the error that ended the sweep
 
     ~KtSweep() {
         front.reset();
@@ -781,6 +782,12 @@ struct KtSweep {
         front.reset(new TriFront(ctx, W, nullptr));
     }
 
+    void give_up(ga_csr out, int code) {
+        csr_destroy(ctx, out);
+        front.reset();
+        broken = code;
+    }
+
     // The next C_k (owned by the caller), or nullptr after the empty one.
     ga_csr next(int* k_out, int* iters) {
         if (k_out) *k_out = k;
@@ -789,24 +796,37 @@ struct KtSweep {
         ga_csr out = nullptr;
         int it = 0;
         if (fused) {
-            GA_REQUIRE(front != nullptr, GA_ERR_OOM, "k-truss sweep: an earlier call ran out of memory");
-            front->run(k);
-            // the only wait: what follows it runs while the caller takes the
-            // result and asks for the next k
-            out = front->result(&it);
+            if (!front) fail(broken, "k-truss sweep: an earlier call failed; begin another sweep");
+            // An error leaves the state between two k: the supports are
+            // lowered for this k already, or (a wait that ran out) only partly.
+            // A further run on it would report another iteration count or a
+            // wrong truss, so it goes, and later calls report the error.
             try {
+                front->run(k);
+                // the only wait: what follows it runs while the caller takes the
+                // result and asks for the next k
+                out = front->result(&it);
                 maybe_rebuild(out);
+            } catch (const Error& e) {
+                give_up(out, e.code);
+                throw;
             } catch (...) {
-                csr_destroy(ctx, out);
+                give_up(out, GA_ERR_CUDA);
                 throw;
             }
         } else {
             ga_csr res = ktruss_impl(ctx, algo, cur, k, &it, nullptr);
-            csr_destroy(ctx, cur);
-            cur = res;
-            out = copy_csr(ctx, res, GA_INT32);
+            // `cur` stays the next call's input until the result is whole
+            try {
+                out = copy_csr(ctx, res, GA_INT32);
+            } catch (...) {
+                csr_destroy(ctx, res);
+                throw;
+            }
             out->unit = res->unit;
             out->sym = res->sym;
+            csr_destroy(ctx, cur);
+            cur = res;
         }
         if (iters) *iters = it;
         if (out->nnz == 0) finished = true;

@@ -401,7 +401,9 @@ GA_API int ga_ktruss(ga_ctx ctx, ga_algo algo, ga_csr A, int k, ga_csr* C, int* 
  * next: the triangles are listed once for the whole sweep and each k starts
  * from the supports the previous k left; other cases run one ga_ktruss per
  * k. A is copied by ga_ktruss_sweep_begin; free the sweep before its
- * context. No counterpart in the reference (its CLI runs one k per call). */
+ * context. An error (memory ran out, a wait ran out) ends a sweep whose
+ * state stays on the device: later calls return the same error. In the other
+ * cases the call can be made again. No counterpart in the reference (its CLI runs one k per call). */
 typedef struct ga_kt_sweep_s* ga_kt_sweep;
 GA_API int ga_ktruss_sweep_begin(ga_ctx ctx, ga_algo algo, ga_csr A, int kmin, ga_kt_sweep* sweep);
 GA_API int ga_ktruss_sweep_next(ga_kt_sweep sweep, ga_csr* C, int* k, int* iters);
