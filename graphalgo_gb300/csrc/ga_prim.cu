@@ -816,7 +816,11 @@ extern "C" {
 int ga_transpose(ga_ctx ctx, ga_csr A, ga_csr* AT) {
     if (!ctx || !A || !AT) return GA_ERR_INVALID_ARG;
     *AT = nullptr;
-    GA_API_BODY(ctx, *AT = transpose_csr(ctx, A));
+    GA_API_BODY(ctx, {
+        ga_csr T = transpose_csr(ctx, A);
+        settle_reads(ctx, A);
+        *AT = T;
+    });
 }
 
 int ga_extract_lower(ga_ctx ctx, ga_csr A, ga_csr* L) {
