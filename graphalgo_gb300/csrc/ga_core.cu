@@ -555,6 +555,7 @@ int ga_csr_download(ga_ctx ctx, ga_csr A, int32_t* rst, int32_t* col, void* val)
 
 int ga_csr_device_ptrs(ga_csr A, void** rst, void** col, void** val) {
     if (!A) return GA_ERR_INVALID_ARG;
+    A->lent = true;
     if (rst) *rst = A->rst;
     if (col) *col = A->col;
     if (val) *val = A->val;
@@ -568,6 +569,7 @@ int ga_csr_set_symmetric(ga_ctx ctx, ga_csr A, int symmetric) {
         return GA_ERR_SHAPE;
     }
     A->sym = symmetric;
+    A->declared = symmetric >= 0;
     return GA_OK;
 }
 

@@ -112,6 +112,8 @@ struct ga_csr_s {
     size_t cap = 0;  // allocated entries of col/val
     int unit = -1;   // all values equal 1: -1 unknown, 0 no, 1 yes
     int sym = -1;    // pattern and values symmetric: -1 unknown, 0 no, 1 yes
+    bool declared = false;  // sym was declared by the caller (ga_csr_set_symmetric)
+    bool lent = false;      // the caller has had the arrays' addresses: values may have changed since a check
     cudaEvent_t copied = nullptr;  // the handle's last download on the copy stream
 };
 

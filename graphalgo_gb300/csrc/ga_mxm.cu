@@ -1435,12 +1435,15 @@ void mxm_masked_launch(ga_ctx ctx, ga_algo algo, ga_csr A, ga_csr B, ga_csr M, v
 // hybrid 9.3 and 5.0; R-MAT 16 by MSA / MCA / merge 1.65 / 4.04 / 4.47 and
 // 1.17 / 2.69 / 3.08 ms; at 426,000 entries MSA 457 and 384 us; at 110,000
 // hybrid 407 and 437, inner product 122 and 144 us. A handle's first use pays
-// for the check: 0.16 ms at R-MAT 18.
+// for the check: 0.16 ms at R-MAT 18. A check holds for as long as nobody else
+// can write the values: a matrix whose arrays' addresses the caller has asked
+// for is multiplied in full, unless the caller declared it symmetric.
 constexpr int64_t kSymHalfNnz = 1 << 18;
 
 static bool mxm_symmetric(ga_ctx ctx, ga_csr A, ga_csr B, ga_csr M) {
     const bool one = A->rst == B->rst && A->col == B->col && A->val == B->val && A->rst == M->rst && A->col == M->col;
     if (!one || A->m != A->n || A->nnz < kSymHalfNnz) return false;
+    if (A->lent && !A->declared) return false;
     if (A->sym >= 0) return A->sym == 1;
     // the check synchronises: not inside a stream capture
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;

@@ -210,13 +210,23 @@ GA_API int ga_csr_download(ga_ctx ctx, ga_csr A, int32_t* rst, int32_t* col, voi
  * download; ga_csr_free on a handle orders its free after them. */
 GA_API int ga_csr_download_async(ga_ctx ctx, ga_csr A, int32_t* rst, int32_t* col, void* val);
 GA_API int ga_ctx_copy_sync(ga_ctx ctx);
+/* The arrays' device addresses. The pattern must not be written through them.
+ * Values may be written (ordered on the context's stream) with one limit: the
+ * library keeps what it once found out about a handle, whether all values are
+ * 1 and whether the matrix is symmetric, and does not notice the change. So
+ * write values before the handle's first use, or values that are neither all
+ * 1 before nor make a symmetric matrix asymmetric; after the latter call
+ * ga_csr_set_symmetric(ctx, A, -1). (Masked products by GA_MSA, GA_MCA and
+ * GA_HEAP need no such call: once the addresses have been asked for they rely
+ * on symmetry only where it was declared.) */
 GA_API int ga_csr_device_ptrs(ga_csr A, void** rst, void** col, void** val);
 GA_API int ga_csr_free(ga_ctx ctx, ga_csr A);
 /* Declares whether A is symmetric (pattern and values), which the
- * triangle-listing and inner-product forms, the symmetric k-truss loop and
- * BC otherwise check on the device once per handle (a search per entry for
- * its mirror). symmetric = 1: no check is run; A must be symmetric (a false
- * declaration gives wrong results). 0: A is treated as not symmetric. -1:
+ * triangle-listing and inner-product forms, the symmetric k-truss loop, BC
+ * and the masked products C<A> = A*A of 2^18 entries and more (half of a
+ * symmetric one is computed) otherwise check on the device once per handle (a
+ * search per entry for its mirror). symmetric = 1: no check is run; A must be
+ * symmetric, and stay so (a false declaration gives wrong results). 0: A is treated as not symmetric. -1:
  * the check runs again on the next use. No counterpart in the reference
  * (its CLI symmetrises the graphs it reads, src/main.cpp:221-222). */
 GA_API int ga_csr_set_symmetric(ga_ctx ctx, ga_csr A, int symmetric);
