@@ -787,6 +787,41 @@ static int bc_grid(ga_ctx ctx, K kernel) {
     return ctx->num_sms * std::max(per_sm, 1);
 }
 
+// Sizes of the state.
+struct BcSizes {
+    size_t units, pairs;  // (block, vertex) and (vertex, column)
+    int piece;
+    // pieces of the longer of the two heavy lists: at most nnz / piece full
+    // ones and one more per heavy vertex; a heavy vertex has a row in at
+    // most ns levels, and a level's rows of one vertex are one per block
+    size_t pieces, hrows;
+};
+
+static BcSizes bc_sizes(int64_t m, int64_t nnz, int64_t ns) {
+    BcSizes z;
+    z.units = (size_t)m * (size_t)((ns + 63) / 64);
+    z.pairs = (size_t)m * (size_t)ns;
+    z.piece = nnz > (int64_t)kBcDense * m ? kBcPieceDense : kBcPiece;
+    z.pieces = (size_t)(2 * (nnz / z.piece) + 1);
+    z.hrows = std::min(z.pairs, (size_t)(nnz / z.piece) * (size_t)ns) + 1;
+    return z;
+}
+
+// The arrays of bc_device, in its order, behind an FP64 copy and its
+// transpose; or what the transpose takes while it is made.
+int64_t bc_bytes(int64_t m, int64_t nnz, int64_t ns) {
+    const BcSizes z = bc_sizes(m, nnz, ns);
+    const size_t places = z.pieces * (size_t)((ns + 63) / 64);
+    const size_t state = sizeof(BcState) + sizeof(uint32_t) * (size_t)((m + 31) / 32) +
+                         4 * sizeof(unsigned long long) * z.units + 2 * sizeof(double) * z.pairs +
+                         (sizeof(int32_t) + sizeof(unsigned long long)) * z.pairs + sizeof(int32_t) * z.hrows +
+                         sizeof(int2) * z.pieces * (size_t)ns + sizeof(int32_t) * 3 * ((size_t)m + 3) +
+                         sizeof(int4) * z.pieces + sizeof(double) * places * 64 +
+                         (sizeof(unsigned long long) + sizeof(int32_t)) * places + sizeof(int32_t) * z.units;
+    const int64_t matrix = (int64_t)sizeof(int32_t) * (m + 1) + 12 * (nnz + 1);
+    return 2 * matrix + std::max((int64_t)state, transpose_bytes(nnz, GA_FP64));
+}
+
 // accumulate: add this batch's scores to d_bc instead of overwriting it.
 static void bc_device(ga_ctx ctx, ga_csr A, const int32_t* d_sources, int64_t nsrc, double* d_bc,
                       bool accumulate = false, const BcPacking* pk = nullptr) {
@@ -815,13 +850,9 @@ static void bc_device(ga_ctx ctx, ga_csr A, const int32_t* d_sources, int64_t ns
         ga_csr Av = unit ? A : Ad;
         if (!symmetric) AT = transpose_csr(ctx, Av);
         ga_csr ATu = symmetric ? Av : AT;
-        const size_t units = (size_t)m * nblk, pairs = (size_t)m * ns;
-        // pieces of the longer of the two heavy lists: at most nnz / piece full
-        // ones and one more per heavy vertex; a heavy vertex has a row in at
-        // most ns levels, and a level's rows of one vertex are one per block
-        const int piece = A->nnz > (int64_t)kBcDense * m ? kBcPieceDense : kBcPiece;
-        const size_t pieces = (size_t)(2 * (A->nnz / piece) + 1);
-        const size_t hrows = std::min(pairs, (size_t)(A->nnz / piece) * ns) + 1;
+        const BcSizes z = bc_sizes(m, A->nnz, ns);
+        const size_t units = z.units, pairs = z.pairs, pieces = z.pieces, hrows = z.hrows;
+        const int piece = z.piece;
         DBuf<BcState> st(ctx, 1);
         DBuf<uint32_t> seen(ctx, (size_t)(m + 31) / 32);
         DBuf<unsigned long long> words(ctx, 4 * units);  // V, F[0], F[1], F[2]

@@ -214,6 +214,8 @@ void sort_rows_by_key(ga_ctx ctx, const int32_t* rst, int64_t m, int32_t* key, i
 // the two buffers; true when the result is in tkeys / tpay.
 bool radix_sort_u64(ga_ctx ctx, uint64_t* keys, uint64_t* tkeys, int32_t* pay, int32_t* tpay, int64_t n, int bits);
 bool radix_sort_u32(ga_ctx ctx, uint32_t* keys, uint32_t* tkeys, int32_t* pay, int32_t* tpay, int64_t n, int bits);
+// Bytes that either allocates, at most.
+int64_t radix_sort_bytes(int64_t n);
 // Bits of the integers 0 .. n - 1.
 inline int bits_for(int64_t n) {
     int b = 0;
@@ -358,6 +360,8 @@ void tri_count(ga_ctx ctx, ga_csr A, unsigned long long* d_total, unsigned long 
 
 // device-side transpose (counting sort; rows of the result sorted)
 ga_csr transpose_csr(ga_ctx ctx, ga_csr A);
+// Bytes that it allocates beside the result, for nnz entries, at most.
+int64_t transpose_bytes(int64_t nnz, ga_dtype dt);
 ga_csr extract_tri(ga_ctx ctx, ga_csr A, bool lower);
 ga_csr copy_csr(ga_ctx ctx, ga_csr A, ga_dtype to);
 
@@ -397,6 +401,9 @@ bool csr_is_symmetric(ga_ctx ctx, ga_csr A);
 // Values aligned with the symmetric A's entries: those above the diagonal
 // copied to their mirrors.
 void mirror_values(ga_ctx ctx, ga_csr A, void* vals, ga_dtype dt);
+// Bytes that a BC call allocates beside its sources and scores, at most:
+// m vertices, nnz entries, ns source columns.
+int64_t bc_bytes(int64_t m, int64_t nnz, int64_t ns);
 // Batched BC over the block-diagonal union U of `count` graphs (host vertex
 // offsets voff), graph g with the sources [soff[g], soff[g+1]) of the host
 // array `sources` (indices within graph g); scores of U's rows into d_bc.

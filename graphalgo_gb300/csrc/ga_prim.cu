@@ -551,7 +551,8 @@ void sort_rows_by_key(ga_ctx ctx, const int32_t* rst, int64_t m, int32_t* key, i
 // Transpose by a stable sort of the columns: the entries keep their rows'
 // order inside every column, so the result's rows come sorted. R-MAT 18's
 // lower triangle (3.8M entries) in 210 us; counted and scattered with atomics
-// and sorted row by row it took 1,310 us (10,500 entries: 49 and 86 us).
+// and sorted row by row it took 1,310 us (10,500 entries: 49 and 86 us). Beside
+// the result it holds transpose_bytes(): 9 bytes per entry.
 __global__ void k_sorted_rst(const uint32_t* __restrict__ key, int64_t nnz, int64_t n, int32_t* __restrict__ rst) {
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j <= n; j += (int64_t)gridDim.x * blockDim.x) {
         int64_t lo = 0, hi = nnz;  // keys below j
@@ -568,10 +569,10 @@ __global__ void k_iota(int32_t* __restrict__ v, int64_t n) {
         v[i] = (int32_t)i;
 }
 
+// src may be col: a thread reads its source before it writes its column.
 template <typename T>
-__global__ void k_transpose_gather(const int32_t* __restrict__ src, const int32_t* __restrict__ row_of,
-                                   const T* __restrict__ v, int64_t nnz, int32_t* __restrict__ col,
-                                   T* __restrict__ val) {
+__global__ void k_transpose_gather(const int32_t* src, const int32_t* __restrict__ row_of, const T* __restrict__ v,
+                                   int64_t nnz, int32_t* col, T* __restrict__ val) {
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += (int64_t)gridDim.x * blockDim.x) {
         const int32_t s = src[q];
         col[q] = row_of[s];
@@ -579,27 +580,37 @@ __global__ void k_transpose_gather(const int32_t* __restrict__ src, const int32_
     }
 }
 
+int64_t transpose_bytes(int64_t nnz, ga_dtype dt) {
+    const int64_t buffers = dtype_size(dt) >= sizeof(uint32_t) ? 2 : 3;
+    return buffers * 4 * nnz + radix_sort_bytes(nnz) + 64;
+}
+
 ga_csr transpose_csr(ga_ctx ctx, ga_csr A) {
     ProfScope ps(ctx, "transpose");
     const int64_t nnz = A->nnz;
     ga_csr T = csr_alloc(ctx, A->n, A->m, nnz, A->dtype);
     try {
-        DBuf<uint32_t> key(ctx, (size_t)nnz), tkey(ctx, (size_t)nnz);
-        DBuf<int32_t> src(ctx, (size_t)nnz), tsrc(ctx, (size_t)nnz), row_of(ctx, (size_t)nnz);
+        // The sort's other buffers are the result's own arrays: columns are
+        // placed where their sources lay, values where keys were.
+        const bool wide = dtype_size(A->dtype) >= sizeof(uint32_t);
+        DBuf<uint32_t> key(ctx, (size_t)nnz), spare(ctx, wide ? 1 : (size_t)nnz);
+        DBuf<int32_t> tsrc(ctx, (size_t)nnz);
+        uint32_t* tkey = wide ? static_cast<uint32_t*>(T->val) : spare.p;
         const int grid = grid_for(nnz, 256, ctx->num_sms * 8);
         if (nnz) {
             GA_CUDA(cudaMemcpyAsync(key.p, A->col, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, ctx->stream));
-            k_iota<<<grid, 256, 0, ctx->stream>>>(src.p, nnz);
+            k_iota<<<grid, 256, 0, ctx->stream>>>(T->col, nnz);
             post_launch("iota");
-            expand_rows(ctx, A, row_of.p);
         }
-        const bool other = radix_sort_u32(ctx, key.p, tkey.p, src.p, tsrc.p, nnz, bits_for(A->n));
-        k_sorted_rst<<<grid_for(A->n + 1, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(other ? tkey.p : key.p, nnz,
+        const bool other = radix_sort_u32(ctx, key.p, tkey, T->col, tsrc.p, nnz, bits_for(A->n));
+        k_sorted_rst<<<grid_for(A->n + 1, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(other ? tkey : key.p, nnz,
                                                                                         A->n, T->rst);
         post_launch("transpose_rst");
         if (nnz) {
+            int32_t* row_of = reinterpret_cast<int32_t*>(key.p);  // the keys are read
+            expand_rows(ctx, A, row_of);
             GA_DISPATCH_DTYPE(A->dtype, V, {
-                k_transpose_gather<V><<<grid, 256, 0, ctx->stream>>>(other ? tsrc.p : src.p, row_of.p,
+                k_transpose_gather<V><<<grid, 256, 0, ctx->stream>>>(other ? tsrc.p : T->col, row_of,
                                                                      static_cast<const V*>(A->val), nnz, T->col,
                                                                      static_cast<V*>(T->val));
             });

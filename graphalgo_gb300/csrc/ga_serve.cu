@@ -44,9 +44,13 @@ static int64_t bound_ktruss(int64_t m, int64_t nnz) {
 }
 
 static int64_t bound_bc(int64_t m, int64_t nnz, int64_t ns) {
+    // Sources, scores and the call's own arrays. At least what requests have
+    // been admitted by from the start (40 bytes per pair; the call's arrays
+    // take 28 where few neighbour lists are long).
     const int64_t words = (ns + 31) / 32;
-    // FP64 copy (and transpose), entry store, dense W, per-vertex state
-    return 40 * (m + 1) * (ns + 1) + 4 * m * words + 80 * (m + 2) + 32 * nnz + (1 << 20);
+    return std::max(40 * (m + 1) * (ns + 1) + 4 * m * words + 80 * (m + 2) + 32 * nnz,
+                    4 * (ns + 1) + 8 * (m + 1) + bc_bytes(m, nnz, ns)) +
+           (1 << 20);
 }
 
 // ns: the union's sources; ncols: the largest source count of one graph

@@ -138,6 +138,11 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const K* __rest
     }
 }
 
+int64_t radix_sort_bytes(int64_t n) {
+    const int64_t cells = ((n + kRadixTile - 1) / kRadixTile) << kDigitBits;
+    return sizeof(int32_t) * (cells + 1) + (int64_t)scan_scratch_bytes(cells);
+}
+
 template <typename K>
 static bool radix_sort(ga_ctx ctx, K* keys, K* tkeys, int32_t* pay, int32_t* tpay, int64_t n, int bits) {
     if (n <= 1 || bits <= 0) return false;
