@@ -617,8 +617,7 @@ static ga_csr cmask_narrow(ga_ctx ctx, ga_csr A, ga_csr B, CmArgs<T> p) {
     DBuf<int32_t> bpos(ctx, (size_t)B->m * blocks), cnt(ctx, (size_t)m + 1), rst(ctx, (size_t)m + 1);
     DBuf<NarrowTask> tasks(ctx, places);
     DBuf<int32_t> done(ctx, places), ntask(ctx, 1);
-    DBuf<T> part(ctx, places * blocks * 64);
-    const NarrowArgs a{bbits.p, bpos.p, pat.p, B->m, blocks, tasks.p, ntask.p, done.p, part.p};
+    NarrowArgs a{bbits.p, bpos.p, pat.p, B->m, blocks, tasks.p, ntask.p, done.p, nullptr};
     const unsigned grid = (unsigned)((m + kNarrowWarps - 1) / kNarrowWarps);
     {
         ProfScope ps(ctx, "cmask_symbolic");
@@ -630,7 +629,13 @@ static ga_csr cmask_narrow(ga_ctx ctx, ga_csr A, ga_csr B, CmArgs<T> p) {
         post_launch("cmask_narrow_symbolic");
     }
     scan_exclusive_i32(ctx, cnt.p, rst.p, m);
-    const int64_t nnz = read_i32(ctx, rst.p + m);
+    int32_t* h = reinterpret_cast<int32_t*>(ctx->h_pinned);
+    GA_CUDA(cudaMemcpyAsync(h, rst.p + m, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    GA_CUDA(cudaMemcpyAsync(h + 1, ntask.p, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    GA_CUDA(cudaStreamSynchronize(ctx->stream));
+    const int64_t nnz = h[0];
+    DBuf<T> part(ctx, (size_t)h[1] * blocks * 64);  // partial sums of the pieces that there are
+    a.part = part.p;
     ga_csr C = csr_alloc(ctx, m, B->n, nnz, A->dtype);
     try {
         GA_CUDA(cudaMemcpyAsync(C->rst, rst.p, sizeof(int32_t) * (m + 1), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -655,7 +660,16 @@ static ga_csr cmask_typed(ga_ctx ctx, ga_csr A, ga_csr B, const int32_t* mr, con
     p.br = B->rst; p.bc = B->col; p.bv = static_cast<const T*>(B->val);
     p.mr = mr; p.mc = mc; p.m = A->m;
     p.flops = nullptr; p.cnt = nullptr; p.cr = nullptr; p.cc = nullptr; p.cv = nullptr;
-    if (A->m > 0 && B->n >= 1 && B->n <= kNarrowCols) return cmask_narrow<T>(ctx, A, B, p);
+    if (A->m > 0 && B->n >= 1 && B->n <= kNarrowCols) {
+        // Where its words (per 64 columns 12 bytes a row of B and 8 a row of A,
+        // empty rows too) or its partial sums do not fit in memory, the path
+        // below serves: it needs 16 bytes a row of A.
+        try {
+            return cmask_narrow<T>(ctx, A, B, p);
+        } catch (const Error& e) {
+            if (e.code != GA_ERR_OOM) throw;
+        }
+    }
     DBuf<int64_t> flops(ctx, (size_t)A->m + 1);
     DBuf<int32_t> cnt(ctx, (size_t)A->m + 1);
     p.flops = flops.p; p.cnt = cnt.p;
