@@ -11,7 +11,8 @@
 // accumulator and bitmap, which yields sorted output directly.
 //
 // Products with at most kNarrowCols columns (the frontier of a batched search:
-// one column per source) take the narrow path below instead.
+// one column per source) take the narrow path below instead where it pays
+// (narrow_pays).
 #include "ga_device.cuh"
 
 namespace ga {
@@ -608,6 +609,25 @@ __global__ void __launch_bounds__(kNarrowSumThreads) k_narrow_numeric(CmArgs<T> 
     }
 }
 
+// Whether the narrow path is the faster one, in nanoseconds of either beyond
+// what both need. The words are made for every row of B and of A whether an
+// entry of A meets it or not, so few rows of A against a tall B are the general
+// path's, which takes a CTA per row of A that has entries. B of 10^6 x 64 / 10^6
+// x 1,024 with two entries per row, A of 256 rows of 64 entries: 130 / 984 us by
+// words, 60 / 61 by rows; of 2,048: 136 / 1,006 and 133 / 160; 16,384: 182 /
+// 1,269 and 728 / 883; B of 20,000 x 64 / 1,024: 75 / 146 and 62 / 61, 76 / 144
+// and 139 / 159, 123 / 369 and 728 / 883. Rows in pieces are summed twice: 2,048
+// rows of 1,024 entries, B of 20,000 x 1,024, 1,109 and 747. Nearly empty
+// matrices of 2 x 10^6 rows, 0.05 entries each, 64 / 256 / 1,024 columns: 1,180 /
+// 1,781 / 3,973 and 3,600.
+static bool narrow_pays(const ga_csr_s& A, const ga_csr_s& B) {
+    const double rows = (double)std::min(A.m, A.nnz), nnz = (double)A.nnz, tall = (double)B.m;
+    const double by_rows = 22.0 * rows + 0.11 * nnz * (1.0 + (double)B.nnz / std::max(tall, 1.0));
+    const double per_entry = A.nnz > A.m * kNarrowHeavy ? 0.04 : 0.02;
+    const double by_words = 1e4 + (double)((B.n + 63) / 64) * (0.08 * tall + 0.02 * (double)A.m + per_entry * nnz);
+    return by_words < by_rows;
+}
+
 template <typename T>
 static ga_csr cmask_narrow(ga_ctx ctx, ga_csr A, ga_csr B, CmArgs<T> p) {
     const int64_t m = A->m;
@@ -660,7 +680,7 @@ static ga_csr cmask_typed(ga_ctx ctx, ga_csr A, ga_csr B, const int32_t* mr, con
     p.br = B->rst; p.bc = B->col; p.bv = static_cast<const T*>(B->val);
     p.mr = mr; p.mc = mc; p.m = A->m;
     p.flops = nullptr; p.cnt = nullptr; p.cr = nullptr; p.cc = nullptr; p.cv = nullptr;
-    if (A->m > 0 && B->n >= 1 && B->n <= kNarrowCols) {
+    if (A->m > 0 && B->n >= 1 && B->n <= kNarrowCols && narrow_pays(*A, *B)) {
         // Where its words (per 64 columns 12 bytes a row of B and 8 a row of A,
         // empty rows too) or its partial sums do not fit in memory, the path
         // below serves: it needs 16 bytes a row of A.

@@ -1,6 +1,7 @@
-"""Complemented products with few columns: memory that fails inside the narrow
-path, and what it holds. Against the oracle; the values are small integers, so
-the results must be equal.
+"""Complemented products with few columns: the narrow path over its tile edges
+(operands of enough rows that it is chosen), the general path where A has few
+rows, memory that fails inside the narrow path, and what it holds. Against the
+oracle; the values are small integers, so the results must be equal.
 """
 import numpy as np
 import pytest
@@ -29,6 +30,41 @@ def _operands(m, k, n, dtype, long_rows):
     key = rng.integers(0, m, 2 * m) * n + rng.integers(0, n, 2 * m)
     M = _csr(m, n, np.concatenate([key[key // n != 9], 8 * n + np.arange(n)]), dtype, rng)
     return A, B, M
+
+
+def _check(ctx, A, B, M, dtype):
+    od = np.int32 if np.dtype(dtype).kind == "i" else np.float64
+    R = oracle.mxm_cmask(*(oracle.Csr(X.m, X.n, X.rst, X.col, X.val.astype(od)) for X in (A, B, M)))
+    C = ga.mxm_cmask(to_device(ctx, A), to_device(ctx, B), to_device(ctx, M))
+    rst, col, val = C.download()
+    assert np.array_equal(rst, R.rst) and np.array_equal(col, R.col)
+    assert val.dtype == dtype and np.array_equal(val, R.val.astype(dtype))
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 64, 65, 129, 256, 1023, 1024, 1025])
+@pytest.mark.parametrize("dtype", [np.int32, np.int64, np.float32, np.float64])
+def test_narrow(ctx, n, dtype):
+    _check(ctx, *_operands(3000, 4200, n, dtype, [4200, 255, 256, 257, 511, 512, 513, 1025, 1, 300]), dtype)
+
+
+@pytest.mark.parametrize("m", [1, 2, 40, 500, 2048])
+@pytest.mark.parametrize("k", [70, 60000])
+@pytest.mark.parametrize("n", [64, 1000])
+def test_few_rows(ctx, m, k, n):
+    _check(ctx, *_operands(max(m, 10), k, n, np.float64, [min(k, 600), 1][:m]), np.float64)
+
+
+def test_few_rows_make_no_words(ctx):
+    """Few rows of A against a tall B: no words of B's rows (12 bytes each per 64 columns)."""
+    m, k, n = 16, 1 << 20, 1024
+    rng = np.random.default_rng(6)
+    A, B, M = (_csr(r, c, rng.integers(0, r, z) * c + rng.integers(0, c, z), np.float64, rng)
+               for r, c, z in ((m, k, 1000), (k, n, k), (m, n, 100)))
+    dA, dB, dM = to_device(ctx, A), to_device(ctx, B), to_device(ctx, M)
+    ctx.sync()
+    base, _ = ctx.mem_stats(reset_peak=True)
+    ga.mxm_cmask(dA, dB, dM)
+    assert ctx.mem_stats()[1] - base <= 1 << 20
 
 
 def test_memory_fails_inside(ctx):
