@@ -4,7 +4,7 @@
 //  1. k_row_bin computes each output row's mask length m_i and Gustavson
 //     product count P_i = sum_{k in A_i} nnz(B_k). Rows with an
 //     empty mask are skipped, rows without products get explicit zeros, short
-//     light rows (m_i <= kWarpSlots, P_i <= warp_max_flops or a limit of the
+//     light rows (m_i <= warp_slots, P_i <= warp_max_flops or a limit of the
 //     product's own) go to a warp queue, all others to a CTA queue as windows
 //     of at most kCtaSlots mask slots spanning fewer than kWinCols columns
 //     (heavy rows first, the heaviest in more windows).
@@ -54,12 +54,30 @@ namespace ga {
 
 constexpr int kMxmThreads = 512;
 constexpr int kMxmWarps = kMxmThreads / 32;
-// Mask slots per CTA work item and per warp row. Half as many of 8 bytes: the
+// Mask slots per CTA work item. Half as many of 8 bytes: the
 // third CTA fits on an SM then (75 KB each instead of 90), FP64 products of
 // 200,000 x 200,000 under 8-entry mask rows 1,695 -> 1,484 us, 50,021 x
 // 40,009 under 32-entry rows 2,195 -> 2,104.
 template <typename A> constexpr int kCtaSlots = sizeof(A) == 8 ? 2048 : 4096;
-template <typename A> constexpr int kWarpSlots = sizeof(A) == 8 ? 128 : 256;
+// Mask slots per warp row, and those up to which a warp's table holds columns:
+// with accumulators of 8 bytes three CTAs' tables of 256 do not fit on an SM, and
+// longer rows take one of slots (MD_SLOTS), in a kernel of its own for masks of
+// more than kSlotsMean entries per row on average. As CTA items, which take 22
+// ns however few products a row has, such rows were ten times slower: FP64
+// products of 200,000 rows under 129 / 180 / 256 mask entries, 100 products per
+// row 4,440 / 4,560 / 4,710 us, so 323 / 400 / 516; 4,800 per row 11,480 / 11,570
+// / 11,680 and 2,140 / 2,540 / 3,430. That kernel is 3 to 6 % slower where all
+// rows are shorter (60 / 120 entries, 900 products per row 456 / 553 us, so 478 /
+// 579), and up to 20 % where few rows are longer and these have many products
+// (50,021 x 40,009 under power-law rows of 24 entries on average 509 and 624;
+// of 67: 224 and 188). Merging has no table: all its rows up to 256 are a warp's,
+// unless there are so few that CTAs take them side by side (1,000 rows of 900
+// products 41 us by CTAs, 50 by warps; 30,000 rows 354 and 206).
+constexpr int kWarpSlots = 256;
+template <typename A> constexpr int kColumnSlots = sizeof(A) == 8 ? 128 : 256;
+constexpr int kSlotsMean = 64;
+constexpr int kFewRows = 12;   // rows per SM
+constexpr int kNoSlot = 255;
 constexpr int kLeastCtaSlots = 2048;
 constexpr int kWinCols = 1 << 17;          // column span of a CTA work item
 constexpr int kWinWords = kWinCols / 32;   // dense bitmap words
@@ -111,6 +129,7 @@ struct MxmArgs {
     int32_t cta_cap;
     unsigned long long* ctr;  // context work counters (GA_CTR_*)
     int64_t warp_max_flops, heavy_flops;
+    int32_t warp_slots;       // mask entries that a warp row has at most
     bool small;               // warp_max_flops is only a bound, and heavy rows are split
     BinSplit split;
     // hybrid form: rows whose inner-product work (sum over mask entries of
@@ -316,7 +335,7 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
             }
         }
         // warp rows
-        const bool short_row = todo && mi <= kWarpSlots<A> && f <= warp_max;
+        const bool short_row = todo && mi <= p.warp_slots && f <= warp_max;
         unsigned set = __ballot_sync(FULL, short_row);
         if (lane == 0) s_short[wid] = __popc(set);
         __syncthreads();
@@ -381,17 +400,17 @@ __global__ void __launch_bounds__(kBinThreads) k_row_bin(MxmArgs<T, A> p, int ta
 
 // ------------------------------------------------------------------ lookups
 // How a product's column finds its mask slot: MD_DENSE in CTA items, MD_HASHED
-// in warp rows; MD_MERGE merges whole B rows instead.
-enum { MD_DENSE = 0, MD_HASHED = 1, MD_MERGE = 2 };
+// or MD_SLOTS in warp rows; MD_MERGE merges whole B rows instead.
+enum { MD_DENSE = 0, MD_HASHED = 1, MD_MERGE = 2, MD_SLOTS = 3 };
 
 // The mask columns of one work item, staged in shared memory.
 struct SlotView {
-    const int32_t* mcol;    // MD_MERGE: sorted mask columns
+    const int32_t* mcol;    // MD_MERGE, MD_SLOTS: sorted mask columns
     const uint32_t* bits;   // MD_DENSE: bitmap over [lo, lo + kWinCols)
     const uint16_t* wbase;  // MD_DENSE: slot of the first mask column of each bitmap word
-    const uint32_t* filt;   // MD_HASHED: 4096-bit filter of hashed columns
+    const uint32_t* filt;   // MD_HASHED, MD_SLOTS: 4096-bit filter of hashed columns
     const int32_t* hkeys;   // MD_HASHED: open-addressing table (2^kWarpTblBits)
-    const uint8_t* hslot;
+    const uint8_t* hslot;   // MD_HASHED: their slots; MD_SLOTS: the table itself (kNoSlot: none)
     int ns;
     int32_t lo, hi;
 };
@@ -422,6 +441,15 @@ __device__ __forceinline__ int slot_of(const SlotView& v, int32_t c) {
         if (!((v.filt[f >> 5] >> (f & 31)) & 1u)) return -1;
         const uint32_t mask = (1u << kWarpTblBits) - 1u;
         uint32_t pos = h >> (32 - kWarpTblBits);
+        if (MD == MD_SLOTS) {
+            if (c == v.hi) return v.ns - 1;  // slot 255 would be kNoSlot: the last column is not in the table
+            int slot = v.hslot[pos];
+            while (slot != kNoSlot && v.mcol[slot] != c) {
+                pos = (pos + 1) & mask;
+                slot = v.hslot[pos];
+            }
+            return slot == kNoSlot ? -1 : slot;
+        }
         // One way out of the loop. With a return for the hit and one for the
         // empty place inside it, the code that nvcc 13.0 makes left lanes that
         // hit at their first place out of later rounds of the row while others
@@ -434,6 +462,18 @@ __device__ __forceinline__ int slot_of(const SlotView& v, int32_t c) {
         }
         return key == c ? (int)v.hslot[pos] : -1;
     }
+}
+
+// Enters the slot of column c into a table of slots (used: a bit per place, as
+// bytes cannot be claimed by themselves).
+__device__ __forceinline__ void slot_insert(uint32_t* used, uint8_t* hslot, int32_t c, int slot) {
+    uint32_t pos = hash_col(c) >> (32 - kWarpTblBits);
+    while (true) {
+        const uint32_t bit = 1u << (pos & 31);
+        if (!(atomicOr(&used[pos >> 5], bit) & bit)) break;
+        pos = (pos + 1) & ((1u << kWarpTblBits) - 1u);
+    }
+    hslot[pos] = (uint8_t)slot;
 }
 
 // Value modes: VM 0 general, 1 B's values are all ones (no B value loads),
@@ -833,7 +873,7 @@ __device__ __forceinline__ int64_t merge_group(const MxmArgs<T, A>& p, int32_t t
 }
 
 // Shared-memory layout per variant (MD of the CTA phase: MD_DENSE for MSA).
-template <int MD, typename A>
+template <int MD, typename A, bool SLOTS>
 struct MxmSmem {
     static constexpr bool dense = MD == MD_DENSE;
     // CTA phase
@@ -846,14 +886,18 @@ struct MxmSmem {
     static constexpr size_t off_wbase = off_key + (size_t)kWinWords * 4 + 16;  // behind a guard word
     static constexpr size_t cta_bytes =
         dense ? off_wbase + (size_t)kWinWords * 2 : off_key + (size_t)kCtaSlots<A> * 4;
-    // warp phase (per warp): acc, hashed filter and table, or mcol
+    // warp phase (per warp): acc and mcol; or acc, hkeys, hslot and the filter;
+    // or, by slots, acc and mcol over the first two, hslot, the filter and used
     static constexpr size_t w_acc = 0;
-    static constexpr size_t w_filt = w_acc + (size_t)kWarpSlots<A> * sizeof(A);
-    static constexpr size_t w_hkeys = w_filt + (size_t)(1 << kFilterBits) / 8;
+    static constexpr size_t w_mcol = w_acc + (size_t)kWarpSlots * sizeof(A);
+    static constexpr size_t w_hkeys = w_acc + (size_t)kColumnSlots<A> * sizeof(A);
     static constexpr size_t w_hslot = w_hkeys + (size_t)(1 << kWarpTblBits) * 4;
-    static constexpr size_t w_mcol = w_filt;
-    static constexpr size_t warp_one =
-        dense ? w_hslot + (size_t)(1 << kWarpTblBits) : w_mcol + (size_t)kWarpSlots<A> * 4;
+    static constexpr size_t w_filt = w_hslot + (size_t)(1 << kWarpTblBits);
+    static constexpr size_t w_used = w_filt + (size_t)(1 << kFilterBits) / 8;
+    static constexpr size_t warp_one = !dense ? w_mcol + (size_t)kWarpSlots * 4
+                                       : SLOTS ? w_used + (size_t)(1 << kWarpTblBits) / 8
+                                               : w_used;
+    static_assert(!SLOTS || w_mcol + (size_t)kWarpSlots * 4 <= w_hslot, "acc and mcol end before the table of slots");
     static constexpr size_t warp_bytes = warp_one * kMxmWarps;
     static constexpr size_t region = cta_bytes > warp_bytes ? cta_bytes : warp_bytes;
     // per-warp flattening scratch (both phases)
@@ -861,10 +905,10 @@ struct MxmSmem {
     static constexpr size_t total = region + scratch_bytes;
 };
 
-template <int MD, int VM, typename T, typename A>
+template <int MD, int VM, typename T, typename A, bool SLOTS>
 __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    using SM = MxmSmem<MD, A>;
+    using SM = MxmSmem<MD, A, SLOTS>;
     constexpr bool DENSE = MD == MD_DENSE;
     constexpr int WMD = DENSE ? MD_HASHED : MD;  // warp-row lookup
     const unsigned FULL = 0xffffffffu;
@@ -993,6 +1037,7 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
         int32_t* hkeys = reinterpret_cast<int32_t*>(base + SM::w_hkeys);
         uint8_t* hslot = reinterpret_cast<uint8_t*>(base + SM::w_hslot);
         int32_t* mcol = reinterpret_cast<int32_t*>(base + SM::w_mcol);
+        uint32_t* used = reinterpret_cast<uint32_t*>(base + SM::w_used);
         constexpr int FW = (1 << kFilterBits) / 32;
         constexpr int TBL = 1 << kWarpTblBits;
         if (DENSE)
@@ -1019,6 +1064,12 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
             v.mcol = mcol; v.bits = nullptr; v.wbase = nullptr; v.filt = filt; v.hkeys = hkeys; v.hslot = hslot;
             v.ns = mi;
             v.lo = __ldg(gcol); v.hi = __ldg(gcol + mi - 1);
+            const bool by_slots = SLOTS && mi > kColumnSlots<A>;
+            if (by_slots) {
+                if (lane < TBL / 32) used[lane] = 0u;
+                for (int t = lane; t < TBL / 4; t += 32) reinterpret_cast<uint32_t*>(hslot)[t] = ~0u;
+                __syncwarp();
+            }
             for (int s = lane; s < mi; s += 32) {
                 const int32_t c = __ldg(gcol + s);
                 acc[s] = (A)0;
@@ -1026,6 +1077,11 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
                     const uint32_t h = hash_col(c);
                     const uint32_t f = h >> (32 - kFilterBits);
                     atomicOr(&filt[f >> 5], 1u << (f & 31));
+                }
+                if (by_slots) {
+                    mcol[s] = c;
+                    if (s + 1 < mi) slot_insert(used, hslot, c, s);
+                } else if (DENSE) {
                     hash_insert<uint8_t>(hkeys, hslot, kWarpTblBits, c, (uint8_t)s);
                 } else {
                     mcol[s] = c;
@@ -1037,6 +1093,10 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
                 for (int32_t g = ab; g < ae; g += 32)
                     executed += (unsigned long long)merge_group<T, A, false>(p, g, ae, clip, v, acc, nullptr,
                                                                              nullptr, nullptr, nullptr);
+            } else if (by_slots) {
+                for (int32_t g = ab; g < ae; g += 32)
+                    executed += (unsigned long long)group_products<SLOTS ? MD_SLOTS : WMD, VM, T, A, false>(
+                        p, g, ae, clip, v, acc, s_incl, s_off, s_a, nullptr, nullptr, nullptr, nullptr);
             } else {
                 for (int32_t g = ab; g < ae; g += 32)
                     executed += (unsigned long long)group_products<WMD, VM, T, A, false>(
@@ -1044,6 +1104,7 @@ __global__ void __launch_bounds__(kMxmThreads, 3) k_mxm_masked(MxmArgs<T, A> p) 
             }
             __syncwarp();
             for (int s = lane; s < mi; s += 32) p.cv[mb + s] = from_acc<T, A>(acc[s]);
+            if (by_slots) __syncwarp();  // the table of columns lies over acc
             if (DENSE)
                 for (int t = lane; t < FW; t += 32) filt[t] = 0u;
             if (DENSE)
@@ -1083,6 +1144,10 @@ static void launch_masked(ga_ctx ctx, ga_csr A_, ga_csr B_, ga_csr M_, T* cv, Mx
     p.ctr = ctx->d_counters;
     p.heavy_flops = ctx->tune.heavy_flops;
     p.split = LK == MD_MERGE ? kSplitMerge : kSplit;
+    constexpr bool kHasSlots = LK == MD_DENSE && kColumnSlots<Ac> < kWarpSlots;
+    const bool slots = kHasSlots && M_->nnz > (int64_t)kSlotsMean * p.m;
+    const bool all = LK == MD_MERGE ? p.m > (int64_t)kFewRows * ctx->num_sms : slots;
+    p.warp_slots = all ? kWarpSlots : kColumnSlots<Ac>;
     p.warp_max_flops = ctx->tune.warp_max_flops;
     // the limit reaches the option's default at (32,768 / kWarpShare)^2
     // products; rows of mean length give a lower bound of their number
@@ -1098,8 +1163,8 @@ static void launch_masked(ga_ctx ctx, ga_csr A_, ga_csr B_, ga_csr M_, T* cv, Mx
         k_row_bin<T, Ac><<<grid, kBinThreads, 0, ctx->stream>>>(p, take);
         post_launch("mxm_row_bin");
     }
-    const size_t smem = MxmSmem<LK, Ac>::total;
-    auto kern = k_mxm_masked<LK, VM, T, Ac>;
+    const size_t smem = slots ? MxmSmem<LK, Ac, kHasSlots>::total : MxmSmem<LK, Ac, false>::total;
+    auto kern = slots ? k_mxm_masked<LK, VM, T, Ac, kHasSlots> : k_mxm_masked<LK, VM, T, Ac, false>;
     GA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     GA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMxmThreads, smem));
