@@ -101,7 +101,11 @@ GA_API int ga_version(int* major, int* minor);
 
 /* Context options. GA_OPT_DEVICE_LOOPS (default 1): run the k-truss and BC
  * iteration loops as CUDA graphs with device-side WHILE conditions (no host
- * round trip per iteration); 0 runs the same kernels from a host loop.
+ * round trip per iteration), the GA_TRI k-truss of one matrix as one
+ * cooperative launch; 0 runs them from a host loop. A cooperative launch
+ * starts when every SM has room for one of its CTAs: behind a kernel of
+ * another stream that holds SMs and never ends it would wait for ever, so a
+ * program that keeps such a kernel resident sets 0.
  * GA_OPT_PROFILE: when 1, each kernel launch is bracketed by CUDA events and
  * ga_ctx_kernel_stats reports per-kernel totals. GA_OPT_FAIL_ALLOC_AFTER:
  * fault injection for tests — the N-th device allocation from now on fails
@@ -414,6 +418,9 @@ GA_API int ga_ktruss(ga_ctx ctx, ga_algo algo, ga_csr A, int k, ga_csr* C, int* 
  * context. An error (memory ran out, a wait ran out) ends a sweep whose
  * state stays on the device: later calls return the same error. In the other
  * cases the call can be made again. No counterpart in the reference (its CLI runs one k per call). */
+/* Either returns GA_ERR_TIMEOUT when CTAs of its cooperative launch have
+ * waited 2e10 SM clock cycles (about ten seconds) for the others at one
+ * barrier; the context stays usable. */
 typedef struct ga_kt_sweep_s* ga_kt_sweep;
 GA_API int ga_ktruss_sweep_begin(ga_ctx ctx, ga_algo algo, ga_csr A, int kmin, ga_kt_sweep* sweep);
 GA_API int ga_ktruss_sweep_next(ga_kt_sweep sweep, ga_csr* C, int* k, int* iters);
