@@ -127,19 +127,6 @@ __device__ __forceinline__ void hash_insert(int32_t* keys, S* slots, int bits, i
     }
 }
 
-// Returns the payload for key `k`, or -1 when absent.
-template <typename S>
-__device__ __forceinline__ int hash_find(const int32_t* keys, const S* slots, int bits, int32_t k) {
-    const uint32_t mask = (1u << bits) - 1u;
-    uint32_t h = hash_col(k) >> (32 - bits);
-    while (true) {
-        int32_t cur = keys[h];
-        if (cur == k) return (int)slots[h];
-        if (cur == kEmpty) return -1;
-        h = (h + 1) & mask;
-    }
-}
-
 // lower_bound over a sorted int32 array
 __device__ __forceinline__ int lower_bound_i32(const int32_t* a, int n, int32_t x) {
     int lo = 0, hi = n;

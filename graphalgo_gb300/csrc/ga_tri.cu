@@ -1260,13 +1260,7 @@ __global__ void k_trif_mark(const TriFrontArgs* __restrict__ ap) {
     const int t = a.st->t;
     const int32_t n = a.st->cnt[t & 1];
     const int32_t* F = (t & 1) ? a.f1 : a.f0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(&a.ctr[GA_CTR_PRODUCTS], a.st->prod);
-        atomicAdd(&a.ctr[GA_CTR_MASK_ENTRIES], a.st->mask);
-        atomicAdd(&a.ctr[GA_CTR_A_ENTRIES], a.st->ent);
-        atomicAdd(&a.ctr[GA_CTR_LAUNCHES], 1ull);
-        atomicAdd(&a.ctr[GA_CTR_ROWS], (unsigned long long)a.m);
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) trif_count_iteration(a);
     for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
         const int32_t q = F[x];
         if (!kt_frozen(a, a.row_of[q])) a.state[q] = kDying;
@@ -2345,7 +2339,7 @@ struct TriFront::Impl {
         A.col = const_cast<int32_t*>(a.ac);
         expand_rows(ctx, &A, row_of);
         trikt_partition(ctx, a.cr, a.ac, m, nnz, row_of, t, batch, pcol);
-            k_trif_init_rows<<<grid_for(m, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a);
+        k_trif_init_rows<<<grid_for(m, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(a);
         post_launch("trif_init_rows");
         if (nnz) {
             k_trif_records<<<grid_ent, 256, 0, ctx->stream>>>(a, words, t.dpos);
