@@ -75,6 +75,9 @@ DRAM_BYTES_PER_ENTRY = {"tri_support": 7.506, "mxm": 4.543}
 # caches stay warm as in the timed step: 1,721.0 MB) over its 3,805,777
 # pruned edges (profiles/trif_lower_rmat18_sweep.md).
 DRAM_BYTES_PER_FRONT_EDGE = 452.2
+# The same of the loop in one launch: all 162 launches of k_trif_loop in that
+# sweep, 1,912.5 MB (profiles/trif_loop_rmat18.md).
+DRAM_BYTES_PER_LOOP_EDGE = 502.5
 
 
 def parse_args():
@@ -394,24 +397,26 @@ def sweep(ga, ctx, A, algo, kmin, sink=None, per_k=None):
     return out
 
 
-def profile_step(ga, ctx, run, algo, counters, loops):
-    """Runs one step with host-driven loops and per-kernel timing; returns the
-    launch count and the roofline of the step's dominant kernel.
+def profile_step(ga, ctx, run, algo, counters, loops, as_timed=False):
+    """Runs one step with per-kernel timing; returns the launch count and the
+    roofline of the step's dominant kernel. The loops are driven by the host,
+    so that their kernels can be timed; as_timed: they stay as in the timed
+    step (the triangle-listing k-truss of one matrix, whose loop is a kernel).
 
     Gustavson variants: achieved = algorithmic bytes of the Gustavson model
     with int32 values (s = 4): 4(m+1)*2 + nnz(A)*(4+4) + nnz(A)*8 + P*(4+4) +
     nnz(M)*4 + nnz(C)*4, P being the products the kernel processed (the
     support of a symmetric C evaluates its upper triangle and mirrors it),
     divided by the kernel's summed event time. Triangle listing (the sweep
-    lists the triangles once and then prunes by frontier): the frontier
-    kernel k_trif_lower, 48 bytes per pruned edge (its frontier slot, row,
+    lists the triangles once and then prunes by frontier): the loop in one
+    launch, k_trif_loop, or the frontier kernel k_trif_lower, 48 bytes per pruned edge (its frontier slot, row,
     column, diagonal positions, support, both rows' bounds, the oriented
     count and rank of the far row), 34 bytes per probed row entry (column,
     record position, state and rank of the entry, about four binary-search
     steps in the other row, the found entry's record position and state) and
     16 bytes per destroyed triangle (two 4-byte support read-modify-writes),
     over its summed event time."""
-    ctx.set_option(ga.OPT_DEVICE_LOOPS, 0)
+    ctx.set_option(ga.OPT_DEVICE_LOOPS, loops if as_timed else 0)
     ctx.set_option(ga.OPT_PROFILE, 1)
     ctx.reset_kernel_stats()
     ctx.work_counters(reset=True)
@@ -425,11 +430,11 @@ def profile_step(ga, ctx, run, algo, counters, loops):
     ctx.set_option(ga.OPT_PROFILE, 0)
     ctx.set_option(ga.OPT_DEVICE_LOOPS, loops)
     kname = {"msa": "mxm_msa", "mca": "mxm_mca", "heap": "mxm_heap_merge", "dot": "mxm_dot",
-             "hybrid": "mxm_msa", "tri": "trif_lower"}[algo]
+             "hybrid": "mxm_msa", "tri": "ktruss_loop" if as_timed and loops else "trif_lower"}[algo]
     k_launches, k_ms = stats.get(kname, (0, 0.0))
     if algo == "tri":
         bytes_model = 48 * ctr["front_edges"] + 34 * ctr["front_probes"] + 16 * ctr["front_triangles"]
-        tpe = DRAM_BYTES_PER_FRONT_EDGE
+        tpe = DRAM_BYTES_PER_LOOP_EDGE if kname == "ktruss_loop" else DRAM_BYTES_PER_FRONT_EDGE
         traffic_units = ctr["front_edges"]  # the capture's DRAM bytes are per pruned edge
     else:
         # products of the Gustavson kernels; list entries walked for the inner-product one
@@ -443,7 +448,7 @@ def profile_step(ga, ctx, run, algo, counters, loops):
     return {"launches": launches, "kernel_ms": k_ms, "stats": stats, "counters": ctr,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                         "kernel": kname, "peak_kind": peak_kind,
+                         "kernel": "trif_loop" if kname == "ktruss_loop" else kname, "peak_kind": peak_kind,
                          "bytes_per_launch": bytes_model / max(1, k_launches),
                          "avg_launch_ms": k_ms / max(1, k_launches)}}
 
@@ -553,14 +558,16 @@ def other_configs(ga, ctx, args, with_cpu: bool):
         out[f"bc_rmat20_{ns}src"] = r
     # the masked product itself on the same graph (31.4M entries: operands
     # larger than L2), C<A> = A*A with int32 values, default schedule, per
-    # Gustavson variant against the survey's byte model 8(m+1) + 16 nnz(A) +
-    # 8 P + 4 nnz(M) + 4 nnz(C); triangle listing (which performs no
-    # Gustavson products) by time only
+    # Gustavson variant against the byte model 8(m+1) + 16 nnz(A) + 8 P +
+    # 4 nnz(M) + 4 nnz(C), P being the products that the kernels processed
+    # (half of a symmetric product is computed and mirrored; the inner-product
+    # rows of the hybrid form: the list entries walked); triangle listing (which
+    # performs no Gustavson products) by time only
     nnz = len(col)
     mx = {}
     for algo in ("msa", "hybrid", "mca", "tri"):
         ga.mxm_masked(algo, A, A, A).free()
-        best, prods = None, 0
+        best, prods, done = None, 0, 0
         for _ in range(2):
             ctx.work_counters(reset=True)
             ctx.flush_l2()
@@ -568,11 +575,12 @@ def other_configs(ga, ctx, args, with_cpu: bool):
             C = ga.mxm_masked(algo, A, A, A)
             t = ctx.timer_stop()
             C.free()
-            prods = ctx.work_counters(reset=True)["products"]
+            w = ctx.work_counters(reset=True)
+            prods, done = w["products"], w["executed"] + w["executed_dot"]
             best = t if best is None else min(best, t)
         rec = {"ms": best, "reference_equivalent_gflops": 2.0 * prods / best / 1e6}
         if algo != "tri":
-            bm = 8 * (m + 1) + 16 * nnz + 8 * prods + 4 * nnz + 4 * nnz
+            bm = 8 * (m + 1) + 16 * nnz + 8 * done + 4 * nnz + 4 * nnz
             rec["roofline"] = {"bound": "hbm", "achieved": bm / (best * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                                "frac": bm / (best * 1e-3) / 1e9 / peak, "bytes_per_call": bm,
                                "peak_kind": peak_kind, "traffic": None}
@@ -635,7 +643,7 @@ def run_gpu(args, dist: Dist):
     per_k = {}
     prof = profile_step(ga, ctx, lambda: sweep(ga, ctx, A, args.algo, args.kmin, per_k=per_k), args.algo,
                         lambda: {key: sum(v[key] for v in per_k.values()) for key in next(iter(per_k.values()))},
-                        loops)
+                        loops, as_timed=args.algo == "tri")
     launches_per_step = prof["launches"]
     roofline = prof["roofline"]
     roofline["kernel_share_of_step"] = prof["kernel_ms"] / (total_ms / args.steps) if total_ms else None
