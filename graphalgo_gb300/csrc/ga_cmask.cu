@@ -634,14 +634,15 @@ static ga_csr cmask_narrow(ga_ctx ctx, ga_csr A, ga_csr B, CmArgs<T> p) {
     const int blocks = (int)((B->n + 63) / 64);
     const size_t places = (size_t)(A->nnz / kNarrowPiece + A->nnz / kNarrowHeavy + 1);
     DBuf<unsigned long long> bbits(ctx, (size_t)B->m * blocks), pat(ctx, (size_t)m * blocks);
-    DBuf<int32_t> bpos(ctx, (size_t)B->m * blocks), cnt(ctx, (size_t)m + 1), rst(ctx, (size_t)m + 1);
+    DBuf<int32_t> bpos(ctx, (size_t)B->m * blocks), cnt(ctx, (size_t)m + 1), rst(ctx, (size_t)m + 2);
     DBuf<NarrowTask> tasks(ctx, places);
-    DBuf<int32_t> done(ctx, places), ntask(ctx, 1);
-    NarrowArgs a{bbits.p, bpos.p, pat.p, B->m, blocks, tasks.p, ntask.p, done.p, nullptr};
+    DBuf<int32_t> done(ctx, places);
+    int32_t* ntask = rst.p + m + 1;  // behind the entries' number: one copy reads both
+    NarrowArgs a{bbits.p, bpos.p, pat.p, B->m, blocks, tasks.p, ntask, done.p, nullptr};
     const unsigned grid = (unsigned)((m + kNarrowWarps - 1) / kNarrowWarps);
     {
         ProfScope ps(ctx, "cmask_symbolic");
-        GA_CUDA(cudaMemsetAsync(ntask.p, 0, sizeof(int32_t), ctx->stream));
+        GA_CUDA(cudaMemsetAsync(ntask, 0, sizeof(int32_t), ctx->stream));
         k_row_bits<<<grid_for(B->m * 32, 256, ctx->num_sms * 64), 256, 0, ctx->stream>>>(B->rst, B->col, B->m, blocks,
                                                                                          bbits.p, bpos.p);
         post_launch("cmask_row_bits");
@@ -650,8 +651,7 @@ static ga_csr cmask_narrow(ga_ctx ctx, ga_csr A, ga_csr B, CmArgs<T> p) {
     }
     scan_exclusive_i32(ctx, cnt.p, rst.p, m);
     int32_t* h = reinterpret_cast<int32_t*>(ctx->h_pinned);
-    GA_CUDA(cudaMemcpyAsync(h, rst.p + m, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    GA_CUDA(cudaMemcpyAsync(h + 1, ntask.p, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    GA_CUDA(cudaMemcpyAsync(h, rst.p + m, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
     GA_CUDA(cudaStreamSynchronize(ctx->stream));
     const int64_t nnz = h[0];
     DBuf<T> part(ctx, (size_t)h[1] * blocks * 64);  // partial sums of the pieces that there are
